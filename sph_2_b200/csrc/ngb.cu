@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, 6)
             for (int u = 0; u < U; u++) jj[u] = k0 + u < craw ? __ldg(&crow[k0 + u]) : i;
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                pj[u] = p0[jj[u]];
+                pj[u] = ld_wide(p0 + jj[u]);
                 hj[u] = __ldg(&hc[jj[u]]);
             }
 #pragma unroll

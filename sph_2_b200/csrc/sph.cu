@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256)
         const int *row = rows + (size_t)i * K;
         for (int k = sl; k < c; k += LANES) {
             const int j = row[k];
-            const double4 pj = p0[j];
+            const double4 pj = ld_pos<R>(p0 + j);
             const R mj = p1[j].w;
             const R dx = (R)(pi.x - pj.x), dy = (R)(pi.y - pj.y), dz = (R)(pi.z - pj.z);
             const R rr = qsqrt<R>(dx * dx + dy * dy + dz * dz);
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(256)
         const int *row = rows + (size_t)i * K;
         for (int k = sl; k < c; k += LANES) {
             const int j = row[k];
-            const double4 pj = p0[j];
+            const double4 pj = ld_pos<R>(p0 + j);
             const typename R4<R>::T vj = p1[j];
             const R dx = (R)(pi.x - pj.x), dy = (R)(pi.y - pj.y), dz = (R)(pi.z - pj.z);
             const R rr = qsqrt<R>(dx * dx + dy * dy + dz * dz);
@@ -146,7 +146,7 @@ __device__ __forceinline__ void density_divcurl_one(
         const int *row = rows + (size_t)i * K;
         for (int k = sl; k < c; k += LANES) {
             const int j = row[k];
-            const double4 pj = p0[j];
+            const double4 pj = ld_pos<R>(p0 + j);
             const typename R4<R>::T vj = p1[j];
             const R dx = (R)(pi.x - pj.x), dy = (R)(pi.y - pj.y), dz = (R)(pi.z - pj.z);
             const R rr = qsqrt<R>(dx * dx + dy * dy + dz * dz);
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(256, std::is_same<R, float>::value ? SPH_LISTS
         double4 pj = pi;
         if (k < craw) {
             j = crow[k];
-            pj = p0[j];
+            pj = ld_pos<R>(p0 + j);
             hit = ngb_pred(pi.x, pi.y, pi.z, pi.w, pj.x, pj.y, pj.z, pj.w);
         }
         const unsigned m = __ballot_sync(0xffffffffu, hit) & seg;
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(256, std::is_same<R, float>::value ? SPH_FORCE
         const R eta2 = eta * eta;
         for (int k = sl; k < c; k += LANES) {
             const int j = row[k];
-            const double4 pj = p0[j];
+            const double4 pj = ld_pos<R>(p0 + j);
             const typename R4<R>::T vj = p1[j], qj = p2[j];
             const R dx = (R)(pi.x - pj.x), dy = (R)(pi.y - pj.y), dz = (R)(pi.z - pj.z);
             const R rr = qsqrt<R>(dx * dx + dy * dy + dz * dz);

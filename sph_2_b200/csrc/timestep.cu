@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256)
         const int *row = rows + (size_t)i * K;
         for (int k = sl; k < cn; k += LANES) {
             const int j = row[k];
-            const double4 pj = p0[j];
+            const double4 pj = ld_pos<R>(p0 + j);
             const V4 vj = p1[j];
             const R cj = p2[j].z;
             const R dx = (R)(pi.x - pj.x), dy = (R)(pi.y - pj.y), dz = (R)(pi.z - pj.z);
