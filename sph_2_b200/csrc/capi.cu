@@ -397,7 +397,7 @@ int sph_ctx_create(const sph_config *cfg, sph_ctx **out) {
     DAF(ctx->cand_cnt, N);
     DAF(ctx->lflag, N + 3);
     DAF(ctx->mlist, N);
-    DAF(ctx->retry, N); DAF(ctx->hcand, N); DAF(ctx->hiter, N); DAF(ctx->hover, N);
+    DAF(ctx->retry, N); DAF(ctx->hcand, N); DAF(ctx->hover, N);
     DAF(ctx->hsr, N); DAF(ctx->dmv, N); DAF(ctx->gdm, N);
     DAF(ctx->dmv_max, C + 1);
     ctx->rows_ok = (int *)(ctx->dmv_max + C);

@@ -32,6 +32,9 @@
 namespace {
 
 constexpr int SEARCH_WARPS = 4;
+// particles per SM up to which a cloud's searches take 8, 4 or 2 lanes per
+// particle (search_split; the measurements behind the lines stand there)
+constexpr int SPLIT8_PER_SM = 68, SPLIT4_PER_SM = 140, SPLIT2_PER_SM = 300;
 constexpr int SSTK = 512;
 constexpr unsigned FULL = 0xffffffffu;
 // pending bucket particles: ranges of consecutive slots, range r starting at
@@ -140,17 +143,23 @@ struct SearchArgs {
     long long *status;
 };
 
-// Walk the tree for group g and write the rows of the active lanes.
+// Walk the tree from `root` and write the rows of the active lanes' particles.
 // MODE 0: candidates r^2 <= ri^2 (ri = 2 hc_i, the h iteration's gather radius)
 //         with the first Newton evaluation's kernel sums
 // MODE 1: exact lists |r|^2 <= (h_i + h_j)^2
 // MODE 2: candidates r^2 <= ri^2 alone (the count iteration)
-template <int MODE, class R = double>
-__device__ __forceinline__ void group_search(SearchSmem &S, const SearchArgs &A, int g, bool act,
-                                             int i, const double4 &pi, double ri,
-                                             HSums<R> *hs = nullptr) {
+// SPLIT consecutive lanes hold the same particle and each takes 32 / SPLIT of
+// the 32 staged candidates of a chunk (see Unit below); a particle's row is in
+// candidate order for every SPLIT.  hs then holds the lane's part of the sums.
+// Returns the particle's full count on each of its lanes.
+template <int MODE, class R = double, int SPLIT = 1>
+__device__ __forceinline__ int group_search(SearchSmem &S, const SearchArgs &A, int root, bool act,
+                                            int i, const double4 &pi, double ri,
+                                            HSums<R> *hs = nullptr) {
     typedef typename R4<R>::T V4;
     const int lane = threadIdx.x & 31;
+    constexpr int SW = 32 / SPLIT;  // staged candidates per lane of a chunk
+    const int sl = lane & (SPLIT - 1), k0 = sl * SW;
     const unsigned lt = (1u << lane) - 1u;
     const double gx0 = wmin(act ? pi.x : INFINITY), gy0 = wmin(act ? pi.y : INFINITY),
                  gz0 = wmin(act ? pi.z : INFINITY);
@@ -173,7 +182,7 @@ __device__ __forceinline__ void group_search(SearchSmem &S, const SearchArgs &A,
     double hnb = 0.0;
     int sp = 1, nflat = 0, nr = 0;
     bool overflow = false;
-    if (lane == 0) S.stk[0] = A.croot[A.gcloud[g]];
+    if (lane == 0) S.stk[0] = root;
     __syncwarp();
 
     // FP32 prefilter: distances relative to the group's centre, compared
@@ -231,9 +240,9 @@ __device__ __forceinline__ void group_search(SearchSmem &S, const SearchArgs &A,
                 S.fh[lane] = (float)q.w;
             }
             if (MODE == 0 && !FAST) S.smass[lane] = (double)((const V4 *)A.p1)[j].w;
-        } else if (lane < ((m + 3) & ~3)) {
-            // the tail of a chunk up to a multiple of four: entries that
-            // never pass
+        } else if (SPLIT > 1 || lane < ((m + 3) & ~3)) {
+            // the tail of a chunk (up to a multiple of four where one lane
+            // takes them all): entries that never pass
             S.fx[lane] = S.fy[lane] = S.fz[lane] = INFINITY;
             S.fh[lane] = 0.f;
         }
@@ -262,7 +271,7 @@ __device__ __forceinline__ void group_search(SearchSmem &S, const SearchArgs &A,
             if ((reinterpret_cast<uintptr_t>(S.fx) & 15u) == 0) {
                 // four candidates per 128-bit shared load
 #pragma unroll 2
-                for (int k = 0; k < m4; k += 4) {
+                for (int k = SPLIT > 1 ? k0 : 0; k < (SPLIT > 1 ? k0 + SW : m4); k += 4) {
                     const float4 X = ldf4(&S.fx[k]), Y = ldf4(&S.fy[k]), Z = ldf4(&S.fz[k]);
                     const float4 H = MODE == 1 ? ldf4(&S.fh[k]) : X;
                     pair(lo2(X), lo2(Y), lo2(Z), lo2(H));
@@ -271,23 +280,96 @@ __device__ __forceinline__ void group_search(SearchSmem &S, const SearchArgs &A,
             } else {
                 // (a shared array placed on an 8-byte boundary only)
 #pragma unroll 4
-                for (int k = 0; k < m4; k += 2)
+                for (int k = SPLIT > 1 ? k0 : 0; k < (SPLIT > 1 ? k0 + SW : m4); k += 2)
                     pair(ldf2(&S.fx[k]), ldf2(&S.fy[k]), ldf2(&S.fz[k]),
                          MODE == 1 ? ldf2(&S.fh[k]) : bc2(0.f));
             }
             // candidate k's sign bit is at bit m4 - 1 - k (m4 = m rounded up
             // to a multiple of four, 4..32; the padding entries never pass)
-            hit = (__brev(acc) >> (32 - m4)) & (0xffffffffu >> (32 - m4));
+            // (SPLIT > 1: candidate k0 + q at bit q)
+            const int sh = SPLIT > 1 ? 32 - SW : 32 - m4;
+            hit = (__brev(acc) >> sh) & (0xffffffffu >> sh);
         }
         R cs = R(0), cd = R(0);
-        if (FAST) {
+        auto exact_in = [&](int k) {
+            const double4 pj = S.stage[k];
+            const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+            return dx * dx + dy * dy + dz * dz <= ri2;
+        };
+        if constexpr (SPLIT > 1) {
+            // the lane's hits, exactly; their places in the row follow those
+            // of the particle's lower lanes.  A candidate inside the FP32
+            // threshold narrowed by the margin is inside in FP64 too, so the
+            // long FP64 chain runs for the few near the threshold only.
+            unsigned ok = 0;
+            for (unsigned hh = hit; hh; hh &= hh - 1) {
+                const int q = __ffs(hh) - 1, k = k0 + q;
+                const float ax = pfx.x - S.fx[k], ay = pfy.x - S.fy[k], az = pfz.x - S.fz[k];
+                float in2 = ri2lo.x;
+                if (MODE == 1) {
+                    const float sh = hif.x + S.fh[k];
+                    in2 = sh * sh * (1.f - mrg);
+                }
+                bool in = fmaf(az, az, fmaf(ay, ay, ax * ax)) <= in2;
+                if (!in) {
+                    const double4 pj = S.stage[k];
+                    in = MODE == 1 ? ngb_pred(pi.x, pi.y, pi.z, pi.w, pj.x, pj.y, pj.z, pj.w)
+                                   : exact_in(k);
+                }
+                if (in) ok |= 1u << q;
+            }
+            const int c = __popc(ok);
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < SPLIT; o <<= 1) {
+                const int t = __shfl_up_sync(FULL, incl, o, SPLIT);
+                if (sl >= o) incl += t;
+            }
+            int pos = count + incl - c;
+            count += __shfl_sync(FULL, incl, SPLIT - 1, SPLIT);
+            // four hits per trip: independent chains of dependent arithmetic
+            while (ok) {
+                int k[4];
+                R wt[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const bool any = ok != 0;
+                    k[q] = any ? k0 + __ffs(ok) - 1 : k[0];
+                    ok &= ok - 1;
+                    wt[q] = R(0);
+                    if (any) {
+                        if (MODE == 1) {
+                            if (pos < K) A.rows[(size_t)i * K + pos] = S.flat[k[q]];
+                            hnb = fmax(hnb, S.stage[k[q]].w);
+                        } else {
+                            if (pos < K) A.cidx[cbase + pos] = S.flat[k[q]];
+                            if (MODE == 0) wt[q] = FAST ? (R)S.fh[k[q]] : (R)S.smass[k[q]];
+                        }
+                        pos++;
+                    }
+                }
+                if (MODE == 0) {
+                    R w[4], dw[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        R r;
+                        if (FAST) {
+                            const float ax = pfx.x - S.fx[k[q]], ay = pfy.x - S.fy[k[q]],
+                                        az = pfz.x - S.fz[k[q]];
+                            const float r2 = fmaf(az, az, fmaf(ay, ay, ax * ax));
+                            r = r2 * rsqrtf(r2 + 1e-30f);
+                        } else {
+                            r = pair_r<R>(pi, S.stage[k[q]]);
+                        }
+                        hs->terms(r, w[q], dw[q]);
+                    }
+                    cs += (wt[0] * w[0] + wt[1] * w[1]) + (wt[2] * w[2] + wt[3] * w[3]);
+                    cd += (wt[0] * dw[0] + wt[1] * dw[1]) + (wt[2] * dw[2] + wt[3] * dw[3]);
+                }
+            }
+        } else if (FAST) {
             // two hits per trip (independent chains for the scheduler), the
             // sums and the row entries in the same order as one per trip
-            auto exact_in = [&](int k) {
-                const double4 pj = S.stage[k];
-                const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-                return dx * dx + dy * dy + dz * dz <= ri2;
-            };
             while (hit) {
                 const int k1 = __ffs(hit) - 1;
                 hit &= hit - 1;
@@ -323,7 +405,7 @@ __device__ __forceinline__ void group_search(SearchSmem &S, const SearchArgs &A,
                 }
             }
         }
-        while (!FAST && hit) {
+        while (SPLIT == 1 && !FAST && hit) {
             const int k = __ffs(hit) - 1;
             hit &= hit - 1;
             const double4 pj = S.stage[k];
@@ -344,7 +426,7 @@ __device__ __forceinline__ void group_search(SearchSmem &S, const SearchArgs &A,
                 }
             }
         }
-        if (FAST) {
+        if (FAST || (MODE == 0 && SPLIT > 1)) {
             hs->S.add(cs);
             hs->D.add(cd);
         }
@@ -448,7 +530,9 @@ __device__ __forceinline__ void group_search(SearchSmem &S, const SearchArgs &A,
             nr = 0;
         }
     }
-    if (act) {
+    if (MODE == 1 && SPLIT > 1)
+        for (int o = SPLIT / 2; o; o >>= 1) hnb = fmax(hnb, __shfl_xor_sync(FULL, hnb, o));
+    if (act && sl == 0) {
         if (MODE != 1) {
             // the full count: the Newton step shrinks the gather radius of a
             // row that did not fit instead of iterating on a truncated one
@@ -461,26 +545,46 @@ __device__ __forceinline__ void group_search(SearchSmem &S, const SearchArgs &A,
     }
     if (overflow && lane == 0) status_add(A.status, SPH_S_STACK_OVERFLOW, 1);
     __syncwarp();
+    return count;
 }
 
+// The unit of work of a warp: 1 / SPLIT of a group, 32 / SPLIT particles with
+// SPLIT lanes each.  A group's search is one long chain (tree rounds, then the
+// hits of its busiest lane, chunk by chunk), so a small cloud is bound by the
+// length of that chain on a few warps: with SPLIT lanes per particle the chain
+// of hits is SPLIT times shorter and SPLIT times as many warps run.  The tree
+// walk is repeated by each unit, so a cloud that fills the chip keeps SPLIT 1.
+template <int SPLIT> struct Unit {
+    int g, s0, gc, i;
+    bool in;
+    __device__ __forceinline__ Unit(const SearchArgs &A, int item) {
+        constexpr int PW = 32 / SPLIT;
+        const int part = item & (SPLIT - 1);
+        g = item / SPLIT;
+        s0 = A.gstart[g] + part * PW;
+        gc = min(A.gcount[g] - part * PW, PW);
+        const int p = (threadIdx.x & 31) / SPLIT;
+        in = p < gc;
+        i = in ? s0 + p : A.gstart[g];
+    }
+};
+
 // exact lists for every particle
+template <int SPLIT>
 __global__ void __launch_bounds__(SEARCH_WARPS * 32)
     k_lists(const int *__restrict__ ngroup_p, SearchArgs A, unsigned *queue) {
     __shared__ SearchSmem smem[SEARCH_WARPS];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ngroup = *ngroup_p;
+    const int w = threadIdx.x >> 5;
+    const int nunit = *ngroup_p * SPLIT;
     if (A.mlist && !*A.only_all) return;  // the listed particles: k_lists_list
-    for (int g = q_first(queue, blockIdx.x * SEARCH_WARPS + w); g < ngroup;
-         g = q_next(queue, g, gridDim.x * SEARCH_WARPS)) {
-        const int s0 = A.gstart[g], gc = A.gcount[g];
-        bool act = lane < gc;
-        const int i = s0 + (act ? lane : 0);
-        if (A.only && !*A.only_all) {
-            act = act && A.only[i];
-            if (!__any_sync(FULL, act)) continue;
-        }
-        const double4 pi = A.p0[i];
-        group_search<1>(smem[w], A, g, act, i, pi, pi.w);
+    for (int it = q_first(queue, blockIdx.x * SEARCH_WARPS + w); it < nunit;
+         it = q_next(queue, it, gridDim.x * SEARCH_WARPS)) {
+        const Unit<SPLIT> u(A, it);
+        bool act = u.in;
+        if (A.only && !*A.only_all) act = act && A.only[u.i];
+        if (!__any_sync(FULL, act)) continue;
+        const double4 pi = A.p0[u.i];
+        group_search<1, double, SPLIT>(smem[w], A, A.croot[A.gcloud[u.g]], act, u.i, pi, pi.w);
     }
 }
 
@@ -503,7 +607,7 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32)
             else hi = mid - 1;
         }
         const double4 pi = A.p0[i];
-        group_search<1>(smem[w], A, lo, lane == 0, i, pi, pi.w);
+        group_search<1>(smem[w], A, A.croot[A.gcloud[lo]], lane == 0, i, pi, pi.w);
     }
 }
 
@@ -745,70 +849,141 @@ struct NewtonArgs {
     int *kept;       // count of the particles that kept their row (null: not counted)
     int *retry;
     double n_ngb, tol, grow, regrow;
-    int max_iter, last_round;
+    int max_iter, rounds;
 };
 
-// Newton iteration of the particle of every active lane, FP32 or FP64 kernel
-// sums with FP64 update and convergence test.  The first evaluation (at
+// Kernel sums of the rows of the particles of mask m (one lane each, holding
+// the particle i, its trial h and its row's length c), L lanes per row over
+// interleaved entries and 32 / L rows at a time, each row's sums handed to its
+// particle's lane.  The whole warp calls.  One lane per row took as long as
+// the row whatever the number of rows; the first Newton evaluation, which the
+// search leaves, is enough for all but a few particles of a settled step.
+template <class R, int L, int U>
+__device__ __forceinline__ void row_sums(const SearchArgs &A, const NewtonArgs &B, unsigned m,
+                                         int i, double h, int c, double &Ss, double &Ds) {
+    typedef typename R4<R>::T V4;
+    constexpr int NR = 32 / L;
+    const int lane = threadIdx.x & 31, q = lane / L, sl = lane & (L - 1);
+    while (m) {
+        unsigned t = m;
+        for (int x = 0; x < q; x++) t &= t - 1;
+        const int src = t ? __ffs(t) - 1 : lane;
+        const int ii = __shfl_sync(FULL, i, src), cc = __shfl_sync(FULL, c, src);
+        const double hh = __shfl_sync(FULL, h, src);
+        HSums<R> hk;
+        hk.inv_h = R(1.0 / hh);
+        if (t) {
+            const double4 pp = A.p0[ii];
+            const int *rw = A.cidx + (size_t)ii * A.K;
+            // U entries per trip, their loads and their chains of arithmetic
+            // side by side (an entry alone waits for two loads in turn)
+            for (int k = sl; k < cc; k += U * L) {
+                int j[U];
+                R r[U], m[U];
+#pragma unroll
+                for (int x = 0; x < U; x++) j[x] = k + x * L < cc ? rw[k + x * L] : -1;
+#pragma unroll
+                for (int x = 0; x < U; x++) {
+                    r[x] = R(0);
+                    m[x] = R(0);
+                    if (j[x] >= 0) {
+                        r[x] = pair_r<R>(pp, A.p0[j[x]]);
+                        m[x] = (R)((const V4 *)B.p1)[j[x]].w;
+                    }
+                }
+#pragma unroll
+                for (int x = 0; x < U; x++) {
+                    R w, dw;
+                    hk.terms(r[x], w, dw);
+                    hk.S.add(m[x] * w);
+                    hk.D.add(m[x] * dw);
+                }
+            }
+        }
+        const double sS = seg_sum<L>(hk.S.value()), sD = seg_sum<L>(hk.D.value());
+        const int rank = __popc(m & ((1u << lane) - 1u));
+        const double tS = __shfl_sync(FULL, sS, (rank * L) & 31),
+                     tD = __shfl_sync(FULL, sD, (rank * L) & 31);
+        if ((m >> lane & 1u) && rank < NR) {
+            Ss = tS;
+            Ds = tD;
+        }
+        for (int x = 0; x < NR; x++) m &= m - 1;
+    }
+}
+
+// sums at h of the particles with want set, on every lane of the particle
+template <class R, int SPLIT>
+__device__ __forceinline__ void eval_rows(const SearchArgs &A, const NewtonArgs &B, bool want, int i,
+                                          double h, int c, double &Ss, double &Ds) {
+    const int lane = threadIdx.x & 31;
+    const unsigned m = __ballot_sync(FULL, want && (lane & (SPLIT - 1)) == 0);
+    if (!m) return;
+    constexpr int U = SPLIT > 1 ? 4 : 2;
+    if (__popc(m) <= 4) row_sums<R, 16, U>(A, B, m, i, h, c, Ss, Ds);
+    else row_sums<R, 4, U>(A, B, m, i, h, c, Ss, Ds);
+    if (SPLIT > 1) {
+        Ss = __shfl_sync(FULL, Ss, lane & ~(SPLIT - 1));
+        Ds = __shfl_sync(FULL, Ds, lane & ~(SPLIT - 1));
+    }
+}
+
+// Newton iteration of the particles of every lane with run set, FP32 or FP64
+// kernel sums with FP64 update and convergence test.  The first evaluation (at
 // h = pi.w), S0 and D0, comes from the search (searched) or from the kept
 // row; later ones, rare once h has settled from step to step, gather the
-// candidates again through the particle's slot row in the same order, so
-// they sum the same terms in the same order.  No warp collectives: lanes run
-// independent iteration counts.
-template <class R>
-__device__ __forceinline__ void newton_lane(const SearchArgs &A, const NewtonArgs &B, int i,
-                                            const double4 &pi, const int *row, double S0,
-                                            double D0, bool searched) {
+// candidates again through the particle's slot row.  Every lane of the warp
+// calls; the SPLIT lanes of a particle run the same iteration and the first
+// of them writes.  pi.w and hc (the candidate radius / 2) are updated; returns
+// whether the particle has to be searched again.
+template <class R, int SPLIT>
+__device__ __forceinline__ bool newton_rows(const SearchArgs &A, const NewtonArgs &B, bool run,
+                                            int i, double4 &pi, double &hc, int craw, double S0,
+                                            double D0, bool searched, bool last_round) {
     typedef typename R4<R>::T V4;
     const V4 *p1 = (const V4 *)B.p1;
-    const int craw = A.cnt[i];
-    if (searched) B.hsr[i] = craw > A.K ? 0.0 : B.hc[i];
-    if (craw > A.K) {
+    const bool own = (threadIdx.x & (SPLIT - 1)) == 0;
+    bool again = false;
+    bool live = run;
+    if (run && searched && own) B.hsr[i] = craw > A.K ? 0.0 : hc;
+    if (run && craw > A.K) {
         // more candidates inside 2 hc than the row holds: the sums would miss
         // some, so remember that radius, shrink hc towards a three-quarter
         // full row and search again; h restarts at most just below the new
         // radius
-        if (!B.last_round) {
-            B.hover[i] = fmin(B.hover[i], B.hc[i]);
-            const double hc = B.hc[i] * fmax(0.5, cbrt(0.75 * A.K / (double)craw));
-            const double h0 = fmin(pi.w, hc / B.grow);
-            B.hc[i] = hc;
-            B.retry[i] = 1;
-            B.h_out[i] = h0;
-            A.p0[i].w = h0;
-            status_add(A.status, SPH_S_H_RETRY, 1);
-        } else {
-            B.retry[i] = 0;
+        live = false;
+        if (!last_round) {
+            if (own) {
+                B.hover[i] = fmin(B.hover[i], hc);
+                status_add(A.status, SPH_S_H_RETRY, 1);
+            }
+            hc = hc * fmax(0.5, cbrt(0.75 * A.K / (double)craw));
+            pi.w = fmin(pi.w, hc / B.grow);
+            again = true;
+            if (own) {
+                B.h_out[i] = pi.w;
+                A.p0[i].w = pi.w;
+            }
+        } else if (own) {
             status_add(A.status, SPH_S_NGB_OVERFLOW, 1);
             status_add(A.status, SPH_S_H_NOCONV, 1);
         }
-        return;
     }
-    const int c = craw;
+    const bool iterated = live;
     const double mi = (double)p1[i].w;
-    const double cap = B.hc[i];
+    const double cap = hc;
     const double cfac = 4.0 * SPH_PI / 3.0 * 8.0;
     double h = pi.w, lo = 0.0, hi = INFINITY;
     bool ok = false, need = false;
+    double Ssum = S0, Dsum = D0;
     for (int it = 1; it <= B.max_iter; it++) {
-        if (h > cap) {  // 2h would pass the candidate radius 2*cap
+        if (live && h > cap) {  // 2h would pass the candidate radius 2*cap
             need = true;
-            break;
+            live = false;
         }
-        double Ssum, Dsum;
-        if (it == 1) {
-            Ssum = S0;
-            Dsum = D0;
-        } else {
-            HSums<R> hs;
-            hs.inv_h = R(1.0 / h);
-            for (int k = 0; k < c; k++) {
-                const int j = row[k];
-                hs.add(pair_r<R>(pi, A.p0[j]), (R)(double)p1[j].w);
-            }
-            Ssum = hs.S.value();
-            Dsum = hs.D.value();
-        }
+        if (!__any_sync(FULL, live)) break;
+        if (it > 1) eval_rows<R, SPLIT>(A, B, live, i, h, craw, Ssum, Dsum);
+        if (!live) continue;
         const double h3 = h * h * h;
         const double rho = SPH_SIG / h3 * Ssum;
         const double drho = -SPH_SIG / (h3 * h) * Dsum;
@@ -823,7 +998,8 @@ __device__ __forceinline__ void newton_lane(const SearchArgs &A, const NewtonArg
             h = hn;
             if (h > cap) need = true;
             else ok = true;
-            break;
+            live = false;
+            continue;
         }
         // at most a factor 1.25 per iteration (keeps retries inside the rows)
         if (hn > 1.25 * h) hn = 1.25 * h;
@@ -847,89 +1023,65 @@ __device__ __forceinline__ void newton_lane(const SearchArgs &A, const NewtonArg
         if (!clamped && fabs(dh) < B.tol * fabs(h - dh)) {
             if (h > cap) need = true;
             else ok = true;
-            break;
+            live = false;
         }
     }
-    if (need && !B.last_round) {
+    if (!iterated) return again;
+    if (need && !last_round) {
         // a wider search, kept below a radius whose row already overflowed;
         // a kept row that h outgrew is searched at the usual radius
         const double ov = B.hover[i];
         const double g = searched ? h * B.regrow : cand_half_radius(h, B.hnb[i], B.grow);
-        B.hc[i] = h < ov ? fmin(g, h + 0.5 * (ov - h)) : g;
-        B.retry[i] = 1;
-    } else {
-        B.retry[i] = 0;
-        if (!ok) status_add(A.status, SPH_S_H_NOCONV, 1);
+        hc = h < ov ? fmin(g, h + 0.5 * (ov - h)) : g;
+        again = true;
+    } else if (!ok && own) {
+        status_add(A.status, SPH_S_H_NOCONV, 1);
     }
-    if (need) status_add(A.status, SPH_S_H_RETRY, 1);
-    B.h_out[i] = h;
-    A.p0[i].w = h;  // p0 is written only by the lane owning particle i
+    pi.w = h;
+    if (own) {
+        if (need) status_add(A.status, SPH_S_H_RETRY, 1);
+        B.h_out[i] = h;
+        A.p0[i].w = h;  // p0 is written only by the lane owning particle i
+    }
+    return again;
 }
 
-// the first Newton evaluation of the kept rows of a group: four lanes per
-// row over interleaved entries (terms beyond 2 h are zero), eight rows at a
-// time, each row's sums handed to the lane of its particle
-template <class R>
-__device__ __forceinline__ void kept_sums(const SearchArgs &A, const NewtonArgs &B, int s0, int gc,
-                                       double &S0, double &D0) {
-    typedef typename R4<R>::T V4;
-    const int lane = threadIdx.x & 31, q = lane >> 2, sl = lane & 3;
-    S0 = 0.0;
-    D0 = 0.0;
-    for (int p = 0; p < gc; p += 8) {
-        HSums<R> hk;
-        hk.inv_h = R(1);
-        if (p + q < gc) {
-            const int ii = s0 + p + q;
-            const double4 pp = A.p0[ii];
-            hk.inv_h = R(1.0 / pp.w);
-            const int c = A.cnt[ii];
-            const int *rw = A.cidx + (size_t)ii * A.K;
-            for (int k = sl; k < c; k += 4) {
-                const int j = rw[k];
-                hk.add(pair_r<R>(pp, A.p0[j]), (R)(double)((const V4 *)B.p1)[j].w);
-            }
-        }
-        const double sS = seg_sum<4>(hk.S.value()), sD = seg_sum<4>(hk.D.value());
-        const int src = ((lane - p) & 7) * 4;
-        const double tS = __shfl_sync(FULL, sS, src), tD = __shfl_sync(FULL, sD, src);
-        if (lane >= p && lane < p + 8) {
-            S0 = tS;
-            D0 = tD;
-        }
-    }
-}
-
-// candidate search + Newton iteration for the flagged particles of each group
-// (retry 1), and in the first round the Newton iteration from the kept rows
-// (retry 2 and 3) in the same warps, so both share the persistent grid that
-// runs beside the gravity walk (latency-bound: 8 blocks per SM, 64
-// registers, measured faster than 95)
-template <class R>
-__global__ void __launch_bounds__(SEARCH_WARPS * 32, 8)
+// Candidate search + Newton iteration of each unit's particles: the first
+// round for the flagged ones (retry 1) and from the kept rows (retry 2 and 3),
+// then the particles whose h left their candidate radius again, at most
+// `rounds` times.  A particle's rounds depend on no other particle's h, so a
+// warp finishes its unit at once: a launch per round cost a pass over all
+// groups and a tail of half-empty SMs each (8 rounds of 100k particles 732 us,
+// here 448 with the rows re-read by four lanes; the three empty rounds of a
+// 10k step 25 us).  Latency-bound: at SPLIT 1 8 blocks per SM, 64 registers,
+// measured faster than 95; a split cloud fills fewer blocks and takes the
+// registers for the unrolled chains instead.
+template <class R, int SPLIT>
+__global__ void __launch_bounds__(SEARCH_WARPS * 32, SPLIT > 1 ? 4 : 8)
     k_cand_newton(const int *__restrict__ ngroup_p, SearchArgs A, NewtonArgs B, unsigned *queue) {
-    typedef typename R4<R>::T V4;
     __shared__ SearchSmem smem[SEARCH_WARPS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ngroup = *ngroup_p;
-    for (int g = q_first(queue, blockIdx.x * SEARCH_WARPS + w); g < ngroup;
-         g = q_next(queue, g, gridDim.x * SEARCH_WARPS)) {
-        const int s0 = A.gstart[g], gc = A.gcount[g];
-        const bool in = lane < gc;
-        const int i = s0 + (in ? lane : 0);
-        const int rt = in ? B.retry[i] : 0;
-        const double4 pi = A.p0[i];
-        // a group keeps its rows only as a whole: a lane gathering its row
+    const int nunit = *ngroup_p * SPLIT;
+    const bool own = (lane & (SPLIT - 1)) == 0;
+    for (int item = q_first(queue, blockIdx.x * SEARCH_WARPS + w); item < nunit;
+         item = q_next(queue, item, gridDim.x * SEARCH_WARPS)) {
+        const Unit<SPLIT> u(A, item);
+        const int i = u.i;
+        const int rt = u.in ? B.retry[i] : 0;
+        double4 pi = A.p0[i];
+        // a unit keeps its rows only as a whole: a lane gathering its row
         // alone would hold up the warp's search for the others
         bool part = __any_sync(FULL, rt == 1);
+        double hci = B.hc[i];
+        const int root = A.croot[A.gcloud[u.g]];
         if (!part && __any_sync(FULL, rt == 3)) {
-            // the moves of the particles near the group decide: M, bounded
+            // the moves of the particles near the unit decide: M, bounded
             // over the tree nodes within the largest kept radius of the
-            // group's box, must leave each lane's row the radius it needs
+            // unit's box, must leave each lane's row the radius it needs
             const bool l3 = rt == 3;
-            const double hs = l3 ? B.hsr[i] : 0.0, own = l3 ? B.dmv[i] : 0.0;
+            const double hs = l3 ? B.hsr[i] : 0.0, own_mv = l3 ? B.dmv[i] : 0.0;
             const double lim =
-                l3 ? 2.0 * (hs - reuse_need(pi.w, B.hnb[i]) / (1.0 - 1e-12)) - own : INFINITY;
+                l3 ? 2.0 * (hs - reuse_need(pi.w, B.hnb[i]) / (1.0 - 1e-12)) - own_mv : INFINITY;
             const float flim = __double2float_rd(wmin(lim));
             const float fgx0 = __double2float_rd(wmin(l3 ? pi.x : INFINITY)),
                         fgy0 = __double2float_rd(wmin(l3 ? pi.y : INFINITY)),
@@ -938,57 +1090,60 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, 8)
                         fgy1 = __double2float_ru(wmax(l3 ? pi.y : -INFINITY)),
                         fgz1 = __double2float_ru(wmax(l3 ? pi.z : -INFINITY));
             const float frmax = __double2float_ru(wmax(2.0 * hs));
-            const float M = flim >= 0.f ? moved_near(smem[w], A, A.croot[A.gcloud[g]], fgx0, fgy0,
-                                                     fgz0, fgx1, fgy1, fgz1, frmax, flim, B.gdm)
+            const float M = flim >= 0.f ? moved_near(smem[w], A, root, fgx0, fgy0, fgz0, fgx1, fgy1,
+                                                     fgz1, frmax, flim, B.gdm)
                                         : INFINITY;
             if (M <= flim) {
-                if (l3) B.hc[i] = (hs - 0.5 * (own + (double)M)) * (1.0 - 1e-12);
+                if (l3) hci = (hs - 0.5 * (own_mv + (double)M)) * (1.0 - 1e-12);
             } else {
                 part = true;
             }
         }
-        const bool act = rt == 1 || (rt >= 2 && part), keep = rt >= 2 && !part;
-        const unsigned todo = __ballot_sync(FULL, act);
-        const unsigned km = __ballot_sync(FULL, keep);
-        if (!todo && !km) continue;
+        bool act = rt == 1 || (rt >= 2 && part);
+        const bool keep = rt >= 2 && !part;
+        const unsigned km = __ballot_sync(FULL, keep && own);
         if (km && lane == 0 && B.kept) atomicAdd(B.kept, __popc(km));
-        const int *row = A.cidx + (size_t)i * A.K;
-        double hci = act ? B.hc[i] : 0.0;
-        if (rt >= 2 && part) {
-            // searched after all, at the usual radius
-            hci = cand_half_radius(pi.w, B.hnb[i], B.grow);
+        // searched after all, at the usual radius
+        if (rt >= 2 && part) hci = cand_half_radius(pi.w, B.hnb[i], B.grow);
+        for (int round = 0; round < B.rounds; round++) {
+            const bool first_keep = km && round == 0;
+            const bool any = __any_sync(FULL, act);
+            if (!any && !first_keep) break;
+            int craw = 0;
+            double S0 = 0.0, D0 = 0.0;
+            bool run = act;
+            if (any) {
+                HSums<R> hs;
+                hs.inv_h = R(1.0 / pi.w);
+                craw = group_search<0, R, SPLIT>(smem[w], A, root, act, i, pi, 2.0 * hci, &hs);
+                S0 = hs.S.value();
+                D0 = hs.D.value();
+                if (SPLIT > 1) {
+                    S0 = seg_sum<SPLIT>(S0);
+                    D0 = seg_sum<SPLIT>(D0);
+                }
+            } else {
+                // the unit kept its rows (no lane searches)
+                if (keep) craw = A.cnt[i];
+                eval_rows<R, SPLIT>(A, B, keep, i, pi.w, craw, S0, D0);
+                run = keep;
+            }
+            act = newton_rows<R, SPLIT>(A, B, run, i, pi, hci, craw, S0, D0, any,
+                                        round == B.rounds - 1);
+            __syncwarp();
+        }
+        if (u.in && own && rt) {
             B.hc[i] = hci;
-        }
-        HSums<R> hs;
-        hs.inv_h = R(1.0 / pi.w);
-        if (todo) group_search<0, R>(smem[w], A, g, act, i, pi, 2.0 * hci, &hs);
-        if (act) {
-            // each lane reads back only the row entries it wrote itself
-            newton_lane<R>(A, B, i, pi, row, hs.S.value(), hs.D.value(), true);
-        }
-        if (km) {
-            // the group kept its rows (first round only; no lane searches)
-            double S0, D0;
-            kept_sums<R>(A, B, s0, gc, S0, D0);
-            if (keep) newton_lane<R>(A, B, i, pi, row, S0, D0, false);
+            B.retry[i] = 0;
         }
         __syncwarp();
     }
 }
 
-// The reference's count iteration (h_smooth_fast_mpi, MPI_sph/sph_code/
-// libsx.py:854-902) for the particle of one lane: with d_j = |r_j - r_i|
-// (self included) and n(h) = #{j : d_j < 2 h}, h <- h - f h while n(h) > hi_n
-// and h <- h + f h while n(h) < lo_n.  Its only state is h, so a particle
-// whose 2 h would pass its candidate radius 2 hc stops, stores h and
-// resumes in the next round with a wider radius: the sequence of h is that
-// of one uninterrupted iteration.  d_j is rounded as the reference writes it
-// (dx = x_j - x_i, dx dx + dy dy, + dz dz, correctly rounded square root),
-// so the result is bit-exact with it on the same positions.
 struct CountArgs {
     double *h_out, *hc;
-    int *retry, *iters;
-    int lo_n, hi_n, max_iter, last_round;
+    int *retry;
+    int lo_n, hi_n, max_iter, rounds;
     double frac, grow;
 };
 
@@ -997,17 +1152,77 @@ __device__ __forceinline__ double ref_dist(const double4 &pi, const double4 &pj)
     return __dsqrt_rn(xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz)));
 }
 
-__device__ __forceinline__ void count_lane(const SearchArgs &A, const CountArgs &B, int i,
-                                           const double4 &pi, const int *row) {
-    const int craw = A.cnt[i];
-    double h = pi.w;
-    int it = B.iters[i];
-    const double cap = B.hc[i];
+// The distances of one particle's row, entry 32 e + lane in d[e] (infinity past
+// the row's c <= 512 entries): each row is gathered once, by the whole warp.
+constexpr int SEL_MAX = 16;
+struct RowDist {
+    double d[SEL_MAX];
+    int c;
+    __device__ __forceinline__ RowDist(const SearchArgs &A, int i, const double4 &pi, int craw)
+        : c(craw) {
+        const int lane = threadIdx.x & 31;
+        const int *row = A.cidx + (size_t)i * A.K;
+#pragma unroll
+        for (int e = 0; e < SEL_MAX; e++) {
+            d[e] = INFINITY;
+            if (32 * e < c && 32 * e + lane < c) d[e] = ref_dist(pi, A.p0[row[32 * e + lane]]);
+        }
+    }
+    // the k-th smallest distance (k = 1 the smallest), infinity when the row
+    // has fewer; every distance is at most `bound`.  Bisection between 0 and the
+    // bound until a trial value has k or k - 1 distances at or below it, which
+    // names the k-th; equal distances never separate, so the interval also
+    // shrinks by at least one bit pattern a trial (non-negative doubles order
+    // like their patterns) down to the value itself.
+    __device__ __forceinline__ double kth(int k, double bound) const {
+        if (c < k) return INFINITY;
+        unsigned long long lo = 0ull, hi = (unsigned long long)__double_as_longlong(bound);
+        while (lo < hi) {
+            const double a = __longlong_as_double((long long)lo), b = __longlong_as_double((long long)hi);
+            unsigned long long mid = (unsigned long long)__double_as_longlong(0.5 * (a + b));
+            mid = mid < lo ? lo : (mid >= hi ? hi - 1 : mid);
+            const double v = __longlong_as_double((long long)mid);
+            int n = 0;
+            double below = 0.0, above = INFINITY;
+#pragma unroll
+            for (int e = 0; e < SEL_MAX; e++) {
+                if (32 * e < c) {
+                    const bool in = d[e] <= v;
+                    n += __popc(__ballot_sync(FULL, in));
+                    if (in) below = fmax(below, d[e]);
+                    else above = fmin(above, d[e]);
+                }
+            }
+            if (n == k) return wmax(below);
+            if (n == k - 1) return wmin(above);
+            if (n > k) hi = mid;
+            else lo = mid + 1;
+        }
+        return __longlong_as_double((long long)lo);
+    }
+};
+
+// The reference's count iteration (h_smooth_fast_mpi, MPI_sph/sph_code/
+// libsx.py:854-902) for the particle of each lane: with d_j = |r_j - r_i|
+// (self included) and n(h) = #{j : d_j < 2 h}, h <- h - f h while n(h) > hi_n
+// and h <- h + f h while n(h) < lo_n.  d_j is rounded as the reference writes it
+// (dx = x_j - x_i, dx dx + dy dy, + dz dz, correctly rounded square root), so
+// the result is bit-exact with it on the same positions.
+// n(h) >= k exactly when the k-th smallest distance is below 2 h, so two order
+// statistics of the row decide every iteration: t_lo, the lo_n-th distance, and
+// t_hi, the (hi_n + 1)-th.  The iteration's only state is h, so a particle
+// whose 2 h would pass its candidate radius 2 hc stops and resumes after a
+// wider search: the sequence of h is that of one uninterrupted iteration.
+// Returns whether the particle has to be searched again.
+__device__ __forceinline__ bool count_lane(const SearchArgs &A, const CountArgs &B, bool own,
+                                           double &h, double &hc, int &it, int craw, double t_lo,
+                                           double t_hi, bool last_round) {
+    const double cap = hc;
     bool ok = false, done = false, again = false;
     if (craw > A.K) {
         // the row cannot hold every candidate: narrow the radius towards a
         // half-full row and search again
-        B.hc[i] = cap * fmax(0.5, cbrt(0.5 * A.K / (double)craw));
+        hc = cap * fmax(0.5, cbrt(0.5 * A.K / (double)craw));
         again = true;
     } else {
         // every j with d_j < 2 lim is in the row: the search's r^2 test is
@@ -1016,10 +1231,7 @@ __device__ __forceinline__ void count_lane(const SearchArgs &A, const CountArgs 
         if (h > lim) {
             // h beyond the complete radius: n(h) >= n(lim), so while n(lim)
             // is above the window every decrement is the reference's own
-            const double l2 = 2.0 * lim;
-            int nin = 0;
-            for (int k = 0; k < craw; k++) nin += ref_dist(pi, A.p0[row[k]]) < l2;
-            if (nin > B.hi_n) {
+            if (t_hi < 2.0 * lim) {
                 while (h > lim) {
                     h = xsub(h, xmul(B.frac, h));
                     if (++it > B.max_iter) {
@@ -1028,17 +1240,14 @@ __device__ __forceinline__ void count_lane(const SearchArgs &A, const CountArgs 
                     }
                 }
             } else {
-                B.hc[i] = h * B.grow;  // too few inside: search wider
-                again = true;
+                again = true;  // too few inside: search wider
             }
         }
         while (!done && !again && h <= lim) {
             const double h2 = 2.0 * h;
-            int nn = 0;
-            for (int k = 0; k < craw; k++) nn += ref_dist(pi, A.p0[row[k]]) < h2;
-            if (nn > B.hi_n) {
+            if (t_hi < h2) {
                 h = xsub(h, xmul(B.frac, h));
-            } else if (nn < B.lo_n) {
+            } else if (!(t_lo < h2)) {
                 h = xadd(h, xmul(B.frac, h));
             } else {
                 ok = true;
@@ -1046,111 +1255,126 @@ __device__ __forceinline__ void count_lane(const SearchArgs &A, const CountArgs 
             }
             if (++it > B.max_iter) done = true;
         }
-        if (!ok && !done && !again) {
-            B.hc[i] = h * B.grow;  // h passed the radius: search again, wider
-            again = true;
-        }
+        if (!ok && !done && !again) again = true;  // h passed the radius
+        // the wider radius: past h, and past where a uniform density holds
+        // the window's count
+        if (again)
+            hc = fmax(h * B.grow, cap * fmin(1.5, cbrt(1.2 * (B.hi_n + 1) / (double)max(craw, 1))));
     }
-    if (again) status_add(A.status, SPH_S_H_RETRY, 1);
-    again = again && !B.last_round;
-    B.retry[i] = again ? 1 : 0;
-    if (!ok && !again) status_add(A.status, SPH_S_H_NOCONV, 1);
-    B.iters[i] = it;
-    B.h_out[i] = h;
-    A.p0[i].w = h;
+    if (again && own) status_add(A.status, SPH_S_H_RETRY, 1);
+    again = again && !last_round;
+    if (!ok && !again && own) status_add(A.status, SPH_S_H_NOCONV, 1);
+    return again;
 }
 
-// candidate search + count iteration for the flagged particles of each group
-__global__ void __launch_bounds__(SEARCH_WARPS * 32, 8)
+// Candidate search + count iteration of each unit's particles, at most
+// `rounds` searches per particle.  Each row is read once per search (RowDist);
+// one lane gathering its row in every iteration took 2.3 ms for the first
+// round of 30k particles and 3.7 ms in all (a launch per round), this 0.26 ms.
+template <int SPLIT>
+__global__ void __launch_bounds__(SEARCH_WARPS * 32, 4)
     k_cand_count(const int *__restrict__ ngroup_p, SearchArgs A, CountArgs B, unsigned *queue) {
     __shared__ SearchSmem smem[SEARCH_WARPS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ngroup = *ngroup_p;
-    for (int g = q_first(queue, blockIdx.x * SEARCH_WARPS + w); g < ngroup;
-         g = q_next(queue, g, gridDim.x * SEARCH_WARPS)) {
-        const int s0 = A.gstart[g], gc = A.gcount[g];
-        bool act = lane < gc;
-        const int i = s0 + (act ? lane : 0);
-        act = act && B.retry[i];
-        if (!__ballot_sync(FULL, act)) continue;
-        const double4 pi = A.p0[i];
-        group_search<2, double>(smem[w], A, g, act, i, pi, 2.0 * B.hc[i]);
-        if (act) count_lane(A, B, i, pi, A.cidx + (size_t)i * A.K);
+    const int nunit = *ngroup_p * SPLIT;
+    const bool own = (lane & (SPLIT - 1)) == 0;
+    for (int item = q_first(queue, blockIdx.x * SEARCH_WARPS + w); item < nunit;
+         item = q_next(queue, item, gridDim.x * SEARCH_WARPS)) {
+        const Unit<SPLIT> u(A, item);
+        const double4 pi = A.p0[u.i];
+        const int root = A.croot[A.gcloud[u.g]];
+        double h = pi.w, hc = B.hc[u.i];
+        int it = 0;
+        bool act = u.in;
+        for (int round = 0; round < B.rounds && __any_sync(FULL, act); round++) {
+            const int craw = group_search<2, double, SPLIT>(smem[w], A, root, act, u.i, pi, 2.0 * hc);
+            double t_lo = INFINITY, t_hi = INFINITY;
+            for (unsigned m = __ballot_sync(FULL, act && own && craw <= A.K); m; m &= m - 1) {
+                const int src = __ffs(m) - 1;
+                const int ii = __shfl_sync(FULL, u.i, src), cc = __shfl_sync(FULL, craw, src);
+                // every row entry lies within 2 hc up to the rounding of the
+                // search's r^2 test
+                const double bound = 2.0 * __shfl_sync(FULL, hc, src) * (1.0 + 1e-9);
+                const RowDist R(A, ii, A.p0[ii], cc);
+                const double a = R.kth(B.lo_n, bound), b = R.kth(B.hi_n + 1, bound);
+                if ((lane & ~(SPLIT - 1)) == src) {
+                    t_lo = a;
+                    t_hi = b;
+                }
+            }
+            if (act) act = count_lane(A, B, own, h, hc, it, craw, t_lo, t_hi, round == B.rounds - 1);
+        }
+        if (u.in && own) {
+            B.hc[u.i] = hc;
+            B.retry[u.i] = 0;
+            B.h_out[u.i] = h;
+            A.p0[u.i].w = h;
+        }
         __syncwarp();
     }
 }
 
-// Half the k-th smallest distance (self at index 0) of the particle of one
-// lane (smoothing_length_mpi, MPI_sph/sph_code/libsx.py:777-800: np.sort(dist)
-// [50] / 2).  With a complete row (every j with d_j <= 2 hc) holding at least
-// k + 1 entries, the k-th smallest distance overall is the row's; it is found
-// by bisection over the bit patterns of the row's distances (non-negative
-// doubles order like their patterns), so the value is one of the distances,
-// rounded as the reference computes them.  A row with too few entries widens
-// the radius, one that overflows narrows it, and the particle searches again.
-__device__ __forceinline__ void kth_lane(const SearchArgs &A, const CountArgs &B, int i,
-                                         const double4 &pi, const int *row, int k) {
-    const int craw = A.cnt[i];
-    const double cap = B.hc[i];
-    bool again = false;
-    if (craw > A.K) {
-        B.hc[i] = cap * fmax(0.5, cbrt(0.75 * A.K / (double)craw));
-        again = true;
-    } else if (craw < k + 1) {
-        B.hc[i] = cap * (craw > 0 ? fmin(2.0, fmax(1.1, cbrt(1.5 * (k + 1) / (double)craw))) : 2.0);
-        again = true;
-    } else {
-        // every row entry lies within 2 cap up to the rounding of the
-        // search's r^2 test; hi bounds them all
-        unsigned long long lo = 0,
-                           hi = (unsigned long long)__double_as_longlong(2.0 * cap * (1.0 + 1e-9));
-        for (int it = 0; it < 64 && lo < hi; it++) {
-            const unsigned long long mid = lo + (hi - lo) / 2;
-            const double v = __longlong_as_double((long long)mid);
-            int c = 0;
-            for (int q = 0; q < craw; q++) c += ref_dist(pi, A.p0[row[q]]) <= v;
-            if (c >= k + 1) hi = mid;
-            else lo = mid + 1;
-        }
-        const double d = __longlong_as_double((long long)lo);
-        if (d > 2.0 * cap * (1.0 - 1e-12)) {
-            // at the radius itself a particle outside the row could be nearer
-            // by a rounding: search again, wider
-            B.hc[i] = cap * 1.1;
-            again = true;
-        } else {
-            B.h_out[i] = 0.5 * d;
-            A.p0[i].w = 0.5 * d;
-        }
-    }
-    if (again) status_add(A.status, SPH_S_H_RETRY, 1);
-    const bool retry = again && !B.last_round;
-    B.retry[i] = retry ? 1 : 0;
-    if (again && !retry) status_add(A.status, SPH_S_H_NOCONV, 1);
-}
-
-__global__ void __launch_bounds__(SEARCH_WARPS * 32, 8)
+// Half the k-th smallest distance (self at index 0) of each unit's particles
+// (smoothing_length_mpi, MPI_sph/sph_code/libsx.py:777-800: np.sort(dist)[50] /
+// 2), rounded as the reference computes it.  With a complete row (every j with
+// d_j <= 2 hc) holding at least k + 1 entries, the (k + 1)-th smallest
+// distance overall is the row's.  A row with too few entries widens the
+// radius, one that overflows narrows it, and the particle searches again, at
+// most `rounds` times.
+template <int SPLIT>
+__global__ void __launch_bounds__(SEARCH_WARPS * 32, 4)
     k_cand_kth(const int *__restrict__ ngroup_p, SearchArgs A, CountArgs B, int k, unsigned *queue) {
     __shared__ SearchSmem smem[SEARCH_WARPS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ngroup = *ngroup_p;
-    for (int g = q_first(queue, blockIdx.x * SEARCH_WARPS + w); g < ngroup;
-         g = q_next(queue, g, gridDim.x * SEARCH_WARPS)) {
-        const int s0 = A.gstart[g], gc = A.gcount[g];
-        bool act = lane < gc;
-        const int i = s0 + (act ? lane : 0);
-        act = act && B.retry[i];
-        if (!__ballot_sync(FULL, act)) continue;
-        const double4 pi = A.p0[i];
-        group_search<2, double>(smem[w], A, g, act, i, pi, 2.0 * B.hc[i]);
-        if (act) kth_lane(A, B, i, pi, A.cidx + (size_t)i * A.K, k);
+    const int nunit = *ngroup_p * SPLIT;
+    const bool own = (lane & (SPLIT - 1)) == 0;
+    for (int item = q_first(queue, blockIdx.x * SEARCH_WARPS + w); item < nunit;
+         item = q_next(queue, item, gridDim.x * SEARCH_WARPS)) {
+        const Unit<SPLIT> u(A, item);
+        const double4 pi = A.p0[u.i];
+        const int root = A.croot[A.gcloud[u.g]];
+        double hc = B.hc[u.i];
+        bool act = u.in;
+        for (int round = 0; round < B.rounds && __any_sync(FULL, act); round++) {
+            const int craw = group_search<2, double, SPLIT>(smem[w], A, root, act, u.i, pi, 2.0 * hc);
+            double d = INFINITY;
+            for (unsigned m = __ballot_sync(FULL, act && own && craw <= A.K && craw > k); m; m &= m - 1) {
+                const int src = __ffs(m) - 1;
+                const int ii = __shfl_sync(FULL, u.i, src), cc = __shfl_sync(FULL, craw, src);
+                const double bound = 2.0 * __shfl_sync(FULL, hc, src) * (1.0 + 1e-9);
+                const RowDist R(A, ii, A.p0[ii], cc);
+                const double v = R.kth(k + 1, bound);
+                if ((lane & ~(SPLIT - 1)) == src) d = v;
+            }
+            if (!act) continue;
+            bool again = true;
+            if (craw > A.K) {
+                hc *= fmax(0.5, cbrt(0.75 * A.K / (double)craw));
+            } else if (craw < k + 1) {
+                hc *= craw > 0 ? fmin(2.0, fmax(1.1, cbrt(1.5 * (k + 1) / (double)craw))) : 2.0;
+            } else if (d > 2.0 * hc * (1.0 - 1e-12)) {
+                // at the radius itself a particle outside the row could be
+                // nearer by a rounding: search again, wider
+                hc *= 1.1;
+            } else {
+                again = false;
+                if (own) {
+                    B.h_out[u.i] = 0.5 * d;
+                    A.p0[u.i].w = 0.5 * d;
+                }
+            }
+            if (again && own) {
+                status_add(A.status, SPH_S_H_RETRY, 1);
+                if (round == B.rounds - 1) status_add(A.status, SPH_S_H_NOCONV, 1);
+            }
+            act = again;
+        }
+        if (u.in && own) {
+            B.hc[u.i] = hc;
+            B.retry[u.i] = 0;
+        }
         __syncwarp();
     }
-}
-
-__global__ void k_zero_int(int n, int *__restrict__ a) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = 0;
 }
 
 // canonical CSR export, each row sorted ascending
@@ -1197,6 +1421,44 @@ SearchArgs search_args(sph_ctx *ctx, int *rows, int *cnt) {
     return A;
 }
 
+// Lanes per particle of the searches: a cloud whose groups (about 20 particles
+// each) leave warps of the chip idle splits them (see Unit).  Measured with 1 /
+// 2 / 4 / 8 lanes, us, N particles of an Evrard sphere on 148 SMs:
+//   h iteration, settled, FP32:  2k 122 / 73 / 59 / 46;  10k 130 / 83 / 69 / 70;
+//     20k 136 / 97 / 101;  30k 150 / 113 / 123;  45k 160 / 151 / 165;
+//     60k 167 / 171 / 195;  100k 202 / 263 / 309
+//   the same in FP64:  10k 169 / 108 / 84 / 83;  45k 205 / 195 / 201;
+//     60k 208 / 219 / 244
+//   lists, tree search:  2k 64 / 56 / 44 / 34;  20k 77 / 70 / 59;
+//     60k 100 / 107 / 114
+//   count iteration:  2k 219 / 160 / 97 / 67;  30k 323 / 251 / 253;
+//     45k 328 / 392 / 369
+int search_split(const sph_ctx *ctx) {
+    const long long n = ctx->n, sm = ctx->num_sms;
+    return n <= SPLIT8_PER_SM * sm ? 8 : n <= SPLIT4_PER_SM * sm ? 4 : n <= SPLIT2_PER_SM * sm ? 2 : 1;
+}
+#define SPH_SPLIT(ctx, rc, call)                                          \
+    switch (search_split(ctx)) {                                          \
+        case 8: { constexpr int SPLIT = 8; rc = call; break; }            \
+        case 4: { constexpr int SPLIT = 4; rc = call; break; }            \
+        case 2: { constexpr int SPLIT = 2; rc = call; break; }            \
+        default: { constexpr int SPLIT = 1; rc = call; break; }           \
+    }
+
+// one search kernel over the units of the groups on the work queue
+template <class... P, class... Q>
+int search_launch(sph_ctx *ctx, void (*kern)(const int *, P...), int split, Q... args) {
+    // groups hold 1..32 particles, about 20 on average
+    const int units = (div_up(ctx->n, 16) + ctx->ncloud) * split;
+    int g;
+    unsigned *q;
+    int rc = queue_launch(ctx, ctx->stream, WQ_SEARCH, (const void *)kern, SEARCH_WARPS * 32,
+                          max(1, div_up(units, SEARCH_WARPS)), &g, &q);
+    if (rc) return rc;
+    kern<<<g, SEARCH_WARPS * 32, 0, ctx->stream>>>(ctx->d_ngroup, args..., q);
+    return SPH_OK;
+}
+
 }  // namespace
 
 // margin of the step's first candidate radius over h: h may grow by this
@@ -1235,8 +1497,6 @@ int launch_smoothing_h(sph_ctx *ctx) {
     if (reuse)
         k_group_moved<<<ctx->num_sms * 4, 256, 0, s>>>(ctx->d_ngroup, ctx->gstart, ctx->gcount,
                                                        ctx->dmv, ctx->gdm);
-    const int rounds = ctx->prologue_done ? 4 : 8;
-    const int grid = max(1, div_up(div_up(n, 16) + ctx->ncloud, SEARCH_WARPS));
     SearchArgs A = search_args(ctx, nullptr, ctx->cand_cnt);
     NewtonArgs B;
     B.p1 = ctx->p1;
@@ -1254,29 +1514,14 @@ int launch_smoothing_h(sph_ctx *ctx) {
     B.grow = H_GROW;
     B.regrow = H_REGROW;
     B.max_iter = ctx->cfg.h_max_iter;
-    const bool mixed = ctx->cfg.precision == SPH_PREC_MIXED;
-    const void *kern = mixed ? (const void *)k_cand_newton<float> : (const void *)k_cand_newton<double>;
-    for (int r = 0; r < rounds; r++) {
-        B.last_round = r == rounds - 1;
-        int g;
-        unsigned *q;
-        int rc = queue_launch(ctx, s, WQ_SEARCH, kern, SEARCH_WARPS * 32, grid, &g, &q);
-        if (rc) return rc;
-        if (r > 0) {
-            // the later rounds search again only for the few particles whose
-            // h left the candidate radius: a fixed stride over the groups,
-            // which most warps skip after one ballot, costs less than one
-            // work-queue atomic per group (the first round keeps the queue:
-            // after kept rows its share of searched groups ranges from none
-            // to all)
-            g = min(grid, ctx->num_sms * 8);
-            q = nullptr;
-        }
-        if (mixed)
-            k_cand_newton<float><<<g, SEARCH_WARPS * 32, 0, s>>>(ctx->d_ngroup, A, B, q);
-        else
-            k_cand_newton<double><<<g, SEARCH_WARPS * 32, 0, s>>>(ctx->d_ngroup, A, B, q);
+    B.rounds = ctx->prologue_done ? 4 : 8;
+    int rc;
+    if (ctx->cfg.precision == SPH_PREC_MIXED) {
+        SPH_SPLIT(ctx, rc, search_launch(ctx, k_cand_newton<float, SPLIT>, SPLIT, A, B));
+    } else {
+        SPH_SPLIT(ctx, rc, search_launch(ctx, k_cand_newton<double, SPLIT>, SPLIT, A, B));
     }
+    if (rc) return rc;
     // every row now lists the candidates of its hsr (or is marked incomplete)
     CK(cudaMemsetAsync(ctx->rows_ok, 1, sizeof(int), s));
     ctx->rows_host = true;
@@ -1296,31 +1541,22 @@ int launch_smoothing_h_count(sph_ctx *ctx, int n_target, int n_tol, double frac,
     ctx->kept_counted = false;
     k_h_init<<<div_up(n, 256), 256, 0, s>>>(n, ctx->st[c][ST_H], ctx->st[c][ST_HNB], ctx->hcand,
                                             ctx->retry, H_GROW_COUNT, nullptr, ReuseArgs{});
-    k_zero_int<<<div_up(n, 256), 256, 0, s>>>(n, ctx->hiter);
-    // each round widens the radius by H_GROW_COUNT; 0.3 % steps need about 26
-    // iterations for that, so 16 rounds cover a 3.4x change of h
-    const int rounds = 16;
-    const int grid = max(1, div_up(div_up(n, 16) + ctx->ncloud, SEARCH_WARPS));
     SearchArgs A = search_args(ctx, nullptr, ctx->cand_cnt);
     CountArgs B;
     B.h_out = ctx->st[c][ST_H];
     B.hc = ctx->hcand;
     B.retry = ctx->retry;
-    B.iters = ctx->hiter;
     B.lo_n = n_target - n_tol;
     B.hi_n = n_target + n_tol;
     B.max_iter = max_iter;
     B.frac = frac;
     B.grow = H_GROW_COUNT;
-    for (int r = 0; r < rounds; r++) {
-        B.last_round = r == rounds - 1;
-        int g;
-        unsigned *q;
-        int rc = queue_launch(ctx, s, WQ_SEARCH, (const void *)k_cand_count, SEARCH_WARPS * 32,
-                              grid, &g, &q);
-        if (rc) return rc;
-        k_cand_count<<<g, SEARCH_WARPS * 32, 0, s>>>(ctx->d_ngroup, A, B, q);
-    }
+    // each round widens the radius by at least H_GROW_COUNT, so 16 rounds
+    // cover a 3.4x change of h
+    B.rounds = 16;
+    int rc;
+    SPH_SPLIT(ctx, rc, search_launch(ctx, k_cand_count<SPLIT>, SPLIT, A, B));
+    if (rc) return rc;
     ctx->lists_ok = false;
     ctx->cand_ok = true;
     ctx->p2_dirty = true;
@@ -1340,23 +1576,16 @@ int launch_smoothing_kth(sph_ctx *ctx, int k) {
     ctx->kept_counted = false;
     k_h_init<<<div_up(n, 256), 256, 0, s>>>(n, ctx->st[c][ST_H], ctx->st[c][ST_HNB], ctx->hcand,
                                             ctx->retry, H_GROW_COUNT, nullptr, ReuseArgs{});
-    const int grid = max(1, div_up(div_up(n, 16) + ctx->ncloud, SEARCH_WARPS));
     SearchArgs A = search_args(ctx, nullptr, ctx->cand_cnt);
     CountArgs B{};
     B.h_out = ctx->st[c][ST_H];
     B.hc = ctx->hcand;
     B.retry = ctx->retry;
-    B.iters = ctx->hiter;
     B.grow = H_GROW_COUNT;
-    const int rounds = 24;
-    for (int r = 0; r < rounds; r++) {
-        B.last_round = r == rounds - 1;
-        int g;
-        unsigned *q;
-        int rc = queue_launch(ctx, s, WQ_SEARCH, (const void *)k_cand_kth, SEARCH_WARPS * 32, grid, &g, &q);
-        if (rc) return rc;
-        k_cand_kth<<<g, SEARCH_WARPS * 32, 0, s>>>(ctx->d_ngroup, A, B, k, q);
-    }
+    B.rounds = 24;
+    int rc;
+    SPH_SPLIT(ctx, rc, search_launch(ctx, k_cand_kth<SPLIT>, SPLIT, A, B, k));
+    if (rc) return rc;
     ctx->lists_ok = false;
     ctx->cand_ok = false;  // the rows are candidate sets of the search radius, not of h
     ctx->p2_dirty = true;
@@ -1382,11 +1611,8 @@ int launch_neighbours(sph_ctx *ctx) {
     // node h_max only matters to the tree search: skipped when no list needs it
     int rc = launch_refit_hmax(ctx, ctx->cand_ok ? ctx->lflag + n + 1 : nullptr);
     if (rc) return rc;
-    int g;
-    unsigned *q;
-    if ((rc = queue_launch(ctx, s, WQ_SEARCH, (const void *)k_lists, SEARCH_WARPS * 32, grid, &g, &q)))
-        return rc;
-    k_lists<<<g, SEARCH_WARPS * 32, 0, s>>>(ctx->d_ngroup, A, q);
+    SPH_SPLIT(ctx, rc, search_launch(ctx, k_lists<SPLIT>, SPLIT, A));
+    if (rc) return rc;
     ctx->lists_ok = true;
     ctx->rho_ok = ctx->divcurl_ok = false;
     return ctx_check_launch(ctx, "neighbours");
@@ -1397,7 +1623,6 @@ int launch_neighbours(sph_ctx *ctx) {
 int launch_lists_marked(sph_ctx *ctx) {
     const int n = ctx->n;
     if (n <= 0) return SPH_OK;
-    const int grid = max(1, div_up(div_up(n, 16) + ctx->ncloud, SEARCH_WARPS));
     SearchArgs A = search_args(ctx, ctx->ngb, ctx->ngb_cnt);
     A.only = ctx->lflag;
     A.only_all = ctx->lflag + n;
@@ -1405,12 +1630,8 @@ int launch_lists_marked(sph_ctx *ctx) {
     A.mcount = ctx->lflag + n + 2;
     int rc = launch_refit_hmax(ctx, ctx->lflag + n + 1);
     if (rc) return rc;
-    int g;
-    unsigned *q;
-    if ((rc = queue_launch(ctx, ctx->stream, WQ_SEARCH, (const void *)k_lists, SEARCH_WARPS * 32,
-                           grid, &g, &q)))
-        return rc;
-    k_lists<<<g, SEARCH_WARPS * 32, 0, ctx->stream>>>(ctx->d_ngroup, A, q);
+    SPH_SPLIT(ctx, rc, search_launch(ctx, k_lists<SPLIT>, SPLIT, A));
+    if (rc) return rc;
     k_lists_list<<<ctx->num_sms * 2, SEARCH_WARPS * 32, 0, ctx->stream>>>(ctx->d_ngroup, A);
     return ctx_check_launch(ctx, "lists_marked");
 }

@@ -126,7 +126,6 @@ struct sph_ctx {
     int *mlist = nullptr;     // the particles the fused list pass marked, each once
     bool cand_ok = false;     // candidate rows match the current order, positions and h
     int *retry = nullptr;        // per particle: 1 search, 2 or 3 keep the row, 0 done
-    int *hiter = nullptr;        // per particle: iterations of the count iteration so far
     double *hcand = nullptr;     // candidate radius / 2 used per particle
     double *hover = nullptr;     // smallest candidate radius / 2 whose row overflowed this call
     // candidate rows kept between the h iterations of refit steps: a row
