@@ -64,9 +64,9 @@ int sph_cooling_setup(sph_ctx *ctx, const sph_cooling_params *p, const double *l
     cudaSetDevice(ctx->device);
     if (!ctx->cool_table) {
         void *q = nullptr;
-        CK(cudaMalloc(&q, sizeof(double) * 2 * 4097));
+        CK(cudaMalloc(&q, COOL_BYTES));
         ctx->allocs.push_back(q);
-        ctx->dev_bytes += sizeof(double) * 2 * 4097;
+        ctx->dev_bytes += COOL_BYTES;
         ctx->cool_table = (double *)q;
     }
     CK(cudaMemcpyAsync(ctx->cool_table, log_lambda, sizeof(double) * (p->n_bins + 1),
@@ -76,7 +76,29 @@ int sph_cooling_setup(sph_ctx *ctx, const sph_cooling_params *p, const double *l
         const double dl = (p->logT1 - p->logT0) / p->n_bins;
         std::vector<double> lamT(p->n_bins + 1);
         for (int e = 0; e <= p->n_bins; e++) lamT[e] = pow(10.0, log_lambda[e] - (p->logT0 + e * dl));
-        CK(cudaMemcpyAsync(ctx->cool_table + 4097, lamT.data(), sizeof(double) * (p->n_bins + 1),
+        CK(cudaMemcpyAsync(ctx->cool_table + COOL_EDGES, lamT.data(), sizeof(double) * (p->n_bins + 1),
+                           cudaMemcpyHostToDevice, ctx->stream));
+        std::vector<CoolBin> bin(p->n_bins);
+        for (int e = 0; e < p->n_bins; e++) {
+            const double slope = (log_lambda[e + 1] - log_lambda[e]) / dl;
+            bin[e] = {lamT[e], pow(10.0, -(p->logT0 + e * dl)), pow(10.0, p->logT0 + e * dl),
+                      (float)(slope - 1.0), (short)e, (short)e, log_lambda[e], slope,
+                      log_lambda[e + 1] - log_lambda[e], 0.0};
+            if (slope < 0.0 && bin[e].sm1 >= -1.f) bin[e].sm1 = nextafterf(-1.f, -2.f);
+            if (e > 0 && bin[e].sm1 >= -1.f && bin[e - 1].sm1 >= -1.f) bin[e].dn = bin[e - 1].dn;
+        }
+        for (int e = p->n_bins - 2; e >= 0; e--)
+            if (bin[e].sm1 >= -1.f && bin[e + 1].sm1 >= -1.f) bin[e].un = bin[e + 1].un;
+        // the FP32 slope as the surrogate's arithmetic formed it bin by bin
+        std::vector<float2> binf(p->n_bins);
+        const float fdl = (float)dl;
+        for (int e = 0; e < p->n_bins; e++) {
+            const float L0 = (float)log_lambda[e], L1 = (float)log_lambda[e + 1];
+            binf[e] = make_float2(L0, (L1 - L0) / fdl);
+        }
+        CK(cudaMemcpyAsync((char *)ctx->cool_table + COOL_AT_BIN, bin.data(), sizeof(CoolBin) * p->n_bins,
+                           cudaMemcpyHostToDevice, ctx->stream));
+        CK(cudaMemcpyAsync((char *)ctx->cool_table + COOL_AT_BINF, binf.data(), sizeof(float2) * p->n_bins,
                            cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
     }

@@ -539,6 +539,10 @@ __global__ void k_cool_list_arrays(CoolDev c, const int *__restrict__ list, int 
 // to the exact solver.
 namespace tc {
 
+#ifndef SPH_TC_CTAS
+#define SPH_TC_CTAS 8
+#endif
+
 constexpr int ROWS = 128;
 constexpr int COLS = 64;          // TMEM columns of the accumulator
 constexpr int SPIN = 1 << 22;     // try_wait polls before a wait gives up
@@ -550,10 +554,14 @@ struct alignas(128) Smem {
     unsigned long long mbar;
     unsigned tmem;
 };
-// dynamic shared memory per CTA: at most 7 CTAs share an SM, 7 x 64 TMEM
-// columns of the 512
-constexpr int SMEM_BYTES = 32 * 1024;
+// CTAs per SM: the registers are bounded for them, their shared memory (1 KB of
+// it the system's) fits 227 KB, and no more than 8 can be resident, 8 x 64
+// TMEM columns of the 512
+constexpr int CTAS = SPH_TC_CTAS;
+constexpr int SMEM_BYTES = 27 * 1024;
 static_assert(sizeof(Smem) <= SMEM_BYTES, "tcgen05 MLP tile does not fit");
+static_assert(CTAS <= 8 && CTAS * (SMEM_BYTES + 1024) <= 227 * 1024 && 9 * (SMEM_BYTES + 1024) > 228 * 1024,
+              "TMEM and shared memory of the resident CTAs");
 
 __device__ __forceinline__ unsigned saddr(const void *p) {
     return (unsigned)__cvta_generic_to_shared(p);
@@ -716,7 +724,7 @@ __device__ __forceinline__ float predict(Smem &S, const float x[3], unsigned &ph
 
 }  // namespace tc
 
-__global__ void __launch_bounds__(tc::ROWS)
+__global__ void __launch_bounds__(tc::ROWS, tc::CTAS)
     k_mlp_forward_tc(int n, const float *__restrict__ X, float *__restrict__ y,
                      const __nv_bfloat16 *__restrict__ pk, const float *__restrict__ P,
                      long long *status) {
@@ -737,7 +745,7 @@ __global__ void __launch_bounds__(tc::ROWS)
 }
 
 // in-step cooling with the tensor-core surrogate, 128 rows per CTA
-__global__ void __launch_bounds__(tc::ROWS)
+__global__ void __launch_bounds__(tc::ROWS, tc::CTAS)
     k_cool_mlp_tc(CoolDev c, int n, const double *__restrict__ rho, double *__restrict__ u,
                   const int *__restrict__ cloud, const double *__restrict__ dt, double ur,
                   double uu, double ut, const __nv_bfloat16 *__restrict__ pk,
@@ -784,7 +792,7 @@ __global__ void __launch_bounds__(tc::ROWS)
 }
 
 // the same for standalone arrays (cgs), with the per-row fallback flag
-__global__ void __launch_bounds__(tc::ROWS)
+__global__ void __launch_bounds__(tc::ROWS, tc::CTAS)
     k_cool_mlp_arrays_tc(CoolDev c, int n, const double *__restrict__ rho,
                          const double *__restrict__ u_old, const double *__restrict__ dtv,
                          double *__restrict__ u_new, int *__restrict__ fell_back,
@@ -827,10 +835,17 @@ __global__ void __launch_bounds__(tc::ROWS)
     tc::teardown(S);
 }
 
-// grid of a tensor-core MLP kernel: at most 7 CTAs per SM (TMEM columns)
+// grid of a tensor-core MLP kernel: the CTAs that are resident at once, each
+// striding over the tiles (7 per SM of kernels whose registers and shared memory
+// allowed 6 left the seventh of each SM to run alone after the others)
 int tc_grid(sph_ctx *ctx, int n) {
-    return max(1, min(div_up(n, tc::ROWS), ctx->num_sms * 7));
+    return max(1, min(div_up(n, tc::ROWS), ctx->num_sms * tc::CTAS));
 }
+// grid of the exact solves of the listed rows, whose number only the device
+// knows: a thread per row for up to a quarter of the n rows (a few blocks per
+// SM gave some threads three rows in turn: 161k of 2^20 rows 101 us, here
+// 79 us), a stride beyond
+int list_grid(sph_ctx *ctx, int n) { return max(ctx->num_sms * 4, div_up(n, 4 * 128)); }
 bool use_tc(const sph_ctx *ctx) { return !(ctx->cfg.flags & SPH_FLAG_MLP_WARP_MMA); }
 
 int grid_for(sph_ctx *ctx, int n) { return max(1, min(div_up(div_up(n, 16), 4), ctx->num_sms * 8)); }
@@ -952,7 +967,7 @@ int launch_cooling_mlp(sph_ctx *ctx) {
             ctx->cool.unit_rho, ctx->cool.unit_u, ctx->cool.unit_t,
             (const __nv_bfloat16 *)ctx->mlp_bf16, ctx->mlp, ctx->cool.mlp_err_tol, ctx->cool_list,
             cap, ctx->status);
-    k_cool_list<<<ctx->num_sms * 4, 128, 0, ctx->stream>>>(
+    k_cool_list<<<list_grid(ctx, n), 128, 0, ctx->stream>>>(
         cool_dev_of(ctx), ctx->cool_list, cap, ctx->rho, ctx->st[c][ST_U], ctx->cloud[c], ctx->dt,
         ctx->cool.unit_rho, ctx->cool.unit_u, ctx->cool.unit_t, ctx->status);
     return ctx_check_launch(ctx, "cooling_mlp");
@@ -1069,7 +1084,7 @@ int sph_cool_solve_mlp(sph_ctx *ctx, int32_t n, const double *rho, const double 
             cool_dev_of(ctx), n, rho, u_old, dt, u_new, fell_back,
             (const __nv_bfloat16 *)ctx->mlp_bf16, ctx->mlp, ctx->cool.mlp_err_tol, ctx->cool_list,
             cap);
-    k_cool_list_arrays<<<ctx->num_sms * 4, 128, 0, ctx->stream>>>(cool_dev_of(ctx), ctx->cool_list,
+    k_cool_list_arrays<<<list_grid(ctx, n), 128, 0, ctx->stream>>>(cool_dev_of(ctx), ctx->cool_list,
                                                                  cap, rho, u_old, dt, u_new);
     return ctx_check_launch(ctx, "cool_solve_mlp");
 }
