@@ -3,8 +3,8 @@
 // in-step surrogate, the standalone solves and sph_mlp_forward) runs its 64 x 64
 // layer on tcgen05.mma with a TMEM accumulator, 128 rows per CTA (namespace
 // tc below); training (forward + backward of minibatches, weight gradients from
-// transposed activations) uses the warp-level mma.sync.aligned.m16n8k16 bf16
-// fragments, and SPH_FLAG_MLP_WARP_MMA selects them for inference too.  All
+// transposed reads of the activations) uses the warp-level mma.sync.aligned.m16n8k16
+// bf16 fragments, and SPH_FLAG_MLP_WARP_MMA selects them for inference too.  All
 // kernels are written here, with Adam, and the in-step use: predict
 // dlog10(u) = log10(u_new/u_old) from (log10 rho, log10 u, log10 dt) [cgs],
 // estimate the error of the prediction with the Newton residual of the
@@ -71,12 +71,6 @@ __device__ __forceinline__ float gelu_fast(float z) {
     return 0.5f * z * (1.0f + t);
 }
 template <bool FAST> __device__ __forceinline__ float act(float z) { return FAST ? gelu_fast(z) : gelu(z); }
-__device__ __forceinline__ float gelu_grad(float z) {
-    const float k = 0.7978845608028654f;
-    const float t = tanhf(k * (z + 0.044715f * z * z * z));
-    return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * k * (1.0f + 3.0f * 0.044715f * z * z);
-}
-
 struct MlpSmem {
     __nv_bfloat16 w[PK_N];     // W1t, W2t, W2
     float b1[H], b2[H], w3[H], b3;
@@ -194,182 +188,323 @@ __global__ void __launch_bounds__(128)
     }
 }
 
-// gradient of L = 0.5/n_total * sum (y - t)^2 over this launch's rows, added
-// into grad (FP32, pre-zeroed); loss added into *loss
-constexpr int GR = 256;        // rows per block
-constexpr int LD = GR + 8;     // padded row stride of the transposed tiles
+// ---- training ----
+// Gradient of L = 0.5 / n sum (y - t)^2: every block walks tiles of 32 rows and
+// leaves its sums in its own slot of `part` (NPART floats: the gradient, then
+// the loss), which k_mlp_update adds up in block order, so a gradient is the
+// same on every run.  A minibatch is a few thousand rows, so the kernel is
+// bound by how few warps a row's chain of layers gives the chip: 4096 rows in
+// blocks of 256 rows by 4 warps used 16 SMs for 165 us a step; 32 rows by 8
+// warps use 128 SMs for 6.2 us, each warp 16 rows by 16 columns of a layer, the
+// layers handed on through shared memory (rows padded to 144 bytes:
+// conflict-free fragments).  A z's tanh is taken once, for GELU and its
+// derivative.  64 training steps of 4096 rows: 11.6 -> 0.62 ms with the update
+// in one launch and both in programmatic stream order.
+constexpr int GROWS = 32;       // rows per tile
+constexpr int GBLOCKS = 2;      // resident blocks per SM (3 spill)
+constexpr int LDH = H + 8;      // row stride of the 64-wide BF16 tiles
+constexpr int LDX = 16 + 8;     // row stride of the 16-wide ones
+constexpr int NPART = NP + 3;   // floats per block slot: gradient, loss, padding to 16 bytes
+
 struct GradSmem {
-    MlpSmem W;
-    __nv_bfloat16 X[GR * 16];  // row-major [r][c]
-    __nv_bfloat16 Xt[16 * LD]; // [c][r]
-    __nv_bfloat16 At1[H * LD]; // gelu(z1) transposed [i][r]
-    __nv_bfloat16 dZ2t[H * LD];
-    __nv_bfloat16 dZ1t[H * LD];
-    float gb1[H], gb2[H], gw3[H], gb3, loss;
+    __nv_bfloat16 W1t[H * LDX], W2t[H * LDH], W2[H * LDH];
+    float b1[H], b2[H], w3[H], b3;
+    alignas(16) __nv_bfloat16 X[2][GROWS * LDX];
+    alignas(16) __nv_bfloat16 A1[GROWS * LDH], dZ2[GROWS * LDH], dZ1[GROWS * LDH];
+    float y[4][GROWS];
+    float red[3][2][H], gb3[2], loss[2];
 };
 
-__global__ void __launch_bounds__(128)
+// The two kernels of a training step follow each other in programmatic stream
+// order: the next one's blocks start while the last one's finish and wait here
+// for all of it (its writes included) before they touch global memory.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// GELU and its derivative from one tanh
+__device__ __forceinline__ void gelu_both(float z, float &g, float &d) {
+    const float k = 0.7978845608028654f;
+    const float t = tanhf(k * (z + 0.044715f * z * z * z));
+    g = 0.5f * z * (1.0f + t);
+    d = 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * k * (1.0f + 3.0f * 0.044715f * z * z);
+}
+__device__ __forceinline__ void st32(__nv_bfloat16 *p, unsigned v) { *reinterpret_cast<unsigned *>(p) = v; }
+// A fragment (rows gid, gid + 8; 16 columns) of a row-major tile
+__device__ __forceinline__ void frag_a(const __nv_bfloat16 *p, int ld, unsigned a[4]) {
+    const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+    p += gid * ld + 2 * tig;
+    a[0] = ld32(p);
+    a[1] = ld32(p + 8 * ld);
+    a[2] = ld32(p + 8);
+    a[3] = ld32(p + 8 * ld + 8);
+}
+// four transposed 8 x 8 tiles: lane l gives the address of row l % 8 of tile l / 8
+__device__ __forceinline__ void ldm4t(const __nv_bfloat16 *p, unsigned r[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+
+__global__ void __launch_bounds__(256, GBLOCKS)
     k_mlp_grad(int n, const float *__restrict__ X, const float *__restrict__ T, float inv_n,
                const __nv_bfloat16 *__restrict__ pk, const float *__restrict__ P,
-               float *__restrict__ grad, float *__restrict__ loss) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    GradSmem &S = *reinterpret_cast<GradSmem *>(smem_raw);
-    load_weights(S.W, pk, P);
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-    const int rb = blockIdx.x * GR;
-    for (int e = threadIdx.x; e < GR * 16; e += blockDim.x) {
-        const int r = e / 16, c = e % 16;
-        const float v = (c < 3 && rb + r < n) ? X[3 * (rb + r) + c] : 0.f;
-        const __nv_bfloat16 bv = __float2bfloat16_rn(v);
-        S.X[e] = bv;
-        S.Xt[c * LD + r] = bv;
+               float *__restrict__ part) {
+    __shared__ GradSmem S;
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31, gid = lane >> 2, tig = lane & 3;
+    for (int e = t; e < 2 * GROWS * LDX / 2; e += 256) reinterpret_cast<unsigned *>(S.X)[e] = 0u;
+    // the weights are the last step's update's
+    grid_wait();
+    grid_release();
+    for (int e = t; e < H * 2; e += 256)
+        *reinterpret_cast<uint4 *>(S.W1t + (e >> 1) * LDX + (e & 1) * 8) =
+            *reinterpret_cast<const uint4 *>(pk + PK_W1T + e * 8);
+    for (int e = t; e < H * 8; e += 256) {
+        const int o = (e >> 3) * LDH + (e & 7) * 8;
+        *reinterpret_cast<uint4 *>(S.W2t + o) = *reinterpret_cast<const uint4 *>(pk + PK_W2T + e * 8);
+        *reinterpret_cast<uint4 *>(S.W2 + o) = *reinterpret_cast<const uint4 *>(pk + PK_W2 + e * 8);
     }
-    for (int k = threadIdx.x; k < H; k += blockDim.x) S.gb1[k] = S.gb2[k] = S.gw3[k] = 0.f;
-    if (threadIdx.x == 0) S.gb3 = S.loss = 0.f;
+    if (t < H) {
+        S.b1[t] = P[OFF_B1 + t];
+        S.b2[t] = P[OFF_B2 + t];
+        S.w3[t] = P[OFF_W3 + t];
+    }
+    if (t == 0) S.b3 = P[OFF_B3];
     __syncthreads();
-    const __nv_bfloat16 *W2 = S.W.w + PK_W2;
-    float pb3 = 0.f, pl = 0.f;
-    for (int tile = w; tile < GR / 16; tile += 4) {
-        const int r0 = tile * 16;
-        unsigned ax[4];
-        x_fragment(S.X + r0 * 16, ax);
-        float z1[8][4], z2[8][4], y0, y1;
-        tile_forward(S.W, ax, z1, z2, y0, y1);
-        const bool ok0 = rb + r0 + gid < n, ok1 = rb + r0 + gid + 8 < n;
-        const float e0 = ok0 ? y0 - T[rb + r0 + gid] : 0.f;
-        const float e1 = ok1 ? y1 - T[rb + r0 + gid + 8] : 0.f;
-        const float dy0 = e0 * inv_n, dy1 = e1 * inv_n;
-        if (tig == 0) {
-            pl += 0.5f * inv_n * (e0 * e0 + e1 * e1);
-            pb3 += dy0 + dy1;
+
+    // this warp: rows 16 rt .. and columns 16 cg .. of each layer; and rows
+    // 16 mi .., columns 32 nh .. of dW2
+    const int rt = w & 1, cg = w >> 1, mi = w & 3, nh = w >> 2;
+    const int c0 = 16 * cg + 2 * tig;  // this lane's columns: c0 + 8 nt, + 1
+    float aw2[4][4] = {}, aw1 = 0.f, gw3[2][2] = {}, gb2[2][2] = {}, gb1[2][2] = {}, gb3 = 0.f, pl = 0.f;
+    const int ntile = (n + GROWS - 1) / GROWS;
+    int buf = 0;
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x, buf ^= 1) {
+        const int rb = tile * GROWS, r0 = rb + 16 * rt + gid, r1 = r0 + 8;
+        if (t < 3 * GROWS) {
+            const int r = t / 3, c = t % 3;
+            S.X[buf][r * LDX + c] = __float2bfloat16_rn(rb + r < n ? X[3 * (size_t)rb + t] : 0.f);
         }
-        // dZ2, bias/W3 partials, transposed tiles for the weight GEMMs
-        float dz2[8][4];
+        const float t0 = r0 < n ? T[r0] : 0.f, t1 = r1 < n ? T[r1] : 0.f;
+        __syncthreads();
+        // layer 1
+        float d1[2][4];
+        {
+            unsigned ax[4];
+            frag_a(S.X[buf] + 16 * rt * LDX, LDX, ax);
 #pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
-            const int col = nt * 8 + 2 * tig;
-            const float w30 = S.W.w3[col], w31 = S.W.w3[col + 1];
-            dz2[nt][0] = dy0 * w30 * gelu_grad(z2[nt][0]);
-            dz2[nt][1] = dy0 * w31 * gelu_grad(z2[nt][1]);
-            dz2[nt][2] = dy1 * w30 * gelu_grad(z2[nt][2]);
-            dz2[nt][3] = dy1 * w31 * gelu_grad(z2[nt][3]);
-            atomicAdd(&S.gw3[col], gelu(z2[nt][0]) * dy0 + gelu(z2[nt][2]) * dy1);
-            atomicAdd(&S.gw3[col + 1], gelu(z2[nt][1]) * dy0 + gelu(z2[nt][3]) * dy1);
-            atomicAdd(&S.gb2[col], dz2[nt][0] + dz2[nt][2]);
-            atomicAdd(&S.gb2[col + 1], dz2[nt][1] + dz2[nt][3]);
-            const int ra = r0 + gid, rc = r0 + gid + 8;
-            S.At1[col * LD + ra] = __float2bfloat16_rn(gelu(z1[nt][0]));
-            S.At1[(col + 1) * LD + ra] = __float2bfloat16_rn(gelu(z1[nt][1]));
-            S.At1[col * LD + rc] = __float2bfloat16_rn(gelu(z1[nt][2]));
-            S.At1[(col + 1) * LD + rc] = __float2bfloat16_rn(gelu(z1[nt][3]));
-            S.dZ2t[col * LD + ra] = __float2bfloat16_rn(dz2[nt][0]);
-            S.dZ2t[(col + 1) * LD + ra] = __float2bfloat16_rn(dz2[nt][1]);
-            S.dZ2t[col * LD + rc] = __float2bfloat16_rn(dz2[nt][2]);
-            S.dZ2t[(col + 1) * LD + rc] = __float2bfloat16_rn(dz2[nt][3]);
-        }
-        // dA1 = dZ2 W2^T  (B[k=j][n=i] = W2[i][j], stored [i][j])
-        unsigned ad[4][4];
-#pragma unroll
-        for (int kk = 0; kk < 4; kk++) {
-            ad[kk][0] = pack2(dz2[2 * kk][0], dz2[2 * kk][1]);
-            ad[kk][1] = pack2(dz2[2 * kk][2], dz2[2 * kk][3]);
-            ad[kk][2] = pack2(dz2[2 * kk + 1][0], dz2[2 * kk + 1][1]);
-            ad[kk][3] = pack2(dz2[2 * kk + 1][2], dz2[2 * kk + 1][3]);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
-            float da[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int kk = 0; kk < 4; kk++) {
-                const __nv_bfloat16 *wb = W2 + (nt * 8 + gid) * 64 + kk * 16 + 2 * tig;
+            for (int nt = 0; nt < 2; nt++) {
+                const int col = c0 + 8 * nt;
+                float z[4] = {S.b1[col], S.b1[col + 1], S.b1[col], S.b1[col + 1]}, g[4];
+                const __nv_bfloat16 *wb = S.W1t + (16 * cg + 8 * nt + gid) * LDX + 2 * tig;
                 const unsigned b[2] = {ld32(wb), ld32(wb + 8)};
-                mma16816(da, ad[kk], b);
+                mma16816(z, ax, b);
+#pragma unroll
+                for (int q = 0; q < 4; q++) gelu_both(z[q], g[q], d1[nt][q]);
+                st32(S.A1 + (16 * rt + gid) * LDH + col, pack2(g[0], g[1]));
+                st32(S.A1 + (16 * rt + gid + 8) * LDH + col, pack2(g[2], g[3]));
             }
-            const int col = nt * 8 + 2 * tig;
-            const float d0 = da[0] * gelu_grad(z1[nt][0]), d1 = da[1] * gelu_grad(z1[nt][1]);
-            const float d2 = da[2] * gelu_grad(z1[nt][2]), d3 = da[3] * gelu_grad(z1[nt][3]);
-            atomicAdd(&S.gb1[col], d0 + d2);
-            atomicAdd(&S.gb1[col + 1], d1 + d3);
-            const int ra = r0 + gid, rc = r0 + gid + 8;
-            S.dZ1t[col * LD + ra] = __float2bfloat16_rn(d0);
-            S.dZ1t[(col + 1) * LD + ra] = __float2bfloat16_rn(d1);
-            S.dZ1t[col * LD + rc] = __float2bfloat16_rn(d2);
-            S.dZ1t[(col + 1) * LD + rc] = __float2bfloat16_rn(d3);
+        }
+        __syncthreads();
+        // layer 2 and this warp's part of layer 3
+        float a2[2][4], d2[2][4], s0 = 0.f, s1 = 0.f;
+        {
+            unsigned a[4][4];
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) frag_a(S.A1 + 16 * rt * LDH + 16 * kk, LDH, a[kk]);
+#pragma unroll
+            for (int nt = 0; nt < 2; nt++) {
+                const int col = c0 + 8 * nt;
+                float z[4] = {S.b2[col], S.b2[col + 1], S.b2[col], S.b2[col + 1]};
+#pragma unroll
+                for (int kk = 0; kk < 4; kk++) {
+                    const __nv_bfloat16 *wb = S.W2t + (16 * cg + 8 * nt + gid) * LDH + 16 * kk + 2 * tig;
+                    const unsigned b[2] = {ld32(wb), ld32(wb + 8)};
+                    mma16816(z, a[kk], b);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) gelu_both(z[q], a2[nt][q], d2[nt][q]);
+                s0 += a2[nt][0] * S.w3[col] + a2[nt][1] * S.w3[col + 1];
+                s1 += a2[nt][2] * S.w3[col] + a2[nt][3] * S.w3[col + 1];
+            }
+        }
+        s0 += __shfl_xor_sync(FULL, s0, 1);
+        s0 += __shfl_xor_sync(FULL, s0, 2);
+        s1 += __shfl_xor_sync(FULL, s1, 1);
+        s1 += __shfl_xor_sync(FULL, s1, 2);
+        if (tig == 0) {
+            S.y[cg][16 * rt + gid] = s0;
+            S.y[cg][16 * rt + gid + 8] = s1;
+        }
+        __syncthreads();
+        // the error, dZ2, and the sums of layer 3 and b2
+        {
+            const int q0 = 16 * rt + gid, q1 = q0 + 8;
+            const float y0 = ((S.y[0][q0] + S.y[1][q0]) + (S.y[2][q0] + S.y[3][q0])) + S.b3;
+            const float y1 = ((S.y[0][q1] + S.y[1][q1]) + (S.y[2][q1] + S.y[3][q1])) + S.b3;
+            const float e0 = r0 < n ? y0 - t0 : 0.f, e1 = r1 < n ? y1 - t1 : 0.f;
+            const float dy0 = e0 * inv_n, dy1 = e1 * inv_n;
+            if (cg == 0 && tig == 0) {
+                pl += 0.5f * inv_n * (e0 * e0 + e1 * e1);
+                gb3 += dy0 + dy1;
+            }
+#pragma unroll
+            for (int nt = 0; nt < 2; nt++) {
+                const int col = c0 + 8 * nt;
+                const float w30 = S.w3[col], w31 = S.w3[col + 1];
+                const float z0 = dy0 * w30 * d2[nt][0], z1 = dy0 * w31 * d2[nt][1];
+                const float z2 = dy1 * w30 * d2[nt][2], z3 = dy1 * w31 * d2[nt][3];
+                gw3[nt][0] += a2[nt][0] * dy0 + a2[nt][2] * dy1;
+                gw3[nt][1] += a2[nt][1] * dy0 + a2[nt][3] * dy1;
+                gb2[nt][0] += z0 + z2;
+                gb2[nt][1] += z1 + z3;
+                st32(S.dZ2 + q0 * LDH + col, pack2(z0, z1));
+                st32(S.dZ2 + q1 * LDH + col, pack2(z2, z3));
+            }
+        }
+        __syncthreads();
+        // dA1 = dZ2 W2^T (B[k = j][n = i] = W2[i][j], stored [i][j]), dZ1
+        {
+            unsigned a[4][4];
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) frag_a(S.dZ2 + 16 * rt * LDH + 16 * kk, LDH, a[kk]);
+#pragma unroll
+            for (int nt = 0; nt < 2; nt++) {
+                const int col = c0 + 8 * nt;
+                float da[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int kk = 0; kk < 4; kk++) {
+                    const __nv_bfloat16 *wb = S.W2 + (16 * cg + 8 * nt + gid) * LDH + 16 * kk + 2 * tig;
+                    const unsigned b[2] = {ld32(wb), ld32(wb + 8)};
+                    mma16816(da, a[kk], b);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) da[q] *= d1[nt][q];
+                gb1[nt][0] += da[0] + da[2];
+                gb1[nt][1] += da[1] + da[3];
+                st32(S.dZ1 + (16 * rt + gid) * LDH + col, pack2(da[0], da[1]));
+                st32(S.dZ1 + (16 * rt + gid + 8) * LDH + col, pack2(da[2], da[3]));
+            }
+        }
+        // dW2[i][j] += sum_r A1[r][i] dZ2[r][j], both read transposed
+#pragma unroll
+        for (int ks = 0; ks < GROWS / 16; ks++) {
+            // A: tiles (r, i), (r, i + 8), (r + 8, i), (r + 8, i + 8)
+            unsigned a[4];
+            ldm4t(S.A1 + (16 * ks + (lane & 7) + 8 * (lane >> 4)) * LDH + 16 * mi + 8 * ((lane >> 3) & 1), a);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                // B: tiles (r, j), (r + 8, j), (r, j + 8), (r + 8, j + 8)
+                unsigned b[4];
+                ldm4t(S.dZ2 + (16 * ks + (lane & 7) + 8 * ((lane >> 3) & 1)) * LDH + 32 * nh + 16 * h +
+                          8 * (lane >> 4),
+                      b);
+                mma16816(aw2[2 * h], a, b);
+                mma16816(aw2[2 * h + 1], a, b + 2);
+            }
+        }
+        __syncthreads();
+        // dW1[c][j] += sum_r X[r][c] dZ1[r][j]
+        if (t < 3 * H) {
+            const __nv_bfloat16 *x = S.X[buf] + t / H, *z = S.dZ1 + t % H;
+#pragma unroll 8
+            for (int r = 0; r < GROWS; r++)
+                aw1 = fmaf(__bfloat162float(x[r * LDX]), __bfloat162float(z[r * LDH]), aw1);
         }
     }
-    if (tig == 0) {
-        atomicAdd(&S.gb3, pb3);
-        atomicAdd(&S.loss, pl);
+    // this block's slot
+    float *out = part + (size_t)blockIdx.x * NPART;
+    if (t < 3 * H) out[OFF_W1 + t] = aw1;
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++) {
+        const int o = OFF_W2 + (16 * mi + gid) * H + 32 * nh + 8 * nt + 2 * tig;
+        *reinterpret_cast<float2 *>(out + o) = make_float2(aw2[nt][0], aw2[nt][1]);
+        *reinterpret_cast<float2 *>(out + o + 8 * H) = make_float2(aw2[nt][2], aw2[nt][3]);
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            float v[3] = {gb1[nt][q], gb2[nt][q], gw3[nt][q]};
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) v[k] += __shfl_xor_sync(FULL, v[k], o);
+                if (gid == 0) S.red[k][rt][c0 + 8 * nt + q] = v[k];
+            }
+        }
+    if (cg == 0) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            gb3 += __shfl_xor_sync(FULL, gb3, o);
+            pl += __shfl_xor_sync(FULL, pl, o);
+        }
+        if (lane == 0) {
+            S.gb3[rt] = gb3;
+            S.loss[rt] = pl;
+        }
     }
     __syncthreads();
-    // dW2[i][j] = sum_r A1[r][i] dZ2[r][j]: warp w owns rows i = 16w..16w+15
-    {
-        float acc[8][4];
-#pragma unroll
-        for (int nt = 0; nt < 8; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-        const int i0 = 16 * w;
-        for (int kk = 0; kk < GR / 16; kk++) {
-            const __nv_bfloat16 *ap = S.At1 + (i0 + gid) * LD + kk * 16 + 2 * tig;
-            const unsigned a[4] = {ld32(ap), ld32(ap + 8 * LD), ld32(ap + 8), ld32(ap + 8 * LD + 8)};
-#pragma unroll
-            for (int nt = 0; nt < 8; nt++) {
-                const __nv_bfloat16 *bp = S.dZ2t + (nt * 8 + gid) * LD + kk * 16 + 2 * tig;
-                const unsigned b[2] = {ld32(bp), ld32(bp + 8)};
-                mma16816(acc[nt], a, b);
-            }
-        }
-#pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
-            const int j = nt * 8 + 2 * tig;
-            atomicAdd(&grad[OFF_W2 + (i0 + gid) * H + j], acc[nt][0]);
-            atomicAdd(&grad[OFF_W2 + (i0 + gid) * H + j + 1], acc[nt][1]);
-            atomicAdd(&grad[OFF_W2 + (i0 + gid + 8) * H + j], acc[nt][2]);
-            atomicAdd(&grad[OFF_W2 + (i0 + gid + 8) * H + j + 1], acc[nt][3]);
-        }
+    if (t < H) {
+        out[OFF_B1 + t] = S.red[0][0][t] + S.red[0][1][t];
+        out[OFF_B2 + t] = S.red[1][0][t] + S.red[1][1][t];
+        out[OFF_W3 + t] = S.red[2][0][t] + S.red[2][1][t];
     }
-    // dW1[c][j] = sum_r X[r][c] dZ1[r][j]: warp w owns columns j = 16w..16w+15
-    {
-        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        for (int kk = 0; kk < GR / 16; kk++) {
-            const __nv_bfloat16 *ap = S.Xt + gid * LD + kk * 16 + 2 * tig;
-            const unsigned a[4] = {ld32(ap), ld32(ap + 8 * LD), ld32(ap + 8), ld32(ap + 8 * LD + 8)};
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const __nv_bfloat16 *bp = S.dZ1t + ((2 * w + q) * 8 + gid) * LD + kk * 16 + 2 * tig;
-                const unsigned b[2] = {ld32(bp), ld32(bp + 8)};
-                mma16816(acc[q], a, b);
-            }
-        }
-        if (gid < 3)
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const int j = (2 * w + q) * 8 + 2 * tig;
-                atomicAdd(&grad[OFF_W1 + gid * H + j], acc[q][0]);
-                atomicAdd(&grad[OFF_W1 + gid * H + j + 1], acc[q][1]);
-            }
-    }
-    for (int k = threadIdx.x; k < H; k += blockDim.x) {
-        atomicAdd(&grad[OFF_B1 + k], S.gb1[k]);
-        atomicAdd(&grad[OFF_B2 + k], S.gb2[k]);
-        atomicAdd(&grad[OFF_W3 + k], S.gw3[k]);
-    }
-    if (threadIdx.x == 0) {
-        atomicAdd(&grad[OFF_B3], S.gb3);
-        atomicAdd(loss, S.loss);
+    if (t == 0) {
+        out[OFF_B3] = S.gb3[0] + S.gb3[1];
+        out[NP] = S.loss[0] + S.loss[1];
     }
 }
 
-__global__ void k_adam(float *__restrict__ P, const float *__restrict__ g, float *__restrict__ m,
-                       float *__restrict__ v, float lr, float b1, float b2, float eps, float c1,
-                       float c2) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= NP) return;
-    const float gk = g[k];
-    const float mk = b1 * m[k] + (1.f - b1) * gk;
-    const float vk = b2 * v[k] + (1.f - b2) * gk * gk;
-    m[k] = mk;
-    v[k] = vk;
-    P[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
+// The sum of the blocks' slots, 32 values per block of 8 warps (each warp a
+// stride of the slots, in order), then either the gradient and loss as they
+// are, or one Adam step of the parameter with its packed BF16 copies: one
+// launch in place of two clears, Adam and the packing.
+struct AdamArgs {
+    float *P, *m, *v;
+    __nv_bfloat16 *pk;
+    float lr, b1, b2, eps, c1, c2;
+};
+template <bool ADAM>
+__global__ void __launch_bounds__(256)
+    k_mlp_update(int nblk, const float *__restrict__ part, float *__restrict__ grad,
+                 float *__restrict__ loss, AdamArgs A) {
+    __shared__ float sum[8][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k = blockIdx.x * 32 + lane;
+    grid_wait();
+    grid_release();
+    float s = 0.f;
+    if (k <= NP) {
+#pragma unroll 8
+        for (int b = w; b < nblk; b += 8) s += part[(size_t)b * NPART + k];
+    }
+    sum[w][lane] = s;
+    __syncthreads();
+    if (w || k > NP) return;
+#pragma unroll
+    for (int q = 1; q < 8; q++) s += sum[q][lane];
+    if (k == NP) {
+        *loss = s;
+        return;
+    }
+    if (!ADAM) {
+        grad[k] = s;
+        return;
+    }
+    const float mk = A.b1 * A.m[k] + (1.f - A.b1) * s;
+    const float vk = A.b2 * A.v[k] + (1.f - A.b2) * s * s;
+    A.m[k] = mk;
+    A.v[k] = vk;
+    const float p = A.P[k] - A.lr * (mk / A.c1) / (sqrtf(vk / A.c2) + A.eps);
+    A.P[k] = p;
+    const __nv_bfloat16 pb = __float2bfloat16_rn(p);
+    if (k < OFF_B1) {
+        A.pk[PK_W1T + (k % H) * 16 + k / H] = pb;
+    } else if (k >= OFF_W2 && k < OFF_B2) {
+        const int i = (k - OFF_W2) / H, j = (k - OFF_W2) % H;
+        A.pk[PK_W2T + j * H + i] = pb;
+        A.pk[PK_W2 + i * H + j] = pb;
+    }
 }
 
 // Surrogate prediction for the 32 rows of one warp (two 16-row MMA tiles):
@@ -897,50 +1032,73 @@ int mlp_forward_dev(sph_ctx *ctx, int n, const float *X, float *y) {
     return ctx_check_launch(ctx, "mlp_forward");
 }
 
-static int grad_launch(sph_ctx *ctx, int n, const float *X, const float *t, float inv_n) {
-    const size_t sm = sizeof(GradSmem);
-    static bool attr = false;
-    if (!attr) {
-        CK(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        attr = true;
-    }
-    k_mlp_grad<<<div_up(n, GR), 128, sm, ctx->stream>>>(
-        n, X, t, inv_n, (const __nv_bfloat16 *)ctx->mlp_bf16, ctx->mlp, ctx->mlp_grad,
-        ctx->mlp_scratch);
-    return ctx_check_launch(ctx, "mlp_grad");
+// the gradient's block slots, kept from the first training call on
+static int ensure_part(sph_ctx *ctx) {
+    if (ctx->mlp_part) return SPH_OK;
+    const size_t bytes = sizeof(float) * NPART * (size_t)ctx->num_sms * GBLOCKS;
+    void *q = nullptr;
+    CK(cudaMalloc(&q, bytes));
+    ctx->allocs.push_back(q);
+    ctx->dev_bytes += bytes;
+    ctx->mlp_part = (float *)q;
+    return SPH_OK;
+}
+
+// launch in programmatic stream order (see grid_wait)
+template <class... P, class... Q>
+static cudaError_t launch_after(cudaStream_t s, int grid, int block, void (*kern)(P...), Q... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
+// gradient of n rows into the slots; *nblk of them are written
+static int grad_launch(sph_ctx *ctx, int n, const float *X, const float *t, float inv_n, int *nblk) {
+    int rc = ensure_part(ctx);
+    if (rc) return rc;
+    *nblk = min(div_up(n, GROWS), ctx->num_sms * GBLOCKS);
+    CK(launch_after(ctx->stream, *nblk, 256, k_mlp_grad, n, X, t, inv_n,
+                    (const __nv_bfloat16 *)ctx->mlp_bf16, ctx->mlp, ctx->mlp_part));
+    return SPH_OK;
 }
 
 int mlp_grad_dev(sph_ctx *ctx, int n, const float *X, const float *t, float *grad, float *loss) {
     if (n <= 0) return SPH_ERR_ARG;
-    CK(cudaMemsetAsync(ctx->mlp_grad, 0, sizeof(float) * NP, ctx->stream));
-    CK(cudaMemsetAsync(ctx->mlp_scratch, 0, sizeof(float), ctx->stream));
-    int rc = grad_launch(ctx, n, X, t, 1.0f / n);
+    int nblk;
+    int rc = grad_launch(ctx, n, X, t, 1.0f / n, &nblk);
     if (rc) return rc;
+    CK(launch_after(ctx->stream, div_up(NP + 1, 32), 256, k_mlp_update<false>, nblk, ctx->mlp_part,
+                    ctx->mlp_grad, ctx->mlp_scratch, AdamArgs{}));
     if (grad) CK(cudaMemcpyAsync(grad, ctx->mlp_grad, sizeof(float) * NP, cudaMemcpyDeviceToDevice,
                                  ctx->stream));
     if (loss) CK(cudaMemcpyAsync(loss, ctx->mlp_scratch, sizeof(float), cudaMemcpyDeviceToDevice,
                                  ctx->stream));
-    return SPH_OK;
+    return ctx_check_launch(ctx, "mlp_update");
 }
 
 int mlp_train_dev(sph_ctx *ctx, int n, const float *X, const float *t, int batch, int nsteps,
                   float lr, float *loss_out) {
     if (n <= 0 || batch <= 0 || nsteps < 0) return SPH_ERR_ARG;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    AdamArgs A{ctx->mlp, ctx->mlp_m, ctx->mlp_v, (__nv_bfloat16 *)ctx->mlp_bf16, lr, 0.9f, 0.999f, 1e-8f, 0.f, 0.f};
     const int nb = max(1, n / batch);
     for (int s = 0; s < nsteps; s++) {
         const int b = s % nb;
         const int rows = min(batch, n - b * batch);
-        CK(cudaMemsetAsync(ctx->mlp_grad, 0, sizeof(float) * NP, ctx->stream));
-        CK(cudaMemsetAsync(ctx->mlp_scratch, 0, sizeof(float), ctx->stream));
-        int rc = grad_launch(ctx, rows, X + 3 * (size_t)b * batch, t + (size_t)b * batch, 1.0f / rows);
+        int nblk;
+        int rc = grad_launch(ctx, rows, X + 3 * (size_t)b * batch, t + (size_t)b * batch, 1.0f / rows, &nblk);
         if (rc) return rc;
         ctx->mlp_step++;
-        const float c1 = 1.f - powf(b1, (float)ctx->mlp_step), c2 = 1.f - powf(b2, (float)ctx->mlp_step);
-        k_adam<<<div_up(NP, 256), 256, 0, ctx->stream>>>(ctx->mlp, ctx->mlp_grad, ctx->mlp_m,
-                                                         ctx->mlp_v, lr, b1, b2, eps, c1, c2);
-        rc = mlp_pack(ctx);
-        if (rc) return rc;
+        A.c1 = 1.f - powf(A.b1, (float)ctx->mlp_step);
+        A.c2 = 1.f - powf(A.b2, (float)ctx->mlp_step);
+        CK(launch_after(ctx->stream, div_up(NP + 1, 32), 256, k_mlp_update<true>, nblk, ctx->mlp_part,
+                        nullptr, ctx->mlp_scratch, A));
     }
     if (loss_out)
         CK(cudaMemcpyAsync(loss_out, ctx->mlp_scratch, sizeof(float), cudaMemcpyDeviceToHost,

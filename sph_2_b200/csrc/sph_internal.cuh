@@ -162,6 +162,7 @@ struct sph_ctx {
     void *mlp_bf16 = nullptr;      // packed BF16 weights for the tensor-core kernels
     float *mlp_grad = nullptr, *mlp_m = nullptr, *mlp_v = nullptr;
     float *mlp_scratch = nullptr;
+    float *mlp_part = nullptr;     // per-block gradient slots (allocated on first use)
     int *cool_list = nullptr;      // surrogate fallback rows (n_max) + their count
     // table cooling: grids (kpc, nH, Z, T, time), u after each time, ion
     // fractions, and the ion fractions of the last call per storage slot
