@@ -372,8 +372,7 @@ int sph_ctx_create(const sph_config *cfg, sph_ctx **out) {
     DAF(tmpb, rs * N); ctx->pw = tmpb;
     DAF(ctx->key[0], N); DAF(ctx->key[1], N); DAF(ctx->key_in, N);
     DAF(ctx->val[0], N); DAF(ctx->val[1], N);
-    ctx->sort_blocks = div_up(N, 2048);
-    DAF(ctx->hist, 256 * (size_t)ctx->sort_blocks + 256);
+    DAF(ctx->hist, sort_scratch(N));
     DAF(ctx->box, 6 * C);
     DAF(ctx->corg, 3 * C);
     DAF(ctx->cloud_start, C + 1);

@@ -8,13 +8,16 @@
 // FP64 min/max (order independent), keys are computed with the roundings
 // spelled out so they equal the oracle's bit for bit, and the sort is stable
 // so the permutation is a pure function of (keys, storage order).
+#include <algorithm>
+#include <cuda/atomic>
+
 #include "sph_internal.cuh"
 
 namespace {
 
-constexpr int SORT_THREADS = 256;
-constexpr int SORT_ITEMS = 8;
-constexpr int SORT_TILE = SORT_THREADS * SORT_ITEMS;
+constexpr int SORT_THREADS = 256, SORT_WARPS = SORT_THREADS / 32;
+constexpr int SORT_PASSES = 8;  // 8-bit digits of the 63-bit key
+static_assert(SORT_PASSES % 2 == 0, "the sorted keys and values end in buffer 0");
 
 __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
     for (int o = 16; o > 0; o >>= 1) {
@@ -116,12 +119,9 @@ __device__ __forceinline__ unsigned long long cell_coord(double x, double lo, do
 
 // key = (cloud << 3*bits) | interleave(ix, iy, iz), x in the top bit of each
 // triple; cubic cells of side ext/2^bits with ext the box's largest side
-__global__ void k_keys(const double *__restrict__ x, const double *__restrict__ y,
-                       const double *__restrict__ z, const int *__restrict__ cloud, int n,
-                       const unsigned long long *__restrict__ box, int bits,
-                       unsigned long long *__restrict__ key) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+__device__ __forceinline__ unsigned long long morton_key(
+    const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
+    const int *__restrict__ cloud, int i, const unsigned long long *__restrict__ box, int bits) {
     int c = cloud[i];
     double lo[3], hi[3];
     for (int d = 0; d < 3; d++) {
@@ -133,115 +133,195 @@ __global__ void k_keys(const double *__restrict__ x, const double *__restrict__ 
     unsigned long long ix = cell_coord(x[i], lo[0], ext, bits);
     unsigned long long iy = cell_coord(y[i], lo[1], ext, bits);
     unsigned long long iz = cell_coord(z[i], lo[2], ext, bits);
-    key[i] = ((unsigned long long)c << (3 * bits)) | (spread3(ix) << 2) | (spread3(iy) << 1) |
-             spread3(iz);
+    return ((unsigned long long)c << (3 * bits)) | (spread3(ix) << 2) | (spread3(iy) << 1) |
+           spread3(iz);
 }
 
-// ---- LSD radix sort, 8-bit digits ----
-// hist layout: hist[d * nb + b] (digit major) so one scan per digit gives the
-// block offsets; tot[d] = count of digit d over all blocks.
+// ---- stable LSD radix sort, 8-bit digits, one launch per digit ----
+// A digit's counts do not depend on the order of the keys, so k_keys counts all
+// eight digits while it makes the keys (tot[pass][digit]).  A pass then reads
+// each key once: its tiles take their place among equal digits of earlier
+// tiles by a decoupled look-back (Merrill and Garland, 2016): every tile
+// publishes its digit counts, adds up those of the tiles before it until one
+// has published the sum of all up to itself, and publishes its own sum.  Tiles
+// are numbered in the order in which they start, so a tile only waits for
+// tiles that run or have run.  (Three launches a digit -- histogram, scan and a
+// scatter of 8 rounds with five barriers each -- took 17.4 us of 10k to 100k
+// particles and 28 us of 1M; one takes 4.9, 7.7 and 24.8.)
+// state[tile][digit]: 0 not yet, LOCAL | count of the tile, TOTAL | count up to
+// and including it.
+constexpr unsigned LOCAL = 1u << 30, TOTAL = 2u << 30, VALUE = (1u << 30) - 1u;
+constexpr int LOOK = 4;  // tiles read per step of the look-back (8, 16: 1 to 4 % slower)
+constexpr int LOOK_LIMIT = 1 << 22;  // polls before a wait gives up
+
 __global__ void __launch_bounds__(SORT_THREADS)
-    k_radix_hist(const unsigned long long *__restrict__ kin, int n, int shift, int nb,
-                 unsigned *__restrict__ hist) {
-    __shared__ unsigned h[256];
-    int t = threadIdx.x;
-    h[t] = 0;
+    k_keys(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
+           const int *__restrict__ cloud, int n, const unsigned long long *__restrict__ box, int bits,
+           unsigned long long *__restrict__ key, unsigned *__restrict__ tot) {
+    __shared__ unsigned h[SORT_PASSES][256];
+    for (int k = threadIdx.x; k < SORT_PASSES * 256; k += SORT_THREADS) (&h[0][0])[k] = 0u;
     __syncthreads();
-    int base = blockIdx.x * SORT_TILE;
+    for (int i = blockIdx.x * SORT_THREADS + threadIdx.x; i < n; i += gridDim.x * SORT_THREADS) {
+        const unsigned long long v = morton_key(x, y, z, cloud, i, box, bits);
+        key[i] = v;
 #pragma unroll
-    for (int k = 0; k < SORT_ITEMS; k++) {
-        int idx = base + k * SORT_THREADS + t;
-        if (idx < n) atomicAdd(&h[(unsigned)(kin[idx] >> shift) & 255u], 1u);
+        for (int p = 0; p < SORT_PASSES; p++) atomicAdd(&h[p][(unsigned)(v >> (8 * p)) & 255u], 1u);
     }
     __syncthreads();
-    hist[t * nb + blockIdx.x] = h[t];
+    for (int k = threadIdx.x; k < SORT_PASSES * 256; k += SORT_THREADS)
+        if (const unsigned c = (&h[0][0])[k]) atomicAdd(&tot[k], c);
 }
 
-// one block per digit: exclusive scan of hist[d*nb .. d*nb+nb-1] in place
-__global__ void __launch_bounds__(256) k_radix_scan(unsigned *hist, int nb, unsigned *tot) {
-    __shared__ unsigned part[256];
-    int d = blockIdx.x, t = threadIdx.x;
-    unsigned *row = hist + (size_t)d * nb;
-    int per = (nb + 255) / 256;
-    int a = t * per, b = min(nb, a + per);
-    unsigned s = 0;
-    for (int i = a; i < b; i++) s += row[i];
-    part[t] = s;
+// exclusive sum over the block's 256 threads
+__device__ __forceinline__ unsigned scan256(unsigned v, unsigned *tmp) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) tmp[w] = x;
     __syncthreads();
-    // inclusive scan of the 256 partials (Hillis-Steele)
-    for (int o = 1; o < 256; o <<= 1) {
-        unsigned v = t >= o ? part[t - o] : 0;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
-    }
-    unsigned run = t ? part[t - 1] : 0;
-    for (int i = a; i < b; i++) {
-        unsigned v = row[i];
-        row[i] = run;
-        run += v;
-    }
-    if (t == 255) tot[d] = part[255];
+    unsigned before = 0;
+#pragma unroll
+    for (int k = 0; k < SORT_WARPS; k++) before += k < w ? tmp[k] : 0u;
+    return before + x - v;
 }
 
-// Stable scatter.  Item k of thread t of block b is element b*TILE + k*256 + t,
-// so the loop over k (and warps, lanes) walks the tile in storage order; the
-// rank of an element among equal digits is (count in earlier k) + (count in
-// earlier warps of this k) + (lower lanes of its warp with the same digit).
+// One digit.  Warp w of a tile holds its elements 32 ITEMS w .., item k of lane l
+// the one at 32 k + l of them, so tile, warp, item, lane is the storage order.
+// EXCHANGE: the tile is put in digit order in shared memory first, so that equal
+// digits leave in runs (64 bytes on average of 2048 keys) instead of one by one
+template <int ITEMS, bool EXCHANGE>
 __global__ void __launch_bounds__(SORT_THREADS)
-    k_radix_scatter(const unsigned long long *__restrict__ kin, const int *__restrict__ vin,
-                    unsigned long long *__restrict__ kout, int *__restrict__ vout, int n,
-                    int shift, int nb, const unsigned *__restrict__ hist,
-                    const unsigned *__restrict__ tot) {
-    constexpr int NW = SORT_THREADS / 32;
-    __shared__ unsigned s_base[256];
-    __shared__ unsigned s_run[256];
-    __shared__ unsigned s_cnt[NW][257];
-    int t = threadIdx.x, w = t >> 5, lane = t & 31;
-    // exclusive scan of the digit totals
-    s_run[t] = tot[t];
+    k_radix_pass(const unsigned long long *__restrict__ kin, const int *__restrict__ vin,
+                 unsigned long long *__restrict__ kout, int *__restrict__ vout, int n, int shift,
+                 const unsigned *__restrict__ tot, unsigned *state, unsigned *ticket,
+                 long long *status) {
+    __shared__ unsigned cnt[SORT_WARPS][256];  // counts, then places, per warp and digit
+    __shared__ unsigned tmp[SORT_WARPS], tmp2[SORT_WARPS];
+    __shared__ int stile;
+    __shared__ unsigned long long xkey[EXCHANGE ? SORT_THREADS * ITEMS : 1];
+    __shared__ int xval[EXCHANGE ? SORT_THREADS * ITEMS : 1];
+    __shared__ unsigned to[EXCHANGE ? 256 : 1];  // from a place in the tile to the output
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    if (t == 0) stile = (int)atomicAdd(ticket, 1u);
+    for (int k = t; k < SORT_WARPS * 256; k += SORT_THREADS) (&cnt[0][0])[k] = 0u;
     __syncthreads();
-    for (int o = 1; o < 256; o <<= 1) {
-        unsigned v = t >= o ? s_run[t - o] : 0;
-        __syncthreads();
-        s_run[t] += v;
-        __syncthreads();
-    }
-    unsigned excl = s_run[t] - tot[t];
-    __syncthreads();
-    s_base[t] = excl + hist[t * nb + blockIdx.x];
-    s_run[t] = 0;
+    const int tile = stile;
+    const int base = (tile * SORT_WARPS + w) * (32 * ITEMS) + lane;
     const unsigned lt = (1u << lane) - 1u;
-    int base = blockIdx.x * SORT_TILE;
-    for (int k = 0; k < SORT_ITEMS; k++) {
-        int idx = base + k * SORT_THREADS + t;
-        bool ok = idx < n;
-        unsigned long long key = ok ? kin[idx] : 0ULL;
-        int val = ok ? (vin ? vin[idx] : idx) : 0;
-        unsigned d = ok ? (unsigned)(key >> shift) & 255u : 256u;
-        for (int j = lane; j < 257; j += 32) s_cnt[w][j] = 0;
+    unsigned long long key[ITEMS];
+    unsigned place[ITEMS];
+    int val[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const int idx = base + 32 * k;
+        key[k] = idx < n ? kin[idx] : 0ull;
+        val[k] = idx < n && vin ? vin[idx] : idx;
+    }
+    // place among the warp's earlier equal digits
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const bool ok = base + 32 * k < n;
+        const unsigned d = (unsigned)(key[k] >> shift) & 255u;
+        const unsigned peers = __match_any_sync(0xffffffffu, ok ? d : 256u);
+        const unsigned before = ok ? cnt[w][d] : 0u;
+        __syncwarp();
+        place[k] = before + __popc(peers & lt);
+        if (ok && (peers & lt) == 0) cnt[w][d] = before + __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    // thread t owns digit t: the tile's count, the warps' places in it, and the
+    // count of the tiles before
+    unsigned sum = 0;
+#pragma unroll
+    for (int k = 0; k < SORT_WARPS; k++) {
+        const unsigned c = cnt[k][t];
+        cnt[k][t] = sum;
+        sum += c;
+    }
+    cuda::atomic_ref<unsigned, cuda::thread_scope_device> mine(state[(size_t)tile * 256 + t]);
+    mine.store((tile == 0 ? TOTAL : LOCAL) | sum, cuda::memory_order_relaxed);
+    const unsigned start = scan256(tot[t], tmp);  // where digit t begins
+    unsigned prev = 0;
+    if (tile > 0) {
+        int spins = 0;
+        for (int b = tile - 1; b >= 0;) {
+            // up to LOOK earlier tiles at a time
+            unsigned v[LOOK];
+#pragma unroll
+            for (int q = 0; q < LOOK; q++)
+                v[q] = b - q >= 0 ? cuda::atomic_ref<unsigned, cuda::thread_scope_device>(
+                                        state[(size_t)(b - q) * 256 + t])
+                                        .load(cuda::memory_order_relaxed)
+                                  : (unsigned)TOTAL;
+            bool end = false, stall = false;
+#pragma unroll
+            for (int q = 0; q < LOOK; q++) {
+                if (!end && !stall) {
+                    if (v[q] == 0u) {
+                        stall = true;
+                    } else {
+                        prev += v[q] & VALUE;
+                        end = (v[q] & TOTAL) != 0u;
+                        b--;
+                    }
+                }
+            }
+            if (end) break;
+            if (stall && ++spins > LOOK_LIMIT) {
+                status_add(status, SPH_S_WAIT_TIMEOUT, 1);
+                break;
+            }
+        }
+        mine.store(TOTAL | (prev + sum), cuda::memory_order_relaxed);
+    }
+    const unsigned at = start + prev;
+    if constexpr (EXCHANGE) {
+        const unsigned in_tile = scan256(sum, tmp2);
+        to[t] = at - in_tile;
+#pragma unroll
+        for (int k = 0; k < SORT_WARPS; k++) cnt[k][t] += in_tile;
         __syncthreads();
-        unsigned peers = __match_any_sync(0xffffffffu, d);
-        unsigned r = __popc(peers & lt);
-        if (r == 0) s_cnt[w][d] = __popc(peers);
-        __syncthreads();
-        unsigned pre = r;
-        if (ok) {
-            pre += s_run[d];
-            for (int ww = 0; ww < w; ww++) pre += s_cnt[ww][d];
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            if (base + 32 * k < n) {
+                const unsigned p = cnt[w][(unsigned)(key[k] >> shift) & 255u] + place[k];
+                xkey[p] = key[k];
+                xval[p] = val[k];
+            }
         }
         __syncthreads();
-        {
-            unsigned add = 0;
-            for (int ww = 0; ww < NW; ww++) add += s_cnt[ww][t];
-            s_run[t] += add;
+        const int in = min(n - tile * SORT_THREADS * ITEMS, SORT_THREADS * ITEMS);
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const int p = k * SORT_THREADS + t;
+            if (p < in) {
+                const unsigned long long v = xkey[p];
+                const unsigned pos = to[(unsigned)(v >> shift) & 255u] + (unsigned)p;
+                if (pos < (unsigned)n) {  // (always, unless a wait gave up)
+                    kout[pos] = v;
+                    vout[pos] = xval[p];
+                }
+            }
         }
-        if (ok) {
-            unsigned pos = s_base[d] + pre;
-            kout[pos] = key;
-            vout[pos] = val;
+    } else {
+#pragma unroll
+        for (int k = 0; k < SORT_WARPS; k++) cnt[k][t] += at;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            if (base + 32 * k < n) {
+                const unsigned pos = cnt[w][(unsigned)(key[k] >> shift) & 255u] + place[k];
+                if (pos < (unsigned)n) {
+                    kout[pos] = key[k];
+                    vout[pos] = val[k];
+                }
+            }
         }
-        __syncthreads();  // s_cnt is cleared again by the next item
     }
 }
 
@@ -293,6 +373,25 @@ __global__ void k_permute(int n, const int *__restrict__ perm, const PermTab tab
 
 }  // namespace
 
+// Elements per thread of a pass, by the number of particles: a cloud that would
+// leave SMs without a tile takes small ones, and putting a tile in digit order
+// first pays where the chip's writes and not a tile's latency bound the pass.
+// us per pass with 2 / 4 / 8 elements, the last exchanging:  3k 4.0 / 4.8 / -;
+// 30k 5.9 / 6.4 / -;  65k 7.1 / 7.1 / 7.7;  100k 8.7 / 7.7 / 8.1;  200k 12.6 /
+// 10.9 / 9.0;  1M - / 29 / 24.8
+constexpr int SORT_N2 = 50000, SORT_N4 = 130000;
+static int sort_items(int n) { return n <= SORT_N2 ? 2 : n <= SORT_N4 ? 4 : 8; }
+static int sort_tiles(int n) { return div_up(n, SORT_THREADS * sort_items(n)); }
+
+// words of sort scratch for up to n particles: counts of the eight digits, a
+// ticket counter and tile states per pass
+size_t sort_scratch(size_t n) {
+    int tiles = sort_tiles((int)n);
+    if (n > SORT_N2) tiles = std::max(tiles, sort_tiles(SORT_N2));
+    if (n > SORT_N4) tiles = std::max(tiles, sort_tiles(SORT_N4));
+    return SORT_PASSES * 257 + (size_t)SORT_PASSES * 256 * tiles;
+}
+
 static int morton_bits_for(int ncloud) {
     int cb = 0;
     while ((1 << cb) < ncloud) cb++;
@@ -333,30 +432,25 @@ int launch_sort(sph_ctx *ctx) {
     k_box<<<div_up(n, 256), 256, 0, s>>>(st[ST_X], st[ST_Y], st[ST_Z], ctx->cloud[c], n, ctx->box,
                                          ctx->status);
     k_origin<<<div_up(ctx->ncloud, 128), 128, 0, s>>>(ctx->box, ctx->ncloud, ctx->corg);
-    const int bits = morton_bits_for(ctx->ncloud);
-    k_keys<<<div_up(n, 256), 256, 0, s>>>(st[ST_X], st[ST_Y], st[ST_Z], ctx->cloud[c], n, ctx->box,
-                                          bits, ctx->key_in);
-    const int used = 63;
-    const int passes = (used + 7) / 8;
-    const int nb = div_up(n, SORT_TILE);
-    unsigned *tot = ctx->hist + (size_t)256 * nb;
+    const int tiles = sort_tiles(n);
+    unsigned *tot = ctx->hist, *ticket = tot + SORT_PASSES * 256, *state = ticket + SORT_PASSES;
+    CK(cudaMemsetAsync(ctx->hist, 0,
+                       sizeof(unsigned) * (SORT_PASSES * 257 + (size_t)SORT_PASSES * 256 * tiles), s));
+    k_keys<<<std::min(div_up(n, SORT_THREADS), 4 * ctx->num_sms), SORT_THREADS, 0, s>>>(
+        st[ST_X], st[ST_Y], st[ST_Z], ctx->cloud[c], n, ctx->box, morton_bits_for(ctx->ncloud),
+        ctx->key_in, tot);
+    const auto pass = sort_items(n) == 2   ? k_radix_pass<2, false>
+                      : sort_items(n) == 4 ? k_radix_pass<4, false>
+                                           : k_radix_pass<8, true>;
     const unsigned long long *kin = ctx->key_in;
     const int *vin = nullptr;
-    int outb = 1;
-    for (int p = 0; p < passes; p++) {
-        int shift = 8 * p;
-        unsigned long long *kout = ctx->key[outb];
-        int *vout = ctx->val[outb];
-        k_radix_hist<<<nb, SORT_THREADS, 0, s>>>(kin, n, shift, nb, ctx->hist);
-        k_radix_scan<<<256, 256, 0, s>>>(ctx->hist, nb, tot);
-        k_radix_scatter<<<nb, SORT_THREADS, 0, s>>>(kin, vin, kout, vout, n, shift, nb, ctx->hist,
-                                                    tot);
-        kin = kout;
-        vin = vout;
-        outb ^= 1;
+    for (int p = 0; p < SORT_PASSES; p++) {
+        const int o = (p + 1) & 1;
+        pass<<<tiles, SORT_THREADS, 0, s>>>(kin, vin, ctx->key[o], ctx->val[o], n, 8 * p, tot + 256 * p,
+                                            state + (size_t)p * 256 * tiles, ticket + p, ctx->status);
+        kin = ctx->key[o];
+        vin = ctx->val[o];
     }
-    // passes is even, so the sorted keys/values end in buffer 0
-    static_assert(((63 + 7) / 8) % 2 == 0, "radix pass count must be even");
     ctx->perm = ctx->val[0];
     const int d = c ^ 1;
     PermTab tab;

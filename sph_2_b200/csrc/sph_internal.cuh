@@ -83,8 +83,7 @@ struct sph_ctx {
     int *val[2] = {};
     unsigned long long *key_in = nullptr;  // keys of the storage order before the last sort
     int *perm = nullptr;         // permutation of the last sort
-    unsigned *hist = nullptr;    // radix histograms
-    int sort_blocks = 0;
+    unsigned *hist = nullptr;    // radix digit counts, tickets and tile states (sort_scratch words)
     unsigned long long *box = nullptr;  // per cloud 6 ordered-uint64 (min xyz, max xyz)
     // per cloud: the origin of the mixed walk's FP32 coordinates (x, y, z; the
     // centre of the cloud's box at the last sort, 0 before the first)
@@ -369,6 +368,7 @@ enum { WQ_WALK = 0, WQ_SG_WALK = 1, WQ_SEARCH = 2, WQ_N = 3 };
 
 // ---- host-side launch helpers implemented per translation unit ----
 int launch_sort(sph_ctx *ctx);
+size_t sort_scratch(size_t n);
 int launch_sort_refit(sph_ctx *ctx);
 int launch_scan(sph_ctx *ctx, const int *in, int *out, int n, int *total);
 int launch_groups(sph_ctx *ctx);
