@@ -64,6 +64,8 @@ int queue_launch(sph_ctx *ctx, cudaStream_t s, int slot, const void *kernel, int
 
 namespace {
 
+constexpr int LOAD_STAGE = 16384;  // largest load from host arrays through pinned staging
+
 template <class T>
 int dalloc(sph_ctx *ctx, T **p, size_t count) {
     size_t bytes = std::max<size_t>(count * sizeof(T), 256);
@@ -100,6 +102,61 @@ __global__ void k_gather_by_id(int n, const int *__restrict__ id, const double *
                                double *__restrict__ dst) {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < n) dst[s] = src[id[s]];
+}
+
+// A load in one kernel: the state from the caller's eight arrays (a null one
+// is zeros), the identity order, zeroed results, the packed records, and for
+// one cloud its tables.  (Fourteen copies and clears of a few microseconds each
+// before.)
+struct LoadArgs {
+    const double *src[8], *u;  // x y z vx vy vz m h, and u
+    double *st[ST_N];
+    int *id, *cloud, *cloud_start;
+    double *asph, *agrav, *divV, *curlV, *pot;
+    double4 *p0;
+    const double *corg;
+    double *dt;
+    unsigned long long *dt_bits;
+    double dt0;
+    int one_cloud;
+};
+template <class R>
+__global__ void k_load(int n, LoadArgs a, typename R4<R>::T *__restrict__ p1,
+                       typename R4<R>::T *__restrict__ pw) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a.one_cloud && i == 0) {
+        a.cloud_start[0] = 0;
+        a.cloud_start[1] = n;
+        a.dt[0] = a.dt0;
+        a.dt_bits[0] = ~0ull;
+    }
+    if (i >= n) return;
+    double v[ST_N];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = a.src[k] ? a.src[k][i] : 0.0;
+    v[ST_U] = a.u[i];
+    v[ST_DUDT_PREV] = v[ST_HNB] = 0.0;
+#pragma unroll
+    for (int k = 0; k < ST_N; k++) a.st[k][i] = v[k];
+    a.id[i] = i;
+    if (a.one_cloud) a.cloud[i] = 0;
+    const int c = a.one_cloud ? 0 : a.cloud[i];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        a.asph[(size_t)k * n + i] = 0.0;
+        a.agrav[(size_t)k * n + i] = 0.0;
+    }
+    a.divV[i] = a.curlV[i] = a.pot[i] = 0.0;
+    typename R4<R>::T q, w;
+    q.x = (R)v[ST_VX]; q.y = (R)v[ST_VY]; q.z = (R)v[ST_VZ]; q.w = (R)v[ST_M];
+    const double *org = a.corg + 3 * c;
+    w.x = (R)(v[ST_X] - WalkOrigin<R>::off(org, 0));
+    w.y = (R)(v[ST_Y] - WalkOrigin<R>::off(org, 1));
+    w.z = (R)(v[ST_Z] - WalkOrigin<R>::off(org, 2));
+    w.w = (R)v[ST_M];
+    p1[i] = q;
+    pw[i] = w;
+    a.p0[i] = make_double4(v[ST_X], v[ST_Y], v[ST_Z], v[ST_H]);
 }
 
 bool valid_lanes(int l) { return l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32; }
@@ -451,6 +508,7 @@ void sph_ctx_destroy(sph_ctx *ctx) {
     for (int k = 0; k < 4; k++)
         if (ctx->ev_io[k]) cudaEventDestroy(ctx->ev_io[k]);
     if (ctx->io_stage) cudaFree(ctx->io_stage);
+    if (ctx->load_stage) cudaFreeHost(ctx->load_stage);
     if (ctx->stream_io) cudaStreamDestroy(ctx->stream_io);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->stream_g) cudaStreamDestroy(ctx->stream_g);
@@ -520,53 +578,86 @@ int sph_load(sph_ctx *ctx, int32_t n, const int32_t *cloud, const double *x, con
     if (n > ctx->cfg.n_max) return SPH_ERR_CAPACITY;
     drop_graphs(ctx);
     CK(cudaStreamSynchronize(ctx->stream));
-    // clouds: counts per id on the host
-    std::vector<int> cl(n > 0 ? n : 1, 0);
+    cudaStream_t s = ctx->stream;
+    int ncl = 1;
+    std::vector<int> cl;
     if (cloud) {
+        // clouds: counts per id on the host
+        cl.resize(n > 0 ? n : 1, 0);
         if (host) memcpy(cl.data(), cloud, sizeof(int) * n);
         else CK(cudaMemcpy(cl.data(), cloud, sizeof(int) * n, cudaMemcpyDeviceToHost));
+        for (int i = 0; i < n; i++) {
+            if (cl[i] < 0 || cl[i] >= ctx->cfg.n_cloud_max) return SPH_ERR_CAPACITY;
+            ncl = std::max(ncl, cl[i] + 1);
+        }
+        std::vector<int> cnt(ncl, 0);
+        for (int i = 0; i < n; i++) cnt[cl[i]]++;
+        ctx->cloud_start_h.assign(ncl + 1, 0);
+        for (int k = 0; k < ncl; k++) ctx->cloud_start_h[k + 1] = ctx->cloud_start_h[k] + cnt[k];
+        if (n > 0) CK(cudaMemcpyAsync(ctx->cloud[0], cl.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
+    } else {
+        ctx->cloud_start_h = {0, n};
     }
-    int ncl = 1;
-    for (int i = 0; i < n; i++) {
-        if (cl[i] < 0 || cl[i] >= ctx->cfg.n_cloud_max) return SPH_ERR_CAPACITY;
-        ncl = std::max(ncl, cl[i] + 1);
-    }
-    std::vector<int> cnt(ncl, 0);
-    for (int i = 0; i < n; i++) cnt[cl[i]]++;
-    ctx->cloud_start_h.assign(ncl + 1, 0);
-    for (int k = 0; k < ncl; k++) ctx->cloud_start_h[k + 1] = ctx->cloud_start_h[k] + cnt[k];
     ctx->n = n;
     ctx->ncloud = ncl;
     ctx->ngroup = n + ncl;
     ctx->cur = 0;
-    cudaStream_t s = ctx->stream;
-    cudaMemcpyKind kind = host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
-    const double *src[ST_N] = {x, y, z, vx, vy, vz, m, h, u, nullptr};
-    for (int k = 0; k < ST_N; k++) {
-        if (n == 0) break;
-        if (src[k]) CK(cudaMemcpyAsync(ctx->st[0][k], src[k], sizeof(double) * n, kind, s));
-        else CK(cudaMemsetAsync(ctx->st[0][k], 0, sizeof(double) * n, s));
+    const double dt0 = ctx->cfg.dt_fixed > 0 ? ctx->cfg.dt_fixed : 0.0;
+    const std::vector<double> dts(ncl, dt0);
+    if (cloud || n == 0) {
+        CK(cudaMemcpyAsync(ctx->cloud_start, ctx->cloud_start_h.data(), sizeof(int) * (ncl + 1),
+                           cudaMemcpyHostToDevice, s));
+        CK(cudaMemsetAsync(ctx->dt_bits, 0xff, sizeof(unsigned long long) * ncl, s));
+        CK(cudaMemcpyAsync(ctx->dt, dts.data(), sizeof(double) * ncl, cudaMemcpyHostToDevice, s));
     }
-    if (n > 0) {
-        CK(cudaMemcpyAsync(ctx->cloud[0], cl.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
-        k_iota<<<div_up(n, 256), 256, 0, s>>>(n, ctx->id[0]);
-    }
-    CK(cudaMemcpyAsync(ctx->cloud_start, ctx->cloud_start_h.data(), sizeof(int) * (ncl + 1),
-                       cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(ctx->d_ngroup, 0, sizeof(int), s));
-    CK(cudaMemsetAsync(ctx->dt_bits, 0xff, sizeof(unsigned long long) * ncl, s));
-    {
-        std::vector<double> dt0(ncl, ctx->cfg.dt_fixed > 0 ? ctx->cfg.dt_fixed : 0.0);
-        CK(cudaMemcpyAsync(ctx->dt, dt0.data(), sizeof(double) * ncl, cudaMemcpyHostToDevice, s));
-    }
     if (n > 0) {
-        CK(cudaMemsetAsync(ctx->asph, 0, 3 * sizeof(double) * n, s));
-        CK(cudaMemsetAsync(ctx->agrav, 0, 3 * sizeof(double) * n, s));
-        CK(cudaMemsetAsync(ctx->divV, 0, sizeof(double) * n, s));
-        CK(cudaMemsetAsync(ctx->curlV, 0, sizeof(double) * n, s));
-        CK(cudaMemsetAsync(ctx->pot, 0, sizeof(double) * n, s));
-        rc = launch_pack_p1(ctx);
-        if (rc) return rc;
+        const double *in[9] = {x, y, z, vx, vy, vz, m, h, u};
+        if (host && n <= LOAD_STAGE) {
+            // small host arrays: gathered in pinned memory, one copy (nine
+            // pageable copies of 3k particles took 100 us); the candidate
+            // rows, invalid after a load, take it on the device
+            if (!ctx->load_stage)
+                CK(cudaHostAlloc((void **)&ctx->load_stage, sizeof(double) * 9 * LOAD_STAGE, cudaHostAllocDefault));
+            int k = 0;
+            double *dev = (double *)ctx->cand_idx;
+            for (const double *&q : in)
+                if (q) {
+                    memcpy(ctx->load_stage + (size_t)k * n, q, sizeof(double) * n);
+                    q = dev + (size_t)k * n;
+                    k++;
+                }
+            CK(cudaMemcpyAsync(dev, ctx->load_stage, sizeof(double) * k * n, cudaMemcpyHostToDevice, s));
+        } else if (host) {
+            for (int k = 0; k < 9; k++)
+                if (in[k]) {
+                    CK(cudaMemcpyAsync(ctx->st[0][k], in[k], sizeof(double) * n, cudaMemcpyHostToDevice, s));
+                    in[k] = ctx->st[0][k];
+                }
+        }
+        LoadArgs a;
+        for (int k = 0; k < 8; k++) a.src[k] = in[k];
+        a.u = in[8];
+        for (int k = 0; k < ST_N; k++) a.st[k] = ctx->st[0][k];
+        a.id = ctx->id[0];
+        a.cloud = ctx->cloud[0];
+        a.cloud_start = ctx->cloud_start;
+        a.asph = ctx->asph;
+        a.agrav = ctx->agrav;
+        a.divV = ctx->divV;
+        a.curlV = ctx->curlV;
+        a.pot = ctx->pot;
+        a.p0 = ctx->p0;
+        a.corg = ctx->corg;
+        a.dt = ctx->dt;
+        a.dt_bits = ctx->dt_bits;
+        a.dt0 = dt0;
+        a.one_cloud = cloud ? 0 : 1;
+        if (ctx->cfg.precision == SPH_PREC_MIXED)
+            k_load<float><<<div_up(n, 256), 256, 0, s>>>(n, a, (float4 *)ctx->p1, (float4 *)ctx->pw);
+        else
+            k_load<double><<<div_up(n, 256), 256, 0, s>>>(n, a, (double4 *)ctx->p1, (double4 *)ctx->pw);
+        if ((rc = launch_rows_invalidate(ctx))) return rc;
     }
     CK(cudaStreamSynchronize(s));
     ctx->tree_ok = ctx->lists_ok = ctx->rho_ok = ctx->divcurl_ok = ctx->cand_ok = false;
@@ -905,32 +996,41 @@ static int direct_common(sph_ctx *ctx, const double *eps, int32_t nt, const int3
     if (nt == 0) return SPH_OK;
     for (int t = 0; host && t < nt; t++)
         if (targets[t] < 0 || targets[t] >= ctx->n) return SPH_ERR_ARG;
-    int *dt_ = nullptr;
-    double *dout = nullptr, *deps = nullptr;
-    CK(cudaMalloc(&dt_, sizeof(int) * nt));
-    CK(cudaMalloc(&dout, sizeof(double) * width * nt));
-    cudaMemcpyKind kin = host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
-    // copies on the context's non-blocking stream, ordered before the kernels
-    CK(cudaMemcpyAsync(dt_, targets, sizeof(int) * nt, kin, ctx->stream));
+    const int *tg = targets;
+    double *res = out;
+    const double *ep = eps;
+    void *tmp = nullptr;  // device copies of host arrays: eps, results, targets
+    if (host) {
+        const size_t ne = eps ? ctx->n : 0, no = (size_t)width * nt;
+        CK(cudaMalloc(&tmp, sizeof(double) * (ne + no) + sizeof(int) * nt));
+        double *d = (double *)tmp;
+        ep = d;
+        res = d + ne;
+        int *t = (int *)(res + no);
+        tg = t;
+        // copies on the context's non-blocking stream, ordered before the kernels
+        cudaError_t e = cudaMemcpyAsync(t, targets, sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream);
+        if (e == cudaSuccess && eps)
+            e = cudaMemcpyAsync(d, eps, sizeof(double) * ctx->n, cudaMemcpyHostToDevice, ctx->stream);
+        if (e != cudaSuccess) {
+            cudaFree(tmp);
+            return ctx_fail(ctx, e, "cudaMemcpyAsync", __LINE__);
+        }
+    }
     if (eps) {
-        CK(cudaMalloc(&deps, sizeof(double) * ctx->n));
-        CK(cudaMemcpyAsync(deps, eps, sizeof(double) * ctx->n, kin, ctx->stream));
         // eps is given in the caller's original order: bring it to storage order
-        k_gather_by_id<<<div_up(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->n, ctx->id[ctx->cur],
-                                                                      deps, ctx->red);
-        rc = launch_gravity_direct_spline(ctx, ctx->red, nt, dt_, dout, nbeg,
-                                          nend < 0 ? ctx->n : nend);
+        k_gather_by_id<<<div_up(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->n, ctx->id[ctx->cur], ep,
+                                                                      ctx->red);
+        rc = launch_gravity_direct_spline(ctx, ctx->red, nt, tg, res, nbeg, nend < 0 ? ctx->n : nend);
     } else {
-        rc = launch_gravity_direct(ctx, nt, dt_, dout);
+        rc = launch_gravity_direct(ctx, nt, tg, res);
     }
-    if (!rc) {
-        CK(cudaMemcpyAsync(out, dout, sizeof(double) * width * nt,
-                           host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-    }
-    cudaFree(dt_);
-    cudaFree(dout);
-    if (deps) cudaFree(deps);
+    cudaError_t e = cudaSuccess;
+    if (!rc && host)
+        e = cudaMemcpyAsync(out, res, sizeof(double) * width * nt, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (tmp) cudaFree(tmp);
+    if (!rc && e != cudaSuccess) return ctx_fail(ctx, e, "direct sum", __LINE__);
     return rc;
 }
 

@@ -55,6 +55,7 @@ struct sph_ctx {
     cudaStream_t stream_io = nullptr;   // copies of sph_step_io (created on first use)
     double *io_stage = nullptr;         // io_slots x n_max doubles (allocated on first use)
     int io_slots = 0;
+    double *load_stage = nullptr;       // pinned staging of small host loads (allocated on first use)
     std::string err;
     int n = 0, ncloud = 0;
     std::vector<int> cloud_start_h;  // ncloud+1

@@ -78,16 +78,24 @@ def _is_cuda_tensor(a) -> bool:
     return hasattr(a, "is_cuda") and bool(getattr(a, "is_cuda"))
 
 
-def _column(a, k=None):
-    """A C-contiguous float64 column: (pointer, host flag, keep-alive)."""
-    if _is_cuda_tensor(a):
+def _columns(vectors, scalars):
+    """C-contiguous float64 columns, three of each (n, 3) array of `vectors` and
+    one of each array of `scalars`: (pointers, host flag, keep-alive).  CUDA
+    tensors take one kernel each and one synchronisation in all."""
+    kinds = {_is_cuda_tensor(a) for a in [*vectors, *scalars]}
+    if len(kinds) != 1:
+        raise ValueError("mix of host arrays and CUDA tensors in one call")
+    if kinds.pop():
         import torch
-        t = (a[:, k] if k is not None else a).to(torch.float64).contiguous()
-        # the library reads it on its own stream: let torch's work finish first
+        keep = [a[:, :3].to(torch.float64).t().contiguous() for a in vectors]
+        cols = [c for t in keep for c in t]
+        cols += [a.to(torch.float64).contiguous() for a in scalars]
+        # the library reads them on its own stream: let torch's work finish first
         torch.cuda.current_stream().synchronize()
-        return C.c_void_p(t.data_ptr()), 0, t
-    x = np.ascontiguousarray(np.asarray(a)[:, k] if k is not None else a, dtype=np.float64)
-    return x.ctypes.data_as(C.c_void_p), 1, x
+        return [C.c_void_p(c.data_ptr()) for c in cols], 0, cols
+    cols = [np.ascontiguousarray(np.asarray(a)[:, k], dtype=np.float64) for a in vectors for k in range(3)]
+    cols += [np.ascontiguousarray(a, dtype=np.float64) for a in scalars]
+    return [c.ctypes.data_as(C.c_void_p) for c in cols], 1, cols
 
 
 def _load_state(pos, m, h, v=None):
@@ -95,26 +103,13 @@ def _load_state(pos, m, h, v=None):
     bring it to Morton order with a fresh tree."""
     n = int(pos.shape[0])
     ctx = _ctx(n)
-    keep, args, hosts = [], [], set()
-    cols = [(pos, 0), (pos, 1), (pos, 2)]
-    cols += [(v, 0), (v, 1), (v, 2)] if v is not None else [None, None, None]
-    cols += [(m, None), (h, None)]
-    for c in cols:
-        if c is None:
-            args.append(None)
-            continue
-        p, host, k = _column(*c)
-        args.append(p)
-        hosts.add(host)
-        keep.append(k)
-    if len(hosts) != 1:
-        raise ValueError("mix of host arrays and CUDA tensors in one call")
-    host = hosts.pop()
-    u = np.zeros(n) if host else _zeros_like_dev(n)
-    pu = u.ctypes.data_as(C.c_void_p) if host else C.c_void_p(u.data_ptr())
-    x, y, z, vx, vy, vz, pm, ph = args
+    u = _zeros_like_dev(n) if _is_cuda_tensor(pos) else np.zeros(n)
+    ptrs, host, keep = _columns([pos] if v is None else [pos, v], [m, h, u])
+    x, y, z = ptrs[:3]
+    vx, vy, vz = (None, None, None) if v is None else ptrs[3:6]
+    pm, ph, pu = ptrs[-3:]
+    # returns when the copies have read `keep`
     ctx._chk(ctx._L.sph_load(ctx._h, n, None, x, y, z, vx, vy, vz, pm, ph, pu, host), "sph_load")
-    ctx.sync()   # the copies have read `keep` before it goes out of scope
     ctx.sort()
     ctx.build_tree()
     return ctx
@@ -135,21 +130,37 @@ def _zeros_like_dev(n):
     return torch.zeros(n, dtype=torch.float64, device="cuda")
 
 
-def _set(ctx, name, a):
-    p, host, keep = _column(a)
-    ctx._chk(ctx._L.sph_set_field(ctx._h, L.FIELD[name], p, host, 0), f"set {name}")
-    return keep
+def _ids_ptrs(names, ptrs):
+    return ((C.c_int32 * len(names))(*[L.FIELD[k] for k in names]),
+            (C.c_void_p * len(names))(*[p.value for p in ptrs]))
 
 
-def _out(ctx, name, like):
-    """Field in original order, as a NumPy array or (for CUDA inputs) a tensor."""
+def _set(ctx, fields):
+    """Several fields ({name: array}), those on the host and those on the device
+    in one library call each."""
+    for dev in (False, True):
+        part = {k: a for k, a in fields.items() if _is_cuda_tensor(a) == dev}
+        if part:
+            ptrs, host, keep = _columns([], list(part.values()))
+            ids, pp = _ids_ptrs(list(part), ptrs)
+            # returns when the copies have read `keep`
+            ctx._chk(ctx._L.sph_set_fields(ctx._h, len(part), ids, pp, host, 0), "set fields")
+
+
+def _out(ctx, names, like):
+    """A field in original order, or three as the columns of an (n, 3) array, as
+    a NumPy array or (for CUDA inputs) a tensor."""
+    one = isinstance(names, str)
+    names = [names] if one else list(names)
     if _is_cuda_tensor(like):
         import torch
-        t = torch.empty(ctx.n, dtype=torch.float64, device="cuda")
-        ctx._chk(ctx._L.sph_get_field(ctx._h, L.FIELD[name], C.c_void_p(t.data_ptr()), 0, 0),
-                 f"get {name}")
-        return t
-    return ctx.get(name)
+        t = torch.empty((len(names), ctx.n), dtype=torch.float64, device="cuda")
+        torch.cuda.current_stream().synchronize()   # earlier readers of its memory
+        ids, pp = _ids_ptrs(names, [C.c_void_p(r.data_ptr()) for r in t])
+        ctx._chk(ctx._L.sph_get_fields(ctx._h, len(names), ids, pp, 0, 0), "get fields")
+        return t[0] if one else t.t().contiguous()
+    got = ctx.get_fields(names)
+    return got[names[0]] if one else np.stack([got[k] for k in names], 1)
 
 
 def _rows(a, nbeg, nend):
@@ -179,7 +190,7 @@ def getDensity(pos, m, h):
 def div_curlVel_mpi(nbeg, nend, pos, v, rho, m, h):
     """shear.py:78-142: (|div v|, |curl v|) of rows nbeg..nend-1."""
     ctx = _load(pos, m, h, v)
-    _set(ctx, "rho", rho)
+    _set(ctx, {"rho": rho})
     ctx.divcurl()
     return (_rows(_out(ctx, "divV", pos), nbeg, nend), _rows(_out(ctx, "curlV", pos), nbeg, nend))
 
@@ -192,17 +203,13 @@ def div_curlVel(pos, v, rho, m, h):
 # ---- SPH accelerations and du/dt ------------------------------------------
 def _sph_pass(nbeg, nend, pos, v, rho, P, c, h, m, divV, curlV, want):
     ctx = _load(pos, m, h, v)
-    keep = [_set(ctx, "rho", rho), _set(ctx, "P", P), _set(ctx, "c", c)]
+    fields = {"rho": rho, "P": P, "c": c}
     if divV is not None:
-        keep += [_set(ctx, "divV", divV), _set(ctx, "curlV", curlV)]
+        fields.update(divV=divV, curlV=curlV)
+    _set(ctx, fields)
     if want == "acc":
         ctx.forces()
-        if _is_cuda_tensor(pos):
-            import torch
-            a = torch.stack([_out(ctx, f"a{k}_sph", pos) for k in "xyz"], 1)
-        else:
-            a = ctx.get_acc("sph")
-        return a[nbeg:nend]
+        return _out(ctx, ("ax_sph", "ay_sph", "az_sph"), pos)[nbeg:nend]
     ctx.dudt()
     return _rows(_out(ctx, "dudt", pos), nbeg, nend)
 
@@ -283,17 +290,33 @@ def getAcc_g_smth_mimj_mpi(nbeg, nend, pos, mass, G, epsilon):
     ctx.set_params(G=float(G))
     ones = np.ones(n) if not _is_cuda_tensor(pos) else _zeros_like_dev(n) + 1.0
     ctx = _load_state(pos, mass, ones)
+    if _is_cuda_tensor(pos):
+        return _spline_dev(ctx, n, nbeg, nend, epsilon, pos.device)
     eps = _host(epsilon)
     if (nbeg, nend) == (0, n):
         inv = np.empty(n, np.int32)
         inv[ctx.ids()] = np.arange(n, dtype=np.int32)  # storage slot of each particle
-        acc = ctx.gravity_direct_spline(eps, inv)
-    else:
-        acc = ctx.gravity_direct_spline_rows(eps, nbeg, nend)
-    if _is_cuda_tensor(pos):
-        import torch
-        return torch.from_numpy(acc).to(pos.device)
-    return acc
+        return ctx.gravity_direct_spline(eps, inv)
+    return ctx.gravity_direct_spline_rows(eps, nbeg, nend)
+
+
+def _spline_dev(ctx, n, nbeg, nend, epsilon, device):
+    """The field on device arrays, without a host round trip."""
+    import torch
+    if (nbeg, nend) != (0, n):
+        return torch.from_numpy(ctx.gravity_direct_spline_rows(_host(epsilon), nbeg, nend)).to(device)
+    eps = torch.as_tensor(epsilon, dtype=torch.float64, device="cuda").contiguous()
+    ids = torch.empty(n, dtype=torch.int32, device="cuda")
+    out = torch.empty((n, 3), dtype=torch.float64, device="cuda")
+    torch.cuda.current_stream().synchronize()
+    ctx._chk(ctx._L.sph_get_ids(ctx._h, C.c_void_p(ids.data_ptr()), 0), "ids")
+    slot = torch.empty_like(ids)                       # storage slot of each particle
+    slot[ids.long()] = torch.arange(n, dtype=torch.int32, device="cuda")
+    torch.cuda.current_stream().synchronize()
+    ctx._chk(ctx._L.sph_gravity_direct_spline(ctx._h, C.c_void_p(eps.data_ptr()), n,
+                                              C.c_void_p(slot.data_ptr()),
+                                              C.c_void_p(out.data_ptr()), 0), "gravity_direct_spline")
+    return out.to(device)
 
 
 def getPE(pos, m, G, epsilon):
