@@ -21,6 +21,8 @@
 // entries at once with the packed f32x2 arithmetic of sm_100 (__ffma2_rn /
 // __fmul2_rn), which halves the issued instructions of this issue-bound loop.
 // Each 32-term chunk is summed plainly and added to a plain accumulator.
+// k_walk is this with a warp per group, for FP32 clouds that fill the chip;
+// k_walk_block takes a block per group, for smaller ones and for FP64.
 // The FP32 walk with theta_local > 0 also sends far accepted cells through
 // per-group Taylor expansions, and starts each group from its super-group's
 // node list with the super-group's own expansion (k_sg_walk).
@@ -60,13 +62,6 @@ template <> __device__ __forceinline__ double rsq<double>(double x) { return rsq
 // slot rf[r] and at offset rs[r] of the pending stream (rs ascending; at most
 // 31 carried ranges + 32 appended by one round)
 constexpr int NRANGE = 64;
-
-template <class R> struct WalkSmem {
-    int stk[WSTK];
-    int clist[64];
-    int rf[NRANGE], rs[NRANGE];
-    typename R4<R>::T sa[32], sb[32], sc[32];
-};
 
 // FP32 staging as one array per field, so that a 64-bit shared load gives the
 // field of two consecutive entries for the packed f32x2 arithmetic
@@ -255,21 +250,136 @@ __device__ __forceinline__ void far_eval(const float *L, float ux, float uy, flo
     phi = L[19] - (L[0] * ux + L[1] * uy + L[2] * uz) - 0.5f * (ux * jx + uy * jy + uz * jz);
 }
 
-template <class R, bool POT>
-__global__ void __launch_bounds__(WALK_WARPS * 32, std::is_same<R, float>::value && !POT ? 6 : 1)
+// Field (and potential) of m staged cells at p, summed plainly.  FP32: field f
+// of cell k at f[f * LD + k], two cells per lane per instruction (f32x2), m even
+// (an odd chunk is padded with a massless, moment-free entry that adds zero).
+template <int LD, bool POT>
+__device__ __forceinline__ void cell_sums(const float *f, int m, const float4 &p, float eps2,
+                                          float &sx_, float &sy_, float &sz_, float &sp_) {
+    const float2 px = f2(p.x), py = f2(p.y), pz = f2(p.z), e2 = f2(eps2);
+    const float2 m1 = f2(-1.f), c15 = f2(1.5f), cm75 = f2(-7.5f), c3 = f2(3.f);
+    float2 sx = f2(0.f), sy = f2(0.f), sz = f2(0.f), spp = f2(0.f);
+#pragma unroll 4
+    for (int k = 0; k < m; k += 2) {
+        const float2 dx = __ffma2_rn(ld2(f + k), m1, px);
+        const float2 dy = __ffma2_rn(ld2(f + LD + k), m1, py);
+        const float2 dz = __ffma2_rn(ld2(f + 2 * LD + k), m1, pz);
+        float2 r2 = __ffma2_rn(dx, dx, e2);
+        r2 = __ffma2_rn(dy, dy, r2);
+        r2 = __ffma2_rn(dz, dz, r2);
+        const float2 rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+        const float2 ri2 = __fmul2_rn(rinv, rinv);
+        const float2 g3 = __fmul2_rn(rinv, ri2), g5 = __fmul2_rn(g3, ri2), g7 = __fmul2_rn(g5, ri2);
+        const float2 qxx = ld2(f + 4 * LD + k), qyy = ld2(f + 5 * LD + k), qzz = ld2(f + 6 * LD + k);
+        const float2 qxy = ld2(f + 7 * LD + k), qxz = ld2(f + 8 * LD + k), qyz = ld2(f + 9 * LD + k);
+        const float2 qx = __ffma2_rn(qxx, dx, __ffma2_rn(qxy, dy, __fmul2_rn(qxz, dz)));
+        const float2 qy = __ffma2_rn(qxy, dx, __ffma2_rn(qyy, dy, __fmul2_rn(qyz, dz)));
+        const float2 qz = __ffma2_rn(qxz, dx, __ffma2_rn(qyz, dy, __fmul2_rn(qzz, dz)));
+        const float2 dqd = __ffma2_rn(dx, qx, __ffma2_rn(dy, qy, __fmul2_rn(dz, qz)));
+        const float2 tr = ld2(f + 10 * LD + k), nm = ld2(f + 3 * LD + k);
+        const float2 a7 = __fmul2_rn(dqd, g7), b5 = __fmul2_rn(tr, g5);
+        // s = -M g3 + 1.5 tr g5 - 7.5 dqd g7
+        const float2 sc = __ffma2_rn(b5, c15, __ffma2_rn(a7, cm75, __fmul2_rn(nm, g3)));
+        const float2 t5 = __fmul2_rn(g5, c3);
+        sx = __ffma2_rn(t5, qx, __ffma2_rn(sc, dx, sx));
+        sy = __ffma2_rn(t5, qy, __ffma2_rn(sc, dy, sy));
+        sz = __ffma2_rn(t5, qz, __ffma2_rn(sc, dz, sz));
+        if (POT) {
+            // -(M rinv + 0.5 (3 dqd g5 - tr g3))
+            const float2 hq = __ffma2_rn(__fmul2_rn(dqd, g5), f2(1.5f),
+                                         __fmul2_rn(__fmul2_rn(tr, g3), f2(-0.5f)));
+            spp = __ffma2_rn(nm, rinv, spp);
+            spp = __ffma2_rn(hq, m1, spp);
+        }
+    }
+    sx_ = sx.x + sx.y;
+    sy_ = sy.x + sy.y;
+    sz_ = sz.x + sz.y;
+    sp_ = spp.x + spp.y;
+}
+template <bool POT, class R, class V4>
+__device__ __forceinline__ void cell_sums(const V4 *sa, const V4 *sb, const V4 *scc, int m, const V4 &p,
+                                          R eps2, R &sx, R &sy, R &sz, R &sp) {
+    sx = sy = sz = sp = R(0);
+#pragma unroll 4
+    for (int k = 0; k < m; k++) {
+        const V4 a = sa[k], b = sb[k], c = scc[k];
+        const R dx = p.x - a.x, dy = p.y - a.y, dz = p.z - a.z;
+        const R r2 = dx * dx + dy * dy + dz * dz + eps2;
+        const R rinv = rsq<R>(r2);
+        const R ri2 = rinv * rinv;
+        const R g3 = rinv * ri2, g5 = g3 * ri2, g7 = g5 * ri2;
+        const R qx = b.x * dx + c.x * dy + c.y * dz;
+        const R qy = c.x * dx + b.y * dy + c.z * dz;
+        const R qz = c.y * dx + c.z * dy + b.z * dz;
+        const R dqd = dx * qx + dy * qy + dz * qz;
+        const R tr = c.w;
+        const R s = -b.w * g3 + R(1.5) * tr * g5 - R(7.5) * dqd * g7;
+        const R t5 = R(3) * g5;
+        sx += s * dx + t5 * qx;
+        sy += s * dy + t5 * qy;
+        sz += s * dz + t5 * qz;
+        if (POT) sp -= b.w * rinv + R(0.5) * (R(3) * dqd * g5 - tr * g3);
+    }
+}
+// the same of m staged particles
+template <int LD, bool POT>
+__device__ __forceinline__ void part_sums(const float *f, int m, const float4 &p, float eps2,
+                                          float &sx_, float &sy_, float &sz_, float &sp_) {
+    const float2 px = f2(p.x), py = f2(p.y), pz = f2(p.z), e2 = f2(eps2), m1 = f2(-1.f);
+    float2 sx = f2(0.f), sy = f2(0.f), sz = f2(0.f), spp = f2(0.f);
+#pragma unroll 4
+    for (int k = 0; k < m; k += 2) {
+        const float2 dx = __ffma2_rn(ld2(f + k), m1, px);
+        const float2 dy = __ffma2_rn(ld2(f + LD + k), m1, py);
+        const float2 dz = __ffma2_rn(ld2(f + 2 * LD + k), m1, pz);
+        const float2 nm = ld2(f + 3 * LD + k);  // -m
+        float2 r2 = __ffma2_rn(dx, dx, e2);
+        r2 = __ffma2_rn(dy, dy, r2);
+        r2 = __ffma2_rn(dz, dz, r2);
+        const float2 rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+        const float2 nmr = __fmul2_rn(nm, rinv);
+        const float2 g = __fmul2_rn(nmr, __fmul2_rn(rinv, rinv));  // -m / r^3
+        sx = __ffma2_rn(g, dx, sx);
+        sy = __ffma2_rn(g, dy, sy);
+        sz = __ffma2_rn(g, dz, sz);
+        if (POT) spp = __fadd2_rn(spp, nmr);
+    }
+    sx_ = sx.x + sx.y;
+    sy_ = sy.x + sy.y;
+    sz_ = sz.x + sz.y;
+    sp_ = spp.x + spp.y;
+}
+template <bool POT, class R, class V4>
+__device__ __forceinline__ void part_sums(const V4 *sa, int m, const V4 &p, R eps2, R &sx, R &sy, R &sz,
+                                          R &sp) {
+    sx = sy = sz = sp = R(0);
+#pragma unroll 8
+    for (int k = 0; k < m; k++) {
+        const V4 a = sa[k];
+        const R dx = p.x - a.x, dy = p.y - a.y, dz = p.z - a.z;
+        const R r2 = dx * dx + dy * dy + dz * dz + eps2;
+        const R rinv = rsq<R>(r2);
+        const R gg = a.w * rinv * rinv * rinv;
+        sx -= gg * dx;
+        sy -= gg * dy;
+        sz -= gg * dz;
+        if (POT) sp -= a.w * rinv;
+    }
+}
+
+template <bool POT>
+__global__ void __launch_bounds__(WALK_WARPS * 32, POT ? 1 : 6)
     k_walk(const int *__restrict__ ngroup_p, const int *__restrict__ gstart, const int *__restrict__ gcount,
            const int *__restrict__ gcloud, const int *__restrict__ croot,
-           const typename R4<R>::T *__restrict__ pw, const typename R4<R>::T *__restrict__ wA,
-           const typename R4<R>::T *__restrict__ wB, const typename R4<R>::T *__restrict__ wC,
-           const int4 *__restrict__ wL, int leaf_size, R eps2, double G, int n,
+           const float4 *__restrict__ pw, const float4 *__restrict__ wA,
+           const float4 *__restrict__ wB, const float4 *__restrict__ wC,
+           const int4 *__restrict__ wL, int leaf_size, float eps2, double G, int n,
            double *__restrict__ agrav, double *__restrict__ pot, unsigned *work,
            unsigned long long *counters, long long *status, float theta_local, SgArgs sg) {
-    typedef typename R4<R>::T V4;
-    constexpr bool PACKED = std::is_same<R, float>::value;
-    typedef typename std::conditional<PACKED, WalkSmemF, WalkSmem<R>>::type SM;
-    __shared__ SM smem[WALK_WARPS];
+    __shared__ WalkSmemF smem[WALK_WARPS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    SM &S = smem[w];
+    WalkSmemF &S = smem[w];
     const unsigned lt = (1u << lane) - 1u;
     int maxsp = 0;
     const int ngroup = *ngroup_p;
@@ -281,43 +391,41 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, std::is_same<R, float>::value
         const int s0 = gstart[g], gc = gcount[g];
         const bool act = lane < gc;
         const int i = s0 + (act ? lane : 0);
-        const V4 pi = pw[i];
-        const R bx0 = wmin<R>(act ? pi.x : R(INFINITY)), by0 = wmin<R>(act ? pi.y : R(INFINITY)),
-                bz0 = wmin<R>(act ? pi.z : R(INFINITY));
-        const R bx1 = wmax<R>(act ? pi.x : R(-INFINITY)), by1 = wmax<R>(act ? pi.y : R(-INFINITY)),
-                bz1 = wmax<R>(act ? pi.z : R(-INFINITY));
+        const float4 pi = pw[i];
+        const float bx0 = wmin<float>(act ? pi.x : INFINITY), by0 = wmin<float>(act ? pi.y : INFINITY),
+                bz0 = wmin<float>(act ? pi.z : INFINITY);
+        const float bx1 = wmax<float>(act ? pi.x : -INFINITY), by1 = wmax<float>(act ? pi.y : -INFINITY),
+                bz1 = wmax<float>(act ? pi.z : -INFINITY);
         // each chunk's sum (at most 32 terms) joins a plain accumulator of
         // the walk's precision: in FP32 the compensated form measured 1.7 %
         // slower (the registers of its correction terms) for a change of
         // 1.3e-7 in the acceleration, against the opening angle's 1e-4
-        PlainSum<R> ax, ay, az, ph;
+        PlainSum<float> ax, ay, az, ph;
         int nC = 0, nP = 0, nF = 0;
         int sp = 1, nc = 0, np = 0, nr = 0, nfar = 0;
         bool overflow = false;
         // the super-group's node list replaces the root when it has one
         int rpos = 0, nrem = 0, sgi = -1;
         const int *rem = nullptr;
-        if constexpr (PACKED) {
-            if (sg.g_sg) {
-                const int s = sg.g_sg[g];
-                const int k = s < sg.cap ? sg.nrem[s] : -1;
-                if (k >= 0) {
-                    sgi = s;
-                    nrem = k;
-                    rem = sg.pool + (size_t)sg.start[s] * SG_POOL;
-                    sp = 0;
-                    // the super-group's expansion at its own centre, first
-                    const float *Ls = sg.L + (size_t)s * SG_LSTRIDE;
-                    float Lt[NLOC];
+        if (sg.g_sg) {
+            const int s = sg.g_sg[g];
+            const int k = s < sg.cap ? sg.nrem[s] : -1;
+            if (k >= 0) {
+                sgi = s;
+                nrem = k;
+                rem = sg.pool + (size_t)sg.start[s] * SG_POOL;
+                sp = 0;
+                // the super-group's expansion at its own centre, first
+                const float *Ls = sg.L + (size_t)s * SG_LSTRIDE;
+                float Lt[NLOC];
 #pragma unroll
-                    for (int q = 0; q < NLOC; q++) Lt[q] = Ls[q];
-                    float fax, fay, faz, fph;
-                    far_eval(Lt, pi.x - Ls[36], pi.y - Ls[37], pi.z - Ls[38], fax, fay, faz, fph);
-                    ax.add(fax);
-                    ay.add(fay);
-                    az.add(faz);
-                    if (POT) ph.add(fph);
-                }
+                for (int q = 0; q < NLOC; q++) Lt[q] = Ls[q];
+                float fax, fay, faz, fph;
+                far_eval(Lt, pi.x - Ls[36], pi.y - Ls[37], pi.z - Ls[38], fax, fay, faz, fph);
+                ax.add(fax);
+                ay.add(fay);
+                az.add(faz);
+                if (POT) ph.add(fph);
             }
         }
         if (lane == 0 && sgi < 0) S.stk[0] = croot[gcloud[g]];
@@ -325,123 +433,49 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, std::is_same<R, float>::value
         // com is at least R_g / theta_local from the group centre x0 (R_g the
         // group's radius about x0) enter a Taylor expansion at x0 once per
         // group instead of being evaluated for every particle
-        R fx0 = R(0), fy0 = R(0), fz0 = R(0), rfar2 = R(INFINITY);
-        if constexpr (PACKED) {
-            if (theta_local > 0.f) {
-                fx0 = 0.5f * (bx0 + bx1);
-                fy0 = 0.5f * (by0 + by1);
-                fz0 = 0.5f * (bz0 + bz1);
-                const float ux = pi.x - fx0, uy = pi.y - fy0, uz = pi.z - fz0;
-                const float rg2 = wmax<float>(act ? ux * ux + uy * uy + uz * uz : 0.f);
-                rfar2 = rg2 / (theta_local * theta_local);
+        float fx0 = 0.f, fy0 = 0.f, fz0 = 0.f, rfar2 = INFINITY;
+        if (theta_local > 0.f) {
+            fx0 = 0.5f * (bx0 + bx1);
+            fy0 = 0.5f * (by0 + by1);
+            fz0 = 0.5f * (bz0 + bz1);
+            const float ux = pi.x - fx0, uy = pi.y - fy0, uz = pi.z - fz0;
+            const float rg2 = wmax<float>(act ? ux * ux + uy * uy + uz * uz : 0.f);
+            rfar2 = rg2 / (theta_local * theta_local);
 #pragma unroll
-                for (int q = 0; q < NLOC; q++) S.red[q][lane] = 0.f;
-            }
+            for (int q = 0; q < NLOC; q++) S.red[q][lane] = 0.f;
         }
         __syncwarp();
 
         auto flush_cells = [&](int m) {
-          if constexpr (PACKED) {
-            // two cells per lane per instruction (f32x2); odd chunks are padded
-            // with a massless, moment-free entry that contributes zero
-            const int m2 = (m + 1) & ~1;
-            if (lane < m2) {
-                float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, c = a;
-                if (lane < m) {
-                    const int nd = S.clist[lane];
-                    a = wA[nd];
-                    b = wB[nd];
-                    c = wC[nd];
-                }
-                S.f[0][lane] = a.x; S.f[1][lane] = a.y; S.f[2][lane] = a.z; S.f[3][lane] = -b.w;
-                S.f[4][lane] = b.x; S.f[5][lane] = b.y; S.f[6][lane] = b.z;
-                S.f[7][lane] = c.x; S.f[8][lane] = c.y; S.f[9][lane] = c.z; S.f[10][lane] = c.w;
-            }
-            __syncwarp();
-            const float2 px = f2(pi.x), py = f2(pi.y), pz = f2(pi.z), e2 = f2(eps2);
-            const float2 m1 = f2(-1.f), c15 = f2(1.5f), cm75 = f2(-7.5f), c3 = f2(3.f);
-            float2 sx = f2(0.f), sy = f2(0.f), sz = f2(0.f), spp = f2(0.f);
-#pragma unroll 4
-            for (int k = 0; k < m2; k += 2) {
-                const float2 dx = __ffma2_rn(ld2(&S.f[0][k]), m1, px);
-                const float2 dy = __ffma2_rn(ld2(&S.f[1][k]), m1, py);
-                const float2 dz = __ffma2_rn(ld2(&S.f[2][k]), m1, pz);
-                float2 r2 = __ffma2_rn(dx, dx, e2);
-                r2 = __ffma2_rn(dy, dy, r2);
-                r2 = __ffma2_rn(dz, dz, r2);
-                const float2 rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                const float2 ri2 = __fmul2_rn(rinv, rinv);
-                const float2 g3 = __fmul2_rn(rinv, ri2), g5 = __fmul2_rn(g3, ri2),
-                             g7 = __fmul2_rn(g5, ri2);
-                const float2 qxx = ld2(&S.f[4][k]), qyy = ld2(&S.f[5][k]), qzz = ld2(&S.f[6][k]);
-                const float2 qxy = ld2(&S.f[7][k]), qxz = ld2(&S.f[8][k]), qyz = ld2(&S.f[9][k]);
-                const float2 qx = __ffma2_rn(qxx, dx, __ffma2_rn(qxy, dy, __fmul2_rn(qxz, dz)));
-                const float2 qy = __ffma2_rn(qxy, dx, __ffma2_rn(qyy, dy, __fmul2_rn(qyz, dz)));
-                const float2 qz = __ffma2_rn(qxz, dx, __ffma2_rn(qyz, dy, __fmul2_rn(qzz, dz)));
-                const float2 dqd = __ffma2_rn(dx, qx, __ffma2_rn(dy, qy, __fmul2_rn(dz, qz)));
-                const float2 tr = ld2(&S.f[10][k]), nm = ld2(&S.f[3][k]);
-                const float2 a7 = __fmul2_rn(dqd, g7), b5 = __fmul2_rn(tr, g5);
-                // s = -M g3 + 1.5 tr g5 - 7.5 dqd g7
-                const float2 sc = __ffma2_rn(b5, c15, __ffma2_rn(a7, cm75, __fmul2_rn(nm, g3)));
-                const float2 t5 = __fmul2_rn(g5, c3);
-                sx = __ffma2_rn(t5, qx, __ffma2_rn(sc, dx, sx));
-                sy = __ffma2_rn(t5, qy, __ffma2_rn(sc, dy, sy));
-                sz = __ffma2_rn(t5, qz, __ffma2_rn(sc, dz, sz));
-                if (POT) {
-                    // -(M rinv + 0.5 (3 dqd g5 - tr g3))
-                    const float2 hq = __ffma2_rn(__fmul2_rn(dqd, g5), f2(1.5f),
-                                                 __fmul2_rn(__fmul2_rn(tr, g3), f2(-0.5f)));
-                    spp = __ffma2_rn(nm, rinv, spp);
-                    spp = __ffma2_rn(hq, m1, spp);
-                }
-            }
-            ax.add(sx.x + sx.y); ay.add(sy.x + sy.y); az.add(sz.x + sz.y);
-            if (POT) ph.add(spp.x + spp.y);
-            nC += m;
-            __syncwarp();
-          } else {
-            if (lane < m) {
-                int nd = S.clist[lane];
-                S.sa[lane] = wA[nd];
-                S.sb[lane] = wB[nd];
-                S.sc[lane] = wC[nd];
-            }
-            __syncwarp();
-            R sx = 0, sy = 0, sz = 0, sp_ = 0;
-#pragma unroll 4
-            for (int k = 0; k < m; k++) {
-                const V4 a = S.sa[k], b = S.sb[k], c = S.sc[k];
-                const R dx = pi.x - a.x, dy = pi.y - a.y, dz = pi.z - a.z;
-                const R r2 = dx * dx + dy * dy + dz * dz + eps2;
-                const R rinv = rsq<R>(r2);
-                const R ri2 = rinv * rinv;
-                const R g3 = rinv * ri2, g5 = g3 * ri2, g7 = g5 * ri2;
-                const R qx = b.x * dx + c.x * dy + c.y * dz;
-                const R qy = c.x * dx + b.y * dy + c.z * dz;
-                const R qz = c.y * dx + c.z * dy + b.z * dz;
-                const R dqd = dx * qx + dy * qy + dz * qz;
-                const R tr = c.w;
-                const R s = -b.w * g3 + R(1.5) * tr * g5 - R(7.5) * dqd * g7;
-                const R t5 = R(3) * g5;
-                sx += s * dx + t5 * qx;
-                sy += s * dy + t5 * qy;
-                sz += s * dz + t5 * qz;
-                if (POT) sp_ -= b.w * rinv + R(0.5) * (R(3) * dqd * g5 - tr * g3);
-            }
-            ax.add(sx); ay.add(sy); az.add(sz);
-            if (POT) ph.add(sp_);
-            nC += m;
-            __syncwarp();
+          // two cells per lane per instruction (f32x2); odd chunks are padded
+          // with a massless, moment-free entry that contributes zero
+          const int m2 = (m + 1) & ~1;
+          if (lane < m2) {
+              float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, c = a;
+              if (lane < m) {
+                  const int nd = S.clist[lane];
+                  a = wA[nd];
+                  b = wB[nd];
+                  c = wC[nd];
+              }
+              S.f[0][lane] = a.x; S.f[1][lane] = a.y; S.f[2][lane] = a.z; S.f[3][lane] = -b.w;
+              S.f[4][lane] = b.x; S.f[5][lane] = b.y; S.f[6][lane] = b.z;
+              S.f[7][lane] = c.x; S.f[8][lane] = c.y; S.f[9][lane] = c.z; S.f[10][lane] = c.w;
           }
+          __syncwarp();
+          float sx, sy, sz, sp_;
+          cell_sums<32, POT>(&S.f[0][0], m2, pi, eps2, sx, sy, sz, sp_);
+          ax.add(sx); ay.add(sy); az.add(sz);
+          if (POT) ph.add(sp_);
+          nC += m;
+          __syncwarp();
         };
         // far cells: one per lane, added into the lane's own column of
         // partial coefficient sums (summed over the warp once per group)
         auto flush_far = [&](int m) {
-          if constexpr (PACKED) {
-            far_add<1>(S.red, lane, S.flist, m, fx0, fy0, fz0, eps2, wA, wB, wC);
-            nF += m;
-            __syncwarp();
-          }
+          far_add<1>(S.red, lane, S.flist, m, fx0, fy0, fz0, eps2, wA, wB, wC);
+          nF += m;
+          __syncwarp();
         };
         // slot of the particle at offset t of the pending stream: the last
         // range starting at or before t (nr <= NRANGE)
@@ -456,59 +490,19 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, std::is_same<R, float>::value
         };
         // the m pending particles from stream offset h
         auto flush_parts = [&](int m, int h) {
-          if constexpr (PACKED) {
-            const int m2 = (m + 1) & ~1;
-            if (lane < m2) {
-                float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (lane < m) a = pw[part_slot(h + lane)];
-                S.f[0][lane] = a.x; S.f[1][lane] = a.y; S.f[2][lane] = a.z; S.f[3][lane] = -a.w;
-            }
-            __syncwarp();
-            const float2 px = f2(pi.x), py = f2(pi.y), pz = f2(pi.z), e2 = f2(eps2);
-            const float2 m1 = f2(-1.f);
-            float2 sx = f2(0.f), sy = f2(0.f), sz = f2(0.f), spp = f2(0.f);
-#pragma unroll 4
-            for (int k = 0; k < m2; k += 2) {
-                const float2 dx = __ffma2_rn(ld2(&S.f[0][k]), m1, px);
-                const float2 dy = __ffma2_rn(ld2(&S.f[1][k]), m1, py);
-                const float2 dz = __ffma2_rn(ld2(&S.f[2][k]), m1, pz);
-                const float2 nm = ld2(&S.f[3][k]);  // -m
-                float2 r2 = __ffma2_rn(dx, dx, e2);
-                r2 = __ffma2_rn(dy, dy, r2);
-                r2 = __ffma2_rn(dz, dz, r2);
-                const float2 rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                const float2 nmr = __fmul2_rn(nm, rinv);
-                const float2 g = __fmul2_rn(nmr, __fmul2_rn(rinv, rinv));  // -m / r^3
-                sx = __ffma2_rn(g, dx, sx);
-                sy = __ffma2_rn(g, dy, sy);
-                sz = __ffma2_rn(g, dz, sz);
-                if (POT) spp = __fadd2_rn(spp, nmr);
-            }
-            ax.add(sx.x + sx.y); ay.add(sy.x + sy.y); az.add(sz.x + sz.y);
-            if (POT) ph.add(spp.x + spp.y);
-            nP += m;
-            __syncwarp();
-          } else {
-            if (lane < m) S.sa[lane] = pw[part_slot(h + lane)];
-            __syncwarp();
-            R sx = 0, sy = 0, sz = 0, sp_ = 0;
-#pragma unroll 8
-            for (int k = 0; k < m; k++) {
-                const V4 a = S.sa[k];
-                const R dx = pi.x - a.x, dy = pi.y - a.y, dz = pi.z - a.z;
-                const R r2 = dx * dx + dy * dy + dz * dz + eps2;
-                const R rinv = rsq<R>(r2);
-                const R gg = a.w * rinv * rinv * rinv;
-                sx -= gg * dx;
-                sy -= gg * dy;
-                sz -= gg * dz;
-                if (POT) sp_ -= a.w * rinv;
-            }
-            ax.add(sx); ay.add(sy); az.add(sz);
-            if (POT) ph.add(sp_);
-            nP += m;
-            __syncwarp();
+          const int m2 = (m + 1) & ~1;
+          if (lane < m2) {
+              float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (lane < m) a = pw[part_slot(h + lane)];
+              S.f[0][lane] = a.x; S.f[1][lane] = a.y; S.f[2][lane] = a.z; S.f[3][lane] = -a.w;
           }
+          __syncwarp();
+          float sx, sy, sz, sp_;
+          part_sums<32, POT>(&S.f[0][0], m2, pi, eps2, sx, sy, sz, sp_);
+          ax.add(sx); ay.add(sy); az.add(sz);
+          if (POT) ph.add(sp_);
+          nP += m;
+          __syncwarp();
         };
 
         while (sp > 0 || rpos < nrem || nc > 0 || np > 0) {
@@ -529,20 +523,18 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, std::is_same<R, float>::value
                 if (lane < take) {
                     nd = S.stk[sp + lane];
                     // the two 16-byte records a node visit needs, issued together
-                    const V4 a = wA[nd];
+                    const float4 a = wA[nd];
                     const int4 L = wL[nd];
                     f = L.x;
                     cn = L.y;
                     cl = L.z;
                     cr = L.w;
-                    const R d2 = box_d2(bx0, by0, bz0, bx1, by1, bz1, a.x, a.y, a.z);
+                    const float d2 = box_d2(bx0, by0, bz0, bx1, by1, bz1, a.x, a.y, a.z);
                     accept = d2 >= a.w && cn > 1;
                     open = !accept;
-                    if constexpr (PACKED) {
-                        if (accept && theta_local > 0.f) {
-                            const float dx = a.x - fx0, dy = a.y - fy0, dz = a.z - fz0;
-                            far = dx * dx + dy * dy + dz * dz >= rfar2;
-                        }
+                    if (accept && theta_local > 0.f) {
+                        const float dx = a.x - fx0, dy = a.y - fy0, dz = a.z - fz0;
+                        far = dx * dx + dy * dy + dz * dz >= rfar2;
                     }
                 }
                 __syncwarp();
@@ -553,19 +545,17 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, std::is_same<R, float>::value
                 const unsigned am = __ballot_sync(FULL, accept && !far);
                 if (accept && !far) S.clist[nc + __popc(am & lt)] = nd;
                 nc += __popc(am);
-                if constexpr (PACKED) {
-                    const unsigned fm = __ballot_sync(FULL, far);
-                    if (far) S.flist[nfar + __popc(fm & lt)] = nd;
-                    nfar += __popc(fm);
+                const unsigned fm = __ballot_sync(FULL, far);
+                if (far) S.flist[nfar + __popc(fm & lt)] = nd;
+                nfar += __popc(fm);
+                __syncwarp();
+                if (nfar >= 32) {
+                    flush_far(32);
+                    const int v = S.flist[32 + lane];
                     __syncwarp();
-                    if (nfar >= 32) {
-                        flush_far(32);
-                        const int v = S.flist[32 + lane];
-                        __syncwarp();
-                        if (lane + 32 < nfar) S.flist[lane] = v;
-                        nfar -= 32;
-                        __syncwarp();
-                    }
+                    if (lane + 32 < nfar) S.flist[lane] = v;
+                    nfar -= 32;
+                    __syncwarp();
                 }
                 // children of opened inner nodes
                 const unsigned im = __ballot_sync(FULL, inner);
@@ -651,28 +641,26 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, std::is_same<R, float>::value
                 if (nfar > 0) { flush_far(nfar); nfar = 0; }
             }
         }
-        if constexpr (PACKED) {
-            if (nF > 0) {
-                __syncwarp();
-                for (int q = lane; q < NLOC; q += 32) {  // Kahan sum of the 32 lane columns
-                    KSum<float> t;
-                    for (int k = 0; k < 32; k++) t.add(S.red[q][k]);
-                    S.ltot[q] = (float)t.value();
-                }
-                __syncwarp();
-                float Lt[NLOC];
-#pragma unroll
-                for (int q = 0; q < NLOC; q++) Lt[q] = S.ltot[q];
-                float fax, fay, faz, fph;
-                far_eval(Lt, pi.x - fx0, pi.y - fy0, pi.z - fz0, fax, fay, faz, fph);
-                ax.add(fax);
-                ay.add(fay);
-                az.add(faz);
-                if (POT) ph.add(fph);
+        if (nF > 0) {
+            __syncwarp();
+            for (int q = lane; q < NLOC; q += 32) {  // Kahan sum of the 32 lane columns
+                KSum<float> t;
+                for (int k = 0; k < 32; k++) t.add(S.red[q][k]);
+                S.ltot[q] = (float)t.value();
             }
+            __syncwarp();
+            float Lt[NLOC];
+#pragma unroll
+            for (int q = 0; q < NLOC; q++) Lt[q] = S.ltot[q];
+            float fax, fay, faz, fph;
+            far_eval(Lt, pi.x - fx0, pi.y - fy0, pi.z - fz0, fax, fay, faz, fph);
+            ax.add(fax);
+            ay.add(fay);
+            az.add(faz);
+            if (POT) ph.add(fph);
         }
         if (act) {
-            const double self = POT ? (double)(pi.w * rsq<R>(eps2)) : 0.0;
+            const double self = POT ? (double)(pi.w * rsq<float>(eps2)) : 0.0;
             agrav[i] = G * ax.value();
             agrav[(size_t)n + i] = G * ay.value();
             agrav[2 * (size_t)n + i] = G * az.value();
@@ -686,6 +674,392 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, std::is_same<R, float>::value
         }
     }
     if (lane == 0) atomicMax((unsigned long long *)&status[7], (unsigned long long)maxsp);
+}
+
+// The FP64 walk, and the FP32 walk of a small cloud: a block of BW warps per
+// group.  With a warp per group the walk of a cloud whose groups leave warps of
+// the chip idle lasts as long as its longest group, a chain of rounds (32 nodes each) and of
+// evaluations (32 staged entries each): 10k particles in FP64, 489 groups on
+// 148 SMs, 209 thousand cycles a group, 62 % of them evaluations.  Here a round
+// takes a node per thread, and the pending entries are evaluated 32 by each
+// warp, every warp for all of the group's particles; the warps' sums are
+// added at the end.  The group's box, its tests, and so its interactions are
+// those of k_walk.
+constexpr int BSTK = 1024;
+// (BW warps, BT threads per group)
+template <class R, int BW> struct BlockWalkSmem {
+    static constexpr int BT = 32 * BW;
+    static constexpr bool PACKED = std::is_same<R, float>::value;
+    typedef typename R4<R>::T V4;
+    int stk[BSTK];
+    int clist[2 * BT], flist[2 * BT];
+    int rf[2 * BT], rs[2 * BT];  // pending ranges, as in WalkSmemF (at most BT - 1 carried + BT)
+    int cnt[BW][5];              // a round's near, far, opened, buckets, their particles, per warp
+    int next;
+    // staging of each warp's 32 entries
+    __align__(16) float f[PACKED ? BW : 1][11][32];
+    V4 sa[PACKED ? 1 : BW][32], sb[PACKED ? 1 : BW][32], sc[PACKED ? 1 : BW][32];
+    float red[PACKED ? BW : 1][NLOC][32];
+    float lt[PACKED ? BW : 1][NLOC];
+    R sum[BW][4][32];
+};
+
+template <class R, bool POT, int BW>
+__global__ void __launch_bounds__(32 * BW)
+    k_walk_block(const int *__restrict__ ngroup_p, const int *__restrict__ gstart,
+                 const int *__restrict__ gcount, const int *__restrict__ gcloud,
+                 const int *__restrict__ croot, const typename R4<R>::T *__restrict__ pw,
+                 const typename R4<R>::T *__restrict__ wA, const typename R4<R>::T *__restrict__ wB,
+                 const typename R4<R>::T *__restrict__ wC, const int4 *__restrict__ wL, int leaf_size,
+                 R eps2, double G, int n, double *__restrict__ agrav, double *__restrict__ pot,
+                 unsigned *work, unsigned long long *counters, long long *status, float theta_local,
+                 SgArgs sg) {
+    typedef typename R4<R>::T V4;
+    constexpr bool PACKED = std::is_same<R, float>::value;
+    constexpr int BT = 32 * BW;
+    __shared__ BlockWalkSmem<R, BW> S;
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const int ngroup = *ngroup_p;
+    int maxsp = 0;
+    for (int g = blockIdx.x;; g += gridDim.x) {
+        if (work) {
+            __syncthreads();  // S.next has been read
+            if (t == 0) S.next = (int)atomicAdd(work, 1u);
+            __syncthreads();
+            g = S.next;
+        }
+        if (g >= ngroup) break;
+        const int s0 = gstart[g], gc = gcount[g];
+        const bool act = lane < gc;
+        const int i = s0 + (act ? lane : 0);
+        const V4 pi = pw[i];
+        const R bx0 = wmin<R>(act ? pi.x : R(INFINITY)), by0 = wmin<R>(act ? pi.y : R(INFINITY)),
+                bz0 = wmin<R>(act ? pi.z : R(INFINITY));
+        const R bx1 = wmax<R>(act ? pi.x : R(-INFINITY)), by1 = wmax<R>(act ? pi.y : R(-INFINITY)),
+                bz1 = wmax<R>(act ? pi.z : R(-INFINITY));
+        PlainSum<R> ax, ay, az, ph;
+        int nC = 0, nP = 0, nF = 0;
+        int sp = 1, nc = 0, np = 0, nr = 0, nfar = 0;
+        bool overflow = false;
+        int rpos = 0, nrem = 0, sgi = -1;
+        const int *rem = nullptr;
+        if constexpr (PACKED) {
+            if (sg.g_sg) {
+                const int x = sg.g_sg[g];
+                const int k = x < sg.cap ? sg.nrem[x] : -1;
+                if (k >= 0) {
+                    sgi = x;
+                    nrem = k;
+                    rem = sg.pool + (size_t)sg.start[x] * SG_POOL;
+                    sp = 0;
+                    if (w == 0) {
+                        // the super-group's expansion at its own centre
+                        const float *Ls = sg.L + (size_t)x * SG_LSTRIDE;
+                        float Lt[NLOC];
+#pragma unroll
+                        for (int q = 0; q < NLOC; q++) Lt[q] = Ls[q];
+                        float fax, fay, faz, fph;
+                        far_eval(Lt, pi.x - Ls[36], pi.y - Ls[37], pi.z - Ls[38], fax, fay, faz, fph);
+                        ax.add(fax);
+                        ay.add(fay);
+                        az.add(faz);
+                        if (POT) ph.add(fph);
+                    }
+                }
+            }
+        }
+        if (t == 0 && sgi < 0) S.stk[0] = croot[gcloud[g]];
+        R fx0 = R(0), fy0 = R(0), fz0 = R(0), rfar2 = R(INFINITY);
+        if constexpr (PACKED) {
+            if (theta_local > 0.f) {
+                fx0 = 0.5f * (bx0 + bx1);
+                fy0 = 0.5f * (by0 + by1);
+                fz0 = 0.5f * (bz0 + bz1);
+                const float ux = pi.x - fx0, uy = pi.y - fy0, uz = pi.z - fz0;
+                const float rg2 = wmax<float>(act ? ux * ux + uy * uy + uz * uz : 0.f);
+                rfar2 = rg2 / (theta_local * theta_local);
+#pragma unroll
+                for (int q = 0; q < NLOC; q++) S.red[w][q][lane] = 0.f;
+            }
+        }
+        __syncthreads();
+
+        // this warp's share of m <= BT entries: mw of them from w q on, q even
+        auto share = [&](int m, int &from, int &mw) {
+            const int q = (((m + BW - 1) / BW) + 1) & ~1;
+            from = w * q;
+            mw = max(0, min(q, m - from));
+        };
+        auto flush_cells = [&](int m) {
+            int from, mw;
+            share(m, from, mw);
+            R sx, sy, sz, sp_;
+            if constexpr (PACKED) {
+                const int m2 = (mw + 1) & ~1;
+                if (lane < m2) {
+                    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, c = a;
+                    if (lane < mw) {
+                        const int nd = S.clist[from + lane];
+                        a = wA[nd];
+                        b = wB[nd];
+                        c = wC[nd];
+                    }
+                    float(*f)[32] = S.f[w];
+                    f[0][lane] = a.x; f[1][lane] = a.y; f[2][lane] = a.z; f[3][lane] = -b.w;
+                    f[4][lane] = b.x; f[5][lane] = b.y; f[6][lane] = b.z;
+                    f[7][lane] = c.x; f[8][lane] = c.y; f[9][lane] = c.z; f[10][lane] = c.w;
+                }
+                __syncwarp();
+                cell_sums<32, POT>(&S.f[w][0][0], m2, pi, eps2, sx, sy, sz, sp_);
+            } else {
+                if (lane < mw) {
+                    const int nd = S.clist[from + lane];
+                    S.sa[w][lane] = wA[nd];
+                    S.sb[w][lane] = wB[nd];
+                    S.sc[w][lane] = wC[nd];
+                }
+                __syncwarp();
+                cell_sums<POT, R>(S.sa[w], S.sb[w], S.sc[w], mw, pi, eps2, sx, sy, sz, sp_);
+            }
+            ax.add(sx); ay.add(sy); az.add(sz);
+            if (POT) ph.add(sp_);
+            nC += m;
+            __syncwarp();
+        };
+        auto flush_far = [&](int m) {
+            if constexpr (PACKED) {
+                int from, mw;
+                share(m, from, mw);
+                far_add<1>(S.red[w], lane, S.flist + from, mw, fx0, fy0, fz0, eps2, wA, wB, wC);
+                nF += m;
+            }
+        };
+        auto part_slot = [&](int o) {
+            int r = 0;
+#pragma unroll
+            for (int step = BT; step; step >>= 1) {
+                const int c = r + step;
+                if (c < nr && S.rs[c] <= o) r = c;
+            }
+            return S.rf[r] + (o - S.rs[r]);
+        };
+        auto flush_parts = [&](int m, int h) {
+            int from, mw;
+            share(m, from, mw);
+            R sx, sy, sz, sp_;
+            if constexpr (PACKED) {
+                const int m2 = (mw + 1) & ~1;
+                if (lane < m2) {
+                    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (lane < mw) a = pw[part_slot(h + from + lane)];
+                    float(*f)[32] = S.f[w];
+                    f[0][lane] = a.x; f[1][lane] = a.y; f[2][lane] = a.z; f[3][lane] = -a.w;
+                }
+                __syncwarp();
+                part_sums<32, POT>(&S.f[w][0][0], m2, pi, eps2, sx, sy, sz, sp_);
+            } else {
+                if (lane < mw) S.sa[w][lane] = pw[part_slot(h + from + lane)];
+                __syncwarp();
+                part_sums<POT, R>(S.sa[w], mw, pi, eps2, sx, sy, sz, sp_);
+            }
+            ax.add(sx); ay.add(sy); az.add(sz);
+            if (POT) ph.add(sp_);
+            nP += m;
+            __syncwarp();
+        };
+        // drop the first BT entries of a list of m (every thread calls)
+        auto shift = [&](int *list, int &m) {
+            const int v = list[BT + t];
+            __syncthreads();
+            if (BT + t < m) list[t] = v;
+            m -= BT;
+            __syncthreads();
+        };
+
+        while (sp > 0 || rpos < nrem) {
+            if (sp == 0) {
+                // next nodes of the super-group's list
+                const int take = min(nrem - rpos, BT);
+                if (t < take) S.stk[t] = rem[rpos + t];
+                rpos += take;
+                sp = take;
+                __syncthreads();
+            }
+            const int take = min(sp, BT);
+            sp -= take;
+            int nd = 0, f = 0, cn = 0, cl = 0, cr = 0;
+            bool accept = false, open = false, far = false;
+            if (t < take) {
+                nd = S.stk[sp + t];
+                const V4 a = wA[nd];
+                const int4 L = wL[nd];
+                f = L.x;
+                cn = L.y;
+                cl = L.z;
+                cr = L.w;
+                const R d2 = box_d2(bx0, by0, bz0, bx1, by1, bz1, a.x, a.y, a.z);
+                accept = d2 >= a.w && cn > 1;
+                open = !accept;
+                if constexpr (PACKED) {
+                    if (accept && theta_local > 0.f) {
+                        const float dx = a.x - fx0, dy = a.y - fy0, dz = a.z - fz0;
+                        far = dx * dx + dy * dy + dz * dz >= rfar2;
+                    }
+                }
+            }
+            const bool bucket = open && cn <= leaf_size, inner = open && cn > leaf_size;
+            const bool near = accept && !far;
+            const unsigned am = __ballot_sync(FULL, near), fm = __ballot_sync(FULL, far),
+                           im = __ballot_sync(FULL, inner), bm = __ballot_sync(FULL, bucket);
+            int incl = bucket ? cn : 0;
+            if (bm) {
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int x = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= o) incl += x;
+                }
+            }
+            if (lane == 31) {
+                S.cnt[w][0] = __popc(am);
+                S.cnt[w][1] = __popc(fm);
+                S.cnt[w][2] = __popc(im);
+                S.cnt[w][3] = __popc(bm);
+                S.cnt[w][4] = incl;
+            }
+            __syncthreads();  // the counts; and the stack has been read
+            int off[5] = {0, 0, 0, 0, 0}, tot[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+            for (int x = 0; x < BW; x++)
+#pragma unroll
+                for (int q = 0; q < 5; q++) {
+                    const int c = S.cnt[x][q];
+                    if (x < w) off[q] += c;
+                    tot[q] += c;
+                }
+            if (near) S.clist[nc + off[0] + __popc(am & lt)] = nd;
+            if (far) S.flist[nfar + off[1] + __popc(fm & lt)] = nd;
+            if (sp + 2 * tot[2] <= BSTK) {
+                if (inner) {
+                    const int pos = sp + 2 * (off[2] + __popc(im & lt));
+                    S.stk[pos] = cr;
+                    S.stk[pos + 1] = cl;
+                }
+                sp += 2 * tot[2];
+                maxsp = max(maxsp, sp);
+            } else {
+                overflow = true;
+            }
+            if (bucket) {
+                const int r = nr + off[3] + __popc(bm & lt);
+                S.rf[r] = f;
+                S.rs[r] = np + off[4] + incl - cn;
+            }
+            nc += tot[0];
+            nfar += tot[1];
+            nr += tot[3];
+            np += tot[4];
+            __syncthreads();
+            if (nc >= BT) {
+                flush_cells(BT);
+                shift(S.clist, nc);
+            }
+            if (nfar >= BT) {
+                flush_far(BT);
+                shift(S.flist, nfar);
+            }
+            if (np >= BT) {
+                int h = 0;
+                do {
+                    flush_parts(BT, h);
+                    h += BT;
+                } while (np - h >= BT);
+                np -= h;
+                // keep the ranges from the one holding offset h on, their
+                // offsets taken from h (< BT of them: each keeps at least one
+                // of the < BT pending particles)
+                int r0 = nr;
+                if (np > 0) {
+                    r0 = 0;
+#pragma unroll
+                    for (int step = BT; step; step >>= 1) {
+                        const int c = r0 + step;
+                        if (c < nr && S.rs[c] <= h) r0 = c;
+                    }
+                }
+                const int keep = nr - r0;
+                int vf = 0, vs = 0;
+                if (t < keep) {
+                    vf = S.rf[r0 + t];
+                    vs = S.rs[r0 + t] - h;
+                }
+                __syncthreads();
+                if (t < keep) {
+                    S.rf[t] = vf;
+                    S.rs[t] = vs;
+                }
+                nr = keep;
+                __syncthreads();
+            }
+        }
+        if (nc > 0) flush_cells(nc);
+        if (np > 0) flush_parts(np, 0);
+        if (nfar > 0) flush_far(nfar);
+        // the warps' sums
+        S.sum[w][0][lane] = ax.s;
+        S.sum[w][1][lane] = ay.s;
+        S.sum[w][2][lane] = az.s;
+        if (POT) S.sum[w][3][lane] = ph.s;
+        if constexpr (PACKED) {
+            if (nF > 0) {
+                __syncwarp();
+                for (int q = lane; q < NLOC; q += 32) {  // Kahan sum of the 32 lane columns
+                    KSum<float> x;
+                    for (int k = 0; k < 32; k++) x.add(S.red[w][q][k]);
+                    S.lt[w][q] = (float)x.value();
+                }
+            }
+        }
+        __syncthreads();
+        if (w == 0) {
+            R v[4];
+#pragma unroll
+            for (int d = 0; d < (POT ? 4 : 3); d++) {
+                v[d] = S.sum[0][d][lane];
+                for (int x = 1; x < BW; x++) v[d] += S.sum[x][d][lane];
+            }
+            if constexpr (PACKED) {
+                if (nF > 0) {
+                    float Lt[NLOC];
+#pragma unroll
+                    for (int q = 0; q < NLOC; q++) {
+                        Lt[q] = S.lt[0][q];
+                        for (int x = 1; x < BW; x++) Lt[q] += S.lt[x][q];
+                    }
+                    float fax, fay, faz, fph;
+                    far_eval(Lt, pi.x - fx0, pi.y - fy0, pi.z - fz0, fax, fay, faz, fph);
+                    v[0] += fax;
+                    v[1] += fay;
+                    v[2] += faz;
+                    if (POT) v[3] += fph;
+                }
+            }
+            if (act) {
+                agrav[i] = G * (double)v[0];
+                agrav[(size_t)n + i] = G * (double)v[1];
+                agrav[2 * (size_t)n + i] = G * (double)v[2];
+                if (POT) pot[i] = G * ((double)v[3] + (double)(pi.w * rsq<R>(eps2)));
+            }
+        }
+        if (t == 0) {
+            atomicAdd(&counters[0], (unsigned long long)nC * gc);
+            atomicAdd(&counters[1], (unsigned long long)nP * gc);
+            atomicAdd(&counters[2], (unsigned long long)nF);
+            if (overflow) status_add(status, SPH_S_STACK_OVERFLOW, 1);
+        }
+        if (!work) __syncthreads();  // before the next group's lists
+    }
+    if (t == 0) atomicMax((unsigned long long *)&status[7], (unsigned long long)maxsp);
 }
 
 // Super-group pre-walk of the FP32 walk with group expansions: one warp per
@@ -989,6 +1363,23 @@ __global__ void __cluster_dims__(DS_CLUSTER, 1, 1) __launch_bounds__(DS_WARPS * 
     cluster.sync();  // the others' sums stay until they are read
 }
 
+// Warps per group of the walk (k_walk_block; 1: k_walk).  us of one walk of an
+// Evrard sphere with 1 / 2 / 4 warps:
+//   FP64, theta 0.5:  10k 188 / 113 / 89;  45k 353 / 292 / 267;  100k 661 / 601 /
+//     593;  131k 843 / 763 / 775;  500k 3229 / 3123 / 3315
+//   FP32 with expansions (theta 0.35):  10k 144 / 83 / 59;  45k 240 / 192 / 179;
+//     65k 254 / 229 / 233;  100k 347 / 330 / 351;  131k 386 / 393 / 426
+//   FP32 without (theta 0.5):  10k 98 / 59 / 47;  45k 200 / 145 / 143;  100k 320 /
+//     290 / 311;  200k 593 / 573 / 643;  300k 853 / 872 / 979
+// The lines are in particles per SM.  (The super-group pre-walk in the same
+// form gained nothing: 131k 55 / 62 / 53 us.)
+int walk_warps(const sph_ctx *ctx) {
+    const long long n = ctx->n, sm = ctx->num_sms;
+    if (ctx->cfg.precision == SPH_PREC_FP64) return n <= 750 * sm ? 4 : 2;
+    const int two = ctx->cfg.theta_local > 0.0 ? 740 : 1700;
+    return n <= 340 * sm ? 4 : n <= two * sm ? 2 : 1;
+}
+
 template <class R, bool POT>
 int run_walk(sph_ctx *ctx, cudaStream_t s) {
     // groups hold 1..32 particles (about 20 on average); size the grid for
@@ -1023,12 +1414,21 @@ int run_walk(sph_ctx *ctx, cudaStream_t s) {
             sg.cap = ctx->sg_cap;
         }
     }
+    // (the FP64 walk takes blocks at every size)
+    const int warps = walk_warps(ctx);
+    auto kern = warps == 4 ? k_walk_block<R, POT, 4> : k_walk_block<R, POT, 2>;
+    if constexpr (std::is_same<R, float>::value)
+        if (warps == 1) kern = k_walk<POT>;
+    const int block = 32 * (warps > 1 ? warps : WALK_WARPS);
+    if (warps > 1) {
+        grid0 = max(1, div_up(ctx->n, 16) + ctx->ncloud);
+        if (ctx->cfg.walk_blocks > 0) grid0 = min(grid0, ctx->num_sms * ctx->cfg.walk_blocks);
+    }
     int grid;
     unsigned *wq;
-    rc = queue_launch(ctx, s, WQ_WALK, (const void *)k_walk<R, POT>, WALK_WARPS * 32, grid0, &grid,
-                      &wq);
+    rc = queue_launch(ctx, s, WQ_WALK, (const void *)kern, block, grid0, &grid, &wq);
     if (rc) return rc;
-    k_walk<R, POT><<<grid, WALK_WARPS * 32, 0, s>>>(
+    kern<<<grid, block, 0, s>>>(
         ctx->d_ngroup, ctx->gstart, ctx->gcount, ctx->groot_g, ctx->croot,
         (const typename R4<R>::T *)ctx->pw, (const typename R4<R>::T *)ctx->wA,
         (const typename R4<R>::T *)ctx->wB, (const typename R4<R>::T *)ctx->wC, ctx->wL,
