@@ -457,7 +457,7 @@ int sph_ctx_create(const sph_config *cfg, sph_ctx **out) {
     DAF(ctx->hsr, N); DAF(ctx->dmv, N); DAF(ctx->gdm, N);
     DAF(ctx->dmv_max, C + 1);
     ctx->rows_ok = (int *)(ctx->dmv_max + C);
-    DAF(ctx->kept_cnt, 3);
+    DAF(ctx->kept_cnt, 5);
     DAF(ctx->dt, C); DAF(ctx->dt_next, C); DAF(ctx->dt_bits, C); DAF(ctx->dtmax_bits, C);
     DAF(ctx->dt_part, N); DAF(ctx->dhdt, N); DAF(ctx->dbin, N);
     DAF(ctx->status, SPH_NSTATUS);
@@ -485,7 +485,7 @@ int sph_ctx_create(const sph_config *cfg, sph_ctx **out) {
         cudaMemsetAsync(ctx->corg, 0, 3 * C * sizeof(double), ctx->stream) ||
         cudaMemsetAsync(ctx->dmv_max, 0, (C + 1) * sizeof(unsigned long long), ctx->stream) ||
         cudaMemsetAsync(ctx->dmv, 0, N * sizeof(double), ctx->stream) ||
-        cudaMemsetAsync(ctx->kept_cnt, 0, 3 * sizeof(int), ctx->stream))
+        cudaMemsetAsync(ctx->kept_cnt, 0, 5 * sizeof(int), ctx->stream))
         return fail(SPH_ERR_CUDA);
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return fail(SPH_ERR_CUDA);
 #undef DAF

@@ -32,9 +32,12 @@
 namespace {
 
 constexpr int SEARCH_WARPS = 4;
-// particles per SM up to which a cloud's searches take 8, 4 or 2 lanes per
-// particle (search_split; the measurements behind the lines stand there)
-constexpr int SPLIT8_PER_SM = 68, SPLIT4_PER_SM = 140, SPLIT2_PER_SM = 300;
+// particles per SM up to which a cloud's searches take 32, 8, 4 or 2 lanes per
+// particle (search_split; the measurements behind the lines stand there), and
+// the longest searches, in chunks per particle per SM, past which the next h
+// iteration leaves 8 lanes for 32 or 32 for 8 (k_kept_shift)
+constexpr int SPLIT32_PER_SM = 34, SPLIT8_PER_SM = 68, SPLIT4_PER_SM = 140, SPLIT2_PER_SM = 300;
+constexpr double LONG8 = 1.6, LONG32 = 0.45;
 constexpr int SSTK = 512;
 constexpr unsigned FULL = 0xffffffffu;
 // pending bucket particles: ranges of consecutive slots, range r starting at
@@ -121,6 +124,7 @@ __device__ __forceinline__ double wmax(double v) {
 
 struct SearchArgs {
     const int *gstart, *gcount, *gcloud, *croot;
+    const int *cloud;  // per particle
     double4 *p0;
     // node boxes in FP32 rounded outward: (min rounded down, h_max rounded
     // up), (max rounded up, 0)
@@ -155,7 +159,8 @@ struct SearchArgs {
 template <int MODE, class R = double, int SPLIT = 1>
 __device__ __forceinline__ int group_search(SearchSmem &S, const SearchArgs &A, int root, bool act,
                                             int i, const double4 &pi, double ri,
-                                            HSums<R> *hs = nullptr) {
+                                            HSums<R> *hs = nullptr, int *chunks = nullptr) {
+    static_assert(MODE != 0 || SPLIT == 1, "split searches leave the sums to the rows");
     typedef typename R4<R>::T V4;
     const int lane = threadIdx.x & 31;
     constexpr int SW = 32 / SPLIT;  // staged candidates per lane of a chunk
@@ -223,6 +228,7 @@ __device__ __forceinline__ int group_search(SearchSmem &S, const SearchArgs &A, 
     };
     // the m pending candidates from stream offset h
     auto process = [&](int m, int h) {
+        if (chunks) ++*chunks;
         if (lane < m) {
             const int j = part_slot(h + lane);
             S.flat[lane] = j;
@@ -268,7 +274,20 @@ __device__ __forceinline__ int group_search(SearchSmem &S, const SearchArgs &A, 
                 acc = __funnelshift_l(__float_as_uint(d.x), acc, 1);
                 acc = __funnelshift_l(__float_as_uint(d.y), acc, 1);
             };
-            if ((reinterpret_cast<uintptr_t>(S.fx) & 15u) == 0) {
+            if (SW < 4) {
+                // a candidate or two per lane
+#pragma unroll
+                for (int k = k0; k < k0 + SW; k++) {
+                    const float dx = pfx.x - S.fx[k], dy = pfy.x - S.fy[k], dz = pfz.x - S.fz[k];
+                    float nlim = nri2f.x;
+                    if (MODE == 1) {
+                        const float sh = hif.x + S.fh[k];
+                        nlim = sh * sh * nwiden.x;
+                    }
+                    const float d = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, nlim)));
+                    acc = __funnelshift_l(__float_as_uint(d), acc, 1);
+                }
+            } else if ((reinterpret_cast<uintptr_t>(S.fx) & 15u) == 0) {
                 // four candidates per 128-bit shared load
 #pragma unroll 2
                 for (int k = SPLIT > 1 ? k0 : 0; k < (SPLIT > 1 ? k0 + SW : m4); k += 4) {
@@ -327,44 +346,13 @@ __device__ __forceinline__ int group_search(SearchSmem &S, const SearchArgs &A, 
             }
             int pos = count + incl - c;
             count += __shfl_sync(FULL, incl, SPLIT - 1, SPLIT);
-            // four hits per trip: independent chains of dependent arithmetic
-            while (ok) {
-                int k[4];
-                R wt[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const bool any = ok != 0;
-                    k[q] = any ? k0 + __ffs(ok) - 1 : k[0];
-                    ok &= ok - 1;
-                    wt[q] = R(0);
-                    if (any) {
-                        if (MODE == 1) {
-                            if (pos < K) A.rows[(size_t)i * K + pos] = S.flat[k[q]];
-                            hnb = fmax(hnb, S.stage[k[q]].w);
-                        } else {
-                            if (pos < K) A.cidx[cbase + pos] = S.flat[k[q]];
-                            if (MODE == 0) wt[q] = FAST ? (R)S.fh[k[q]] : (R)S.smass[k[q]];
-                        }
-                        pos++;
-                    }
-                }
-                if (MODE == 0) {
-                    R w[4], dw[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        R r;
-                        if (FAST) {
-                            const float ax = pfx.x - S.fx[k[q]], ay = pfy.x - S.fy[k[q]],
-                                        az = pfz.x - S.fz[k[q]];
-                            const float r2 = fmaf(az, az, fmaf(ay, ay, ax * ax));
-                            r = r2 * rsqrtf(r2 + 1e-30f);
-                        } else {
-                            r = pair_r<R>(pi, S.stage[k[q]]);
-                        }
-                        hs->terms(r, w[q], dw[q]);
-                    }
-                    cs += (wt[0] * w[0] + wt[1] * w[1]) + (wt[2] * w[2] + wt[3] * w[3]);
-                    cd += (wt[0] * dw[0] + wt[1] * dw[1]) + (wt[2] * dw[2] + wt[3] * dw[3]);
+            for (; ok; ok &= ok - 1, pos++) {
+                const int k = k0 + __ffs(ok) - 1;
+                if (MODE == 1) {
+                    if (pos < K) A.rows[(size_t)i * K + pos] = S.flat[k];
+                    hnb = fmax(hnb, S.stage[k].w);
+                } else if (pos < K) {
+                    A.cidx[cbase + pos] = S.flat[k];
                 }
             }
         } else if (FAST) {
@@ -426,7 +414,7 @@ __device__ __forceinline__ int group_search(SearchSmem &S, const SearchArgs &A, 
                 }
             }
         }
-        if (FAST || (MODE == 0 && SPLIT > 1)) {
+        if (FAST) {
             hs->S.add(cs);
             hs->D.add(cd);
         }
@@ -589,25 +577,18 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32)
 }
 
 // exact lists for the listed particles (A.mlist, *A.mcount entries; nothing
-// when *A.only_all, which k_lists covers): one warp per particle, its own box
-// (the search of one lane), the cloud root of the group holding it
+// when *A.only_all, which k_lists covers): one warp per particle, its own box, a
+// staged candidate per lane (one lane for all of them: 10k 27 us, 1M 50; here 18 and 35)
 __global__ void __launch_bounds__(SEARCH_WARPS * 32)
-    k_lists_list(const int *__restrict__ ngroup_p, SearchArgs A) {
+    k_lists_list(SearchArgs A) {
     __shared__ SearchSmem smem[SEARCH_WARPS];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5;
     if (*A.only_all) return;
-    const int m = *A.mcount, ngroup = *ngroup_p;
+    const int m = *A.mcount;
     for (int e = blockIdx.x * SEARCH_WARPS + w; e < m; e += gridDim.x * SEARCH_WARPS) {
         const int i = A.mlist[e];
-        // the group holding i: the last one starting at or before it
-        int lo = 0, hi = ngroup - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (A.gstart[mid] <= i) lo = mid;
-            else hi = mid - 1;
-        }
         const double4 pi = A.p0[i];
-        group_search<1>(smem[w], A, A.croot[A.gcloud[lo]], lane == 0, i, pi, pi.w);
+        group_search<1, double, 32>(smem[w], A, A.croot[A.cloud[i]], true, i, pi, pi.w);
     }
 }
 
@@ -727,11 +708,25 @@ struct ReuseArgs {
                                 // (INT_MAX after a full search), [2] this one attempts
 };
 
-// the kept-row counts moved on by one h iteration (one thread)
-__global__ void k_kept_shift(int *kept) {
+// the kept-row counts moved on by one h iteration, and the choice of its units
+// (one thread).  With 8 lanes per particle a unit is four particles; where the
+// cloud has grown a dense core, the units of its rim meet hundreds of chunks of
+// the core's particles (10k Evrard particles: 29 at the start, 44 after 60
+// steps, 250 after 120) and the launch lasts as long as they do.  A unit of one
+// particle meets a sixth of them (12, 27 and 38) but the cloud's walks are
+// repeated four times.  The four h iterations of a call, us, 8 / 32 lanes:
+//   10k FP64  460 / 685 at the start, 699 / 817 after 60 steps, 1552 / 1006 after 120
+//   7k FP64   311 / 472, 539 / 651, 1620 / 927;  5k FP64  283 / 337, 639 / 508, 1056 / 555
+// so the last iteration's longest search decides, 8 lanes up to LONG8 chunks per
+// particle of an SM's share, and back below LONG32 of them.  (The same by a
+// second launch for the particles left after the first round: 10k 1422 after 150
+// steps, against 1936 without and 1092 with 32 lanes.)
+__global__ void k_kept_shift(int *kept, int long8, int long32) {
     kept[1] = kept[2] ? kept[0] : INT_MAX;
     kept[0] = 0;
     kept[2] = 0;
+    kept[4] = kept[3] > (kept[4] ? long32 : long8);
+    kept[3] = 0;
 }
 
 __global__ void k_h_init(int n, const double *__restrict__ h, const double *__restrict__ hnb,
@@ -848,6 +843,7 @@ struct NewtonArgs {
     const float *gdm;   // per particle: its group's largest dmv, rounded up
     int *kept;       // count of the particles that kept their row (null: not counted)
     int *retry;
+    int *longest;  // the most chunks a unit has gone through; [1]: a unit is one particle
     double n_ngb, tol, grow, regrow;
     int max_iter, rounds;
 };
@@ -920,7 +916,7 @@ __device__ __forceinline__ void eval_rows(const SearchArgs &A, const NewtonArgs 
     const unsigned m = __ballot_sync(FULL, want && (lane & (SPLIT - 1)) == 0);
     if (!m) return;
     constexpr int U = SPLIT > 1 ? 4 : 2;
-    if (__popc(m) <= 4) row_sums<R, 16, U>(A, B, m, i, h, c, Ss, Ds);
+    if (SPLIT >= 8 || __popc(m) <= 4) row_sums<R, 16, U>(A, B, m, i, h, c, Ss, Ds);
     else row_sums<R, 4, U>(A, B, m, i, h, c, Ss, Ds);
     if (SPLIT > 1) {
         Ss = __shfl_sync(FULL, Ss, lane & ~(SPLIT - 1));
@@ -1057,11 +1053,10 @@ __device__ __forceinline__ bool newton_rows(const SearchArgs &A, const NewtonArg
 // measured faster than 95; a split cloud fills fewer blocks and takes the
 // registers for the unrolled chains instead.
 template <class R, int SPLIT>
-__global__ void __launch_bounds__(SEARCH_WARPS * 32, SPLIT > 1 ? 4 : 8)
-    k_cand_newton(const int *__restrict__ ngroup_p, SearchArgs A, NewtonArgs B, unsigned *queue) {
-    __shared__ SearchSmem smem[SEARCH_WARPS];
+__device__ __forceinline__ void newton_units(SearchSmem &smem, int ngroup, const SearchArgs &A,
+                                             const NewtonArgs &B, unsigned *queue) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nunit = *ngroup_p * SPLIT;
+    const int nunit = ngroup * SPLIT;
     const bool own = (lane & (SPLIT - 1)) == 0;
     for (int item = q_first(queue, blockIdx.x * SEARCH_WARPS + w); item < nunit;
          item = q_next(queue, item, gridDim.x * SEARCH_WARPS)) {
@@ -1090,7 +1085,7 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, SPLIT > 1 ? 4 : 8)
                         fgy1 = __double2float_ru(wmax(l3 ? pi.y : -INFINITY)),
                         fgz1 = __double2float_ru(wmax(l3 ? pi.z : -INFINITY));
             const float frmax = __double2float_ru(wmax(2.0 * hs));
-            const float M = flim >= 0.f ? moved_near(smem[w], A, root, fgx0, fgy0, fgz0, fgx1, fgy1,
+            const float M = flim >= 0.f ? moved_near(smem, A, root, fgx0, fgy0, fgz0, fgx1, fgy1,
                                                      fgz1, frmax, flim, B.gdm)
                                         : INFINITY;
             if (M <= flim) {
@@ -1105,6 +1100,7 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, SPLIT > 1 ? 4 : 8)
         if (km && lane == 0 && B.kept) atomicAdd(B.kept, __popc(km));
         // searched after all, at the usual radius
         if (rt >= 2 && part) hci = cand_half_radius(pi.w, B.hnb[i], B.grow);
+        int chunks = 0;
         for (int round = 0; round < B.rounds; round++) {
             const bool first_keep = km && round == 0;
             const bool any = __any_sync(FULL, act);
@@ -1113,14 +1109,18 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, SPLIT > 1 ? 4 : 8)
             double S0 = 0.0, D0 = 0.0;
             bool run = act;
             if (any) {
-                HSums<R> hs;
-                hs.inv_h = R(1.0 / pi.w);
-                craw = group_search<0, R, SPLIT>(smem[w], A, root, act, i, pi, 2.0 * hci, &hs);
-                S0 = hs.S.value();
-                D0 = hs.D.value();
-                if (SPLIT > 1) {
-                    S0 = seg_sum<SPLIT>(S0);
-                    D0 = seg_sum<SPLIT>(D0);
+                if constexpr (SPLIT > 1) {
+                    // the sums from the rows: a chunk leaves a few hits to a unit, so sums
+                    // inside the search kept most lanes waiting (10k FP64 150 -> 137 us)
+                    craw = group_search<2, R, SPLIT>(smem, A, root, act, i, pi, 2.0 * hci, nullptr,
+                                                     &chunks);
+                    eval_rows<R, SPLIT>(A, B, act && craw <= A.K, i, pi.w, craw, S0, D0);
+                } else {
+                    HSums<R> hs;
+                    hs.inv_h = R(1.0 / pi.w);
+                    craw = group_search<0, R, SPLIT>(smem, A, root, act, i, pi, 2.0 * hci, &hs);
+                    S0 = hs.S.value();
+                    D0 = hs.D.value();
                 }
             } else {
                 // the unit kept its rows (no lane searches)
@@ -1136,8 +1136,18 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, SPLIT > 1 ? 4 : 8)
             B.hc[i] = hci;
             B.retry[i] = 0;
         }
+        if (SPLIT >= 8 && lane == 0 && chunks > B.longest[0]) atomicMax(B.longest, chunks);
         __syncwarp();
     }
+}
+
+template <class R, int SPLIT>
+__global__ void __launch_bounds__(SEARCH_WARPS * 32, SPLIT > 1 ? 4 : 8)
+    k_cand_newton(const int *__restrict__ ngroup_p, SearchArgs A, NewtonArgs B, unsigned *queue) {
+    __shared__ SearchSmem smem[SEARCH_WARPS];
+    SearchSmem &S = smem[threadIdx.x >> 5];
+    if (SPLIT == 8 && B.longest[1]) newton_units<R, 32>(S, *ngroup_p, A, B, queue);
+    else newton_units<R, SPLIT>(S, *ngroup_p, A, B, queue);
 }
 
 struct CountArgs {
@@ -1412,6 +1422,7 @@ SearchArgs search_args(sph_ctx *ctx, int *rows, int *cnt) {
     A.cidx = ctx->cand_idx;
     A.ngb_cnt = ctx->ngb_cnt;
     A.hnb = ctx->st[ctx->cur][ST_HNB];
+    A.cloud = ctx->cloud[ctx->cur];
     A.only = nullptr;
     A.only_all = nullptr;
     A.mlist = nullptr;
@@ -1433,12 +1444,18 @@ SearchArgs search_args(sph_ctx *ctx, int *rows, int *cnt) {
 //     60k 100 / 107 / 114
 //   count iteration:  2k 219 / 160 / 97 / 67;  30k 323 / 251 / 253;
 //     45k 328 / 392 / 369
+// and with 8 / 32 lanes (settled and evolved h iterations: k_kept_shift):
+//   lists, tree search:  1k 31 / 18;  3k 33 / 23;  5k 39 / 31;  8k 42 / 40
+//   count iteration:  1k 106 / 83;  3k 108 / 82;  5k 91 / 92;  8k 130 / 127
+//   h iterations of a call, FP64:  1k 210 / 200;  3k 257 / 227 and 667 / 440 after
+//     60 steps;  5k 283 / 337 and 639 / 508
 int search_split(const sph_ctx *ctx) {
     const long long n = ctx->n, sm = ctx->num_sms;
-    return n <= SPLIT8_PER_SM * sm ? 8 : n <= SPLIT4_PER_SM * sm ? 4 : n <= SPLIT2_PER_SM * sm ? 2 : 1;
+    return n <= SPLIT32_PER_SM * sm ? 32 : n <= SPLIT8_PER_SM * sm ? 8 : n <= SPLIT4_PER_SM * sm ? 4 : n <= SPLIT2_PER_SM * sm ? 2 : 1;
 }
 #define SPH_SPLIT(ctx, rc, call)                                          \
     switch (search_split(ctx)) {                                          \
+        case 32: { constexpr int SPLIT = 32; rc = call; break; }          \
         case 8: { constexpr int SPLIT = 8; rc = call; break; }            \
         case 4: { constexpr int SPLIT = 4; rc = call; break; }            \
         case 2: { constexpr int SPLIT = 2; rc = call; break; }            \
@@ -1490,7 +1507,8 @@ int launch_smoothing_h(sph_ctx *ctx) {
     U.dmv_max = ctx->dmv_max;
     U.cloud = ctx->cloud[c];
     U.kept = ctx->kept_cnt;
-    k_kept_shift<<<1, 1, 0, s>>>(ctx->kept_cnt);
+    const double per_sm = (double)n / ctx->num_sms;
+    k_kept_shift<<<1, 1, 0, s>>>(ctx->kept_cnt, (int)(LONG8 * per_sm), (int)(LONG32 * per_sm));
     ctx->kept_counted = true;
     k_h_init<<<div_up(n, 256), 256, 0, s>>>(n, ctx->st[c][ST_H], ctx->st[c][ST_HNB], ctx->hcand,
                                             ctx->retry, H_GROW, ctx->hover, U);
@@ -1509,6 +1527,7 @@ int launch_smoothing_h(sph_ctx *ctx) {
     B.gdm = ctx->gdm;
     B.kept = ctx->kept_cnt;
     B.retry = ctx->retry;
+    B.longest = ctx->kept_cnt + 3;
     B.n_ngb = ctx->cfg.n_ngb;
     B.tol = ctx->cfg.h_tol;
     B.grow = H_GROW;
@@ -1632,7 +1651,7 @@ int launch_lists_marked(sph_ctx *ctx) {
     if (rc) return rc;
     SPH_SPLIT(ctx, rc, search_launch(ctx, k_lists<SPLIT>, SPLIT, A));
     if (rc) return rc;
-    k_lists_list<<<ctx->num_sms * 2, SEARCH_WARPS * 32, 0, ctx->stream>>>(ctx->d_ngroup, A);
+    k_lists_list<<<ctx->num_sms * 2, SEARCH_WARPS * 32, 0, ctx->stream>>>(A);
     return ctx_check_launch(ctx, "lists_marked");
 }
 

@@ -138,7 +138,8 @@ struct sph_ctx {
     float *gdm = nullptr;   // per particle: the largest dmv of its group (rounded up)
     int *rows_ok = nullptr;  // device flag: the rows, hsr and dmv belong to the storage order
     bool rows_host = false;  // host view of rows_ok, for the choice of launches only
-    int *kept_cnt = nullptr;     // [0] particles whose row the last h iteration kept (3 ints)
+    int *kept_cnt = nullptr;     // [0] particles whose row the last h iteration kept, [3] its longest
+                                 // search, [4] whether units are single particles (5 ints)
     bool kept_counted = false;   // that count belongs to the last h iteration
     bool lists_ok = false, rho_ok = false, divcurl_ok = false;
 
