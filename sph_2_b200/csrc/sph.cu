@@ -219,18 +219,25 @@ __global__ void __launch_bounds__(256)
                            double gamma, int balsara, double *__restrict__ rho_out,
                            double *__restrict__ P_out, double *__restrict__ c_out,
                            double *__restrict__ divV, double *__restrict__ curlV) {
-    const bool every = *all != 0;
-    const int m = every ? n : *mcount;
+    const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)gridDim.x * blockDim.x;
-    // the trip count is the same for every thread (the segment sums need
+    // the trip counts are the same for every thread (the segment sums need
     // the whole warp)
-    for (long long base = 0; base < (long long)m * LANES; base += stride) {
-        const long long t = base + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-        const int e = (int)(t / LANES), sl = (int)(t % LANES);
-        const bool ok = e < m;
-        const int i = ok ? (every ? e : mlist[e]) : 0;
-        density_divcurl_one<R, LANES>(ok, i, sl, p0, p1, p2, rows, cnt, K, u, gamma, balsara,
-                                      rho_out, P_out, c_out, divV, curlV);
+    if (*all != 0) {
+        for (long long base = 0; base < (long long)n * LANES; base += stride) {
+            const int i = (int)((base + first) / LANES), sl = (int)(first % LANES);
+            density_divcurl_one<R, LANES>(i < n, i < n ? i : 0, sl, p0, p1, p2, rows, cnt, K, u,
+                                          gamma, balsara, rho_out, P_out, c_out, divV, curlV);
+        }
+        return;
+    }
+    // a warp per listed particle: a hundred of them fill no SM (4 / 32 lanes:
+    // 10k FP64 11.9 / 4.5 us, 100k 14.4 / 5.1)
+    const int m = *mcount;
+    for (long long base = 0; base < (long long)m * 32; base += stride) {
+        const int e = (int)((base + first) / 32);
+        density_divcurl_one<R, 32>(e < m, e < m ? mlist[e] : 0, threadIdx.x & 31, p0, p1, p2, rows,
+                                   cnt, K, u, gamma, balsara, rho_out, P_out, c_out, divV, curlV);
     }
 }
 
@@ -568,8 +575,27 @@ int run_force(sph_ctx *ctx, bool acc, bool du) {
     return SPH_OK;
 }
 
+// Lanes per particle: the configured number, or more where a cloud would leave
+// the chip idle (a pass is then as long as one lane's share of a list).  us with
+// 4 / 8 / 16 / 32 lanes, an Evrard sphere of N particles on 148 SMs:
+//   lists and density, FP64:  1k 33 / 21 / 13 / 8;  3k 34 / 22 / 13 / 11;
+//     10k 34 / 21 / 21 / 25;  20k 38 / 37 / 37 / 43;  40k 62 / 63 / 65 / 79;
+//     65k 92 / 95 / 104 / 130
+//   the same in FP32:  3k 26 / 16 / 11 / 8;  10k 25 / 17 / 17 / 18;
+//     20k 29 / 28 / 26 / 30;  40k 46 / 41 / 44 / 55;  65k 61 / 62 / 69 / 88
+//   force, FP64:  3k 20 / 13 / 8 / 9;  10k 22 / 22 / 19 / 21;  20k 40 / 33 / 33 / 37;
+//     40k 60 / 57 / 59 / 71;  65k 84 / 84 / 94 / 115
+//   force, FP32:  3k 13 / 9 / 6 / 5;  10k 14 / 10 / 7 / 9;  20k 15 / 11 / 12 / 15;
+//     40k 21 / 20 / 22 / 26
+// The lines are in particles per SM.
+int lanes(const sph_ctx *ctx) {
+    const long long n = ctx->n, sm = ctx->num_sms;
+    const int least = n <= 21 * sm ? 32 : n <= 75 * sm ? 16 : n <= 300 * sm ? 8 : 1;
+    return max(ctx->cfg.ngb_lanes, least);
+}
+
 #define SPH_DISPATCH_LANES(FN, R, ctx, ...)                 \
-    switch ((ctx)->cfg.ngb_lanes) {                         \
+    switch (lanes(ctx)) {                                   \
         case 1: rc = FN<R, 1>(ctx, ##__VA_ARGS__); break;   \
         case 2: rc = FN<R, 2>(ctx, ##__VA_ARGS__); break;   \
         case 4: rc = FN<R, 4>(ctx, ##__VA_ARGS__); break;   \
