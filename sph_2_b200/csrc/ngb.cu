@@ -141,9 +141,11 @@ struct SearchArgs {
     // exact search restricted to the particles with only[i] != 0, or to all
     // of them when *only_all != 0 (null: every particle)
     const int *only, *only_all;
-    // with only: the marked particles also listed (mlist, *mcount entries);
-    // k_lists then runs only when *only_all, k_lists_list otherwise
+    // with only: the marked particles also listed (mlist, *mcount entries): up
+    // to mmax of them are searched one by one (k_lists_list), more by k_lists
     const int *mlist, *mcount;
+    int mmax;
+    __device__ __forceinline__ bool listed() const { return !*only_all && *mcount <= mmax; }
     long long *status;
 };
 
@@ -564,7 +566,7 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32)
     __shared__ SearchSmem smem[SEARCH_WARPS];
     const int w = threadIdx.x >> 5;
     const int nunit = *ngroup_p * SPLIT;
-    if (A.mlist && !*A.only_all) return;  // the listed particles: k_lists_list
+    if (A.only && A.listed()) return;  // k_lists_list
     for (int it = q_first(queue, blockIdx.x * SEARCH_WARPS + w); it < nunit;
          it = q_next(queue, it, gridDim.x * SEARCH_WARPS)) {
         const Unit<SPLIT> u(A, it);
@@ -577,13 +579,13 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32)
 }
 
 // exact lists for the listed particles (A.mlist, *A.mcount entries; nothing
-// when *A.only_all, which k_lists covers): one warp per particle, its own box, a
+// when they are too many, which k_lists covers): one warp per particle, its own box, a
 // staged candidate per lane (one lane for all of them: 10k 27 us, 1M 50; here 18 and 35)
 __global__ void __launch_bounds__(SEARCH_WARPS * 32)
     k_lists_list(SearchArgs A) {
     __shared__ SearchSmem smem[SEARCH_WARPS];
     const int w = threadIdx.x >> 5;
-    if (*A.only_all) return;
+    if (!A.listed()) return;
     const int m = *A.mcount;
     for (int e = blockIdx.x * SEARCH_WARPS + w; e < m; e += gridDim.x * SEARCH_WARPS) {
         const int i = A.mlist[e];
@@ -595,62 +597,90 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32)
 // Exact lists from the candidate rows of the h iteration.  A pair with
 // |r| <= h_i + h_j lies inside 2 max(h_i, h_j), so it sits in the candidate
 // row of the particle with the larger h (2 h <= 2 hc, the radius of that
-// particle's last candidate search).  Each lane filters its own row with the
-// exact predicate (same rounding as the tree search); where a pair's partner
-// j did not hold i in its own row (|r| beyond 2 hc_j, with a margin for
-// rounding), j's list may miss i and j is marked for the tree search.  A row
-// that is not a complete candidate set (overflow, or h above the candidate
-// radius after the last round) sends every particle to the tree search.
-__global__ void __launch_bounds__(SEARCH_WARPS * 32, 6)
-    k_lists_cand(const int *__restrict__ ngroup_p, SearchArgs A, const double *__restrict__ hc,
-                 int *__restrict__ full, int *__restrict__ full_all, int *__restrict__ full_any) {
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ngroup = *ngroup_p;
-    const int K = A.K;
-    for (int g = blockIdx.x * SEARCH_WARPS + w; g < ngroup; g += gridDim.x * SEARCH_WARPS) {
-        const int s0 = A.gstart[g], gc = A.gcount[g];
-        if (lane >= gc) continue;
-        const int i = s0 + lane;
-        const double4 pi = A.p0[i];
-        const int craw = A.cnt[i];
-        if (craw > K || !(pi.w <= hc[i])) {
-            *full_all = 1;
-            *full_any = 1;
-            continue;
+// particle's last candidate search).  The particle's LANES lanes filter its row
+// with the exact predicate (same rounding as the tree search), the list in
+// candidate order; where a pair's partner j did not hold i in its own row (|r|
+// beyond 2 hc_j, with a margin for rounding), j's list may miss i and j is
+// marked for the tree search and listed.  A row that is not a complete
+// candidate set (overflow, or h above the candidate radius after the last
+// round) sends every particle to the tree search.  Bound by the latency of its
+// gathers, two rounds of them under way at a time (a lane per particle, 100k:
+// 130 us; with 4 lanes 63).
+template <int LANES>
+__global__ void __launch_bounds__(256)
+    k_lists_cand(int n, SearchArgs A, const double *__restrict__ hc, int *__restrict__ full,
+                 int *__restrict__ full_all, int *__restrict__ full_any, int *__restrict__ mlist,
+                 int *__restrict__ mcount) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(t / LANES), sl = (int)(t % LANES);
+    const int lane = threadIdx.x & 31, K = A.K;
+    const unsigned seg = LANES == 32 ? FULL : ((1u << LANES) - 1u) << (lane & ~(LANES - 1));
+    const unsigned below = (1u << lane) - 1u;
+    const bool valid = i < n;
+    const double4 *__restrict__ p0 = A.p0;
+    double4 pi = make_double4(0.0, 0.0, 0.0, 1.0);
+    int craw = 0;
+    bool whole = false;
+    if (valid) {
+        pi = p0[i];
+        craw = A.cnt[i];
+        whole = craw <= K && pi.w <= hc[i];
+        if (!whole) {
+            craw = 0;
+            if (sl == 0) {
+                *full_all = 1;
+                *full_any = 1;
+            }
         }
-        const int *crow = A.cidx + (size_t)i * K;
-        const double4 *__restrict__ p0 = A.p0;
-        int count = 0;
-        double hnb = 0.0;
-        // four candidates per round: their index, position and radius loads
-        // are issued together (the loop is bound by gather latency)
-        constexpr int U = 4;
-        for (int k0 = 0; k0 < craw; k0 += U) {
-            int jj[U];
-            double4 pj[U];
-            double hj[U];
+    }
+    // one trip count for the warp: the ballots need every lane
+    int kmax = craw;
+    for (int o = 16; o; o >>= 1) kmax = max(kmax, __shfl_xor_sync(FULL, kmax, o));
+    const int *crow = A.cidx + (size_t)(valid ? i : 0) * K;
+    int count = 0;
+    double hnb = 0.0;
+    constexpr int U = 2;
+    for (int k0 = 0; k0 < kmax; k0 += U * LANES) {
+        int jj[U];
+        double4 pj[U];
+        double hj[U];
 #pragma unroll
-            for (int u = 0; u < U; u++) jj[u] = k0 + u < craw ? __ldg(&crow[k0 + u]) : i;
+        for (int u = 0; u < U; u++) {
+            const int k = k0 + u * LANES + sl;
+            jj[u] = k < craw ? __ldg(&crow[k]) : -1;
+        }
 #pragma unroll
-            for (int u = 0; u < U; u++) {
+        for (int u = 0; u < U; u++) {
+            pj[u] = pi;
+            hj[u] = 0.0;
+            if (jj[u] >= 0) {
                 pj[u] = ld_wide(p0 + jj[u]);
                 hj[u] = __ldg(&hc[jj[u]]);
             }
+        }
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                if (k0 + u < craw && ngb_pred(pi.x, pi.y, pi.z, pi.w, pj[u].x, pj[u].y, pj[u].z, pj[u].w)) {
-                    if (count < K) A.rows[(size_t)i * K + count] = jj[u];
-                    count++;
-                    hnb = fmax(hnb, pj[u].w);
-                    const double dx = pi.x - pj[u].x, dy = pi.y - pj[u].y, dz = pi.z - pj[u].z;
-                    const double rj = 2.0 * hj[u];
-                    if (dx * dx + dy * dy + dz * dz > rj * rj * (1.0 - 1e-9)) {
-                        full[jj[u]] = 1;
-                        *full_any = 1;
-                    }
+        for (int u = 0; u < U; u++) {
+            const int j = jj[u];
+            const bool hit =
+                j >= 0 && ngb_pred(pi.x, pi.y, pi.z, pi.w, pj[u].x, pj[u].y, pj[u].z, pj[u].w);
+            const unsigned m = __ballot_sync(FULL, hit) & seg;
+            if (hit) {
+                const int pos = count + __popc(m & below);
+                if (pos < K) A.rows[(size_t)i * K + pos] = j;
+                hnb = fmax(hnb, pj[u].w);
+                const double dx = pi.x - pj[u].x, dy = pi.y - pj[u].y, dz = pi.z - pj[u].z;
+                const double rj = 2.0 * hj[u];
+                if (dx * dx + dy * dy + dz * dz > rj * rj * (1.0 - 1e-9)) {
+                    // j joins the list of particles to search once
+                    if (atomicExch(&full[j], 1) == 0) mlist[atomicAdd(mcount, 1)] = j;
+                    *full_any = 1;
                 }
             }
+            count += __popc(m);
         }
+    }
+    for (int o = LANES / 2; o; o >>= 1) hnb = fmax(hnb, __shfl_xor_sync(FULL, hnb, o));
+    if (whole && sl == 0) {
         A.ngb_cnt[i] = min(count, K);
         if (count > K) status_add(A.status, SPH_S_NGB_OVERFLOW, 1);
         A.hnb[i] = hnb;
@@ -1427,6 +1457,7 @@ SearchArgs search_args(sph_ctx *ctx, int *rows, int *cnt) {
     A.only_all = nullptr;
     A.mlist = nullptr;
     A.mcount = nullptr;
+    A.mmax = 0;
     A.p1 = ctx->p1;
     A.status = ctx->status;
     return A;
@@ -1611,27 +1642,40 @@ int launch_smoothing_kth(sph_ctx *ctx, int k) {
     return ctx_check_launch(ctx, "smoothing_kth");
 }
 
+// restrict a list search to the particles the pass over the rows marked.  One
+// by one they cost about 1 us per 79 of them, the groups' search of 100k
+// particles 277 us however few a group holds: the lines cross near a fifth.
+static void marked_lists(const sph_ctx *ctx, SearchArgs &A) {
+    A.only = ctx->lflag;
+    A.only_all = ctx->lflag + ctx->n;
+    A.mlist = ctx->mlist;
+    A.mcount = ctx->lflag + ctx->n + 2;
+    A.mmax = max(1024, ctx->n / 8);
+}
+
 int launch_neighbours(sph_ctx *ctx) {
     const int n = ctx->n;
     if (n <= 0) return SPH_OK;
     cudaStream_t s = ctx->stream;
-    const int grid = max(1, div_up(div_up(n, 16) + ctx->ncloud, SEARCH_WARPS));
     SearchArgs A = search_args(ctx, ctx->ngb, ctx->ngb_cnt);
     if (ctx->cand_ok) {
         // lists from the candidate rows, then the tree search for the
         // particles whose rows cannot show that their list is complete
-        CK(cudaMemsetAsync(ctx->lflag, 0, sizeof(int) * (n + 2), s));
-        SearchArgs C = search_args(ctx, ctx->ngb, ctx->cand_cnt);
-        k_lists_cand<<<grid, SEARCH_WARPS * 32, 0, s>>>(ctx->d_ngroup, C, ctx->hcand, ctx->lflag,
-                                                       ctx->lflag + n, ctx->lflag + n + 1);
-        A.only = ctx->lflag;
-        A.only_all = ctx->lflag + n;
+        CK(cudaMemsetAsync(ctx->lflag, 0, sizeof(int) * (n + 3), s));
+        marked_lists(ctx, A);
+        const int l = max(4, pass_lanes(ctx));
+        auto kern = l == 4 ? k_lists_cand<4> : l == 8 ? k_lists_cand<8>
+                                           : l == 16 ? k_lists_cand<16> : k_lists_cand<32>;
+        kern<<<div_up((long long)n * l, 256), 256, 0, s>>>(
+            n, search_args(ctx, ctx->ngb, ctx->cand_cnt), ctx->hcand, ctx->lflag, ctx->lflag + n,
+            ctx->lflag + n + 1, ctx->mlist, ctx->lflag + n + 2);
     }
     // node h_max only matters to the tree search: skipped when no list needs it
     int rc = launch_refit_hmax(ctx, ctx->cand_ok ? ctx->lflag + n + 1 : nullptr);
     if (rc) return rc;
     SPH_SPLIT(ctx, rc, search_launch(ctx, k_lists<SPLIT>, SPLIT, A));
     if (rc) return rc;
+    if (A.only) k_lists_list<<<ctx->num_sms * 2, SEARCH_WARPS * 32, 0, s>>>(A);
     ctx->lists_ok = true;
     ctx->rho_ok = ctx->divcurl_ok = false;
     return ctx_check_launch(ctx, "neighbours");
@@ -1643,10 +1687,7 @@ int launch_lists_marked(sph_ctx *ctx) {
     const int n = ctx->n;
     if (n <= 0) return SPH_OK;
     SearchArgs A = search_args(ctx, ctx->ngb, ctx->ngb_cnt);
-    A.only = ctx->lflag;
-    A.only_all = ctx->lflag + n;
-    A.mlist = ctx->mlist;
-    A.mcount = ctx->lflag + n + 2;
+    marked_lists(ctx, A);
     int rc = launch_refit_hmax(ctx, ctx->lflag + n + 1);
     if (rc) return rc;
     SPH_SPLIT(ctx, rc, search_launch(ctx, k_lists<SPLIT>, SPLIT, A));

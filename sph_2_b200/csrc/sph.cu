@@ -29,6 +29,25 @@
 #define SPH_FORCE_MINB 5
 #endif
 
+// Lanes per particle: the configured number, or more where a cloud would leave
+// the chip idle (a pass is then as long as one lane's share of a list).  us with
+// 4 / 8 / 16 / 32 lanes, an Evrard sphere of N particles on 148 SMs:
+//   lists and density, FP64:  1k 33 / 21 / 13 / 8;  3k 34 / 22 / 13 / 11;
+//     10k 34 / 21 / 21 / 25;  20k 38 / 37 / 37 / 43;  40k 62 / 63 / 65 / 79;
+//     65k 92 / 95 / 104 / 130
+//   the same in FP32:  3k 26 / 16 / 11 / 8;  10k 25 / 17 / 17 / 18;
+//     20k 29 / 28 / 26 / 30;  40k 46 / 41 / 44 / 55;  65k 61 / 62 / 69 / 88
+//   force, FP64:  3k 20 / 13 / 8 / 9;  10k 22 / 22 / 19 / 21;  20k 40 / 33 / 33 / 37;
+//     40k 60 / 57 / 59 / 71;  65k 84 / 84 / 94 / 115
+//   force, FP32:  3k 13 / 9 / 6 / 5;  10k 14 / 10 / 7 / 9;  20k 15 / 11 / 12 / 15;
+//     40k 21 / 20 / 22 / 26
+// The lines are in particles per SM.
+int pass_lanes(const sph_ctx *ctx) {
+    const long long n = ctx->n, sm = ctx->num_sms;
+    const int least = n <= 21 * sm ? 32 : n <= 75 * sm ? 16 : n <= 300 * sm ? 8 : 1;
+    return max(ctx->cfg.ngb_lanes, least);
+}
+
 namespace {
 
 template <class R, int LANES>
@@ -575,27 +594,8 @@ int run_force(sph_ctx *ctx, bool acc, bool du) {
     return SPH_OK;
 }
 
-// Lanes per particle: the configured number, or more where a cloud would leave
-// the chip idle (a pass is then as long as one lane's share of a list).  us with
-// 4 / 8 / 16 / 32 lanes, an Evrard sphere of N particles on 148 SMs:
-//   lists and density, FP64:  1k 33 / 21 / 13 / 8;  3k 34 / 22 / 13 / 11;
-//     10k 34 / 21 / 21 / 25;  20k 38 / 37 / 37 / 43;  40k 62 / 63 / 65 / 79;
-//     65k 92 / 95 / 104 / 130
-//   the same in FP32:  3k 26 / 16 / 11 / 8;  10k 25 / 17 / 17 / 18;
-//     20k 29 / 28 / 26 / 30;  40k 46 / 41 / 44 / 55;  65k 61 / 62 / 69 / 88
-//   force, FP64:  3k 20 / 13 / 8 / 9;  10k 22 / 22 / 19 / 21;  20k 40 / 33 / 33 / 37;
-//     40k 60 / 57 / 59 / 71;  65k 84 / 84 / 94 / 115
-//   force, FP32:  3k 13 / 9 / 6 / 5;  10k 14 / 10 / 7 / 9;  20k 15 / 11 / 12 / 15;
-//     40k 21 / 20 / 22 / 26
-// The lines are in particles per SM.
-int lanes(const sph_ctx *ctx) {
-    const long long n = ctx->n, sm = ctx->num_sms;
-    const int least = n <= 21 * sm ? 32 : n <= 75 * sm ? 16 : n <= 300 * sm ? 8 : 1;
-    return max(ctx->cfg.ngb_lanes, least);
-}
-
 #define SPH_DISPATCH_LANES(FN, R, ctx, ...)                 \
-    switch (lanes(ctx)) {                                   \
+    switch (pass_lanes(ctx)) {                              \
         case 1: rc = FN<R, 1>(ctx, ##__VA_ARGS__); break;   \
         case 2: rc = FN<R, 2>(ctx, ##__VA_ARGS__); break;   \
         case 4: rc = FN<R, 4>(ctx, ##__VA_ARGS__); break;   \

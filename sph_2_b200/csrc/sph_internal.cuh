@@ -394,6 +394,7 @@ int launch_smoothing_h(sph_ctx *ctx);
 int launch_smoothing_h_count(sph_ctx *ctx, int n_target, int n_tol, double frac, int max_iter);
 int launch_smoothing_kth(sph_ctx *ctx, int k);
 int launch_neighbours(sph_ctx *ctx);
+int pass_lanes(const sph_ctx *ctx);  // lanes per particle of the passes over rows and lists
 int launch_density(sph_ctx *ctx);
 int launch_divcurl(sph_ctx *ctx);
 int launch_density_divcurl(sph_ctx *ctx);

@@ -27,6 +27,7 @@ def test_pass_lanes(n, precision, tol):
             ctx.load(d["pos"], vel, d["m"], d["h"], d["u"])
             if fused:
                 ctx.prologue()
+                ctx.step(1)
             else:
                 ctx.sort()
                 ctx.build_tree()
@@ -40,10 +41,37 @@ def test_pass_lanes(n, precision, tol):
             acc, du, vs = O.force_list(x, y, z, *v.T.copy(), rho, P, c, h, m, dv, cv, 1.0, 2.0, 0.1, 1, 1,
                                        off, lst)
             assert _rel(ctx.get("rho", True), rho) < tol
+            go, gl = ctx.neighbour_lists()
+            assert np.array_equal(go, off) and np.array_equal(gl, lst)
+            if fused:
+                continue  # the step's last kick has moved v and u on since its passes
             assert _rel(ctx.get("divV", True), dv) < 10 * tol
             assert _rel(ctx.get("curlV", True), cv) < 10 * tol
-            if fused:
-                continue  # the prologue goes on from these to its first kick
             assert _rel(ctx.get_acc("sph", True), acc) < 10 * tol
             assert _rel(ctx.get("dudt", True), du) < 10 * tol
             assert _rel(ctx.get("vsig", True), vs) < 10 * tol
+
+
+@pytest.mark.parametrize("heavy", [0.0, 0.3])
+def test_marked_lists(heavy):
+    """The lists that the rows cannot show to be complete: most of them before
+    any list has told the rows how far to reach (searched by groups), a few
+    after that (one by one)."""
+    n = 20_000
+    d = ic.evrard(n, seed=6)
+    m = d["m"] * np.where(np.random.default_rng(4).random(n) < heavy, 12.0, 1.0)
+    with Context(Config(n_max=n, precision="fp64", max_ngb=512)) as ctx:
+        ctx.load(d["pos"], d["vel"], m, d["h"], d["u"])
+        ctx.sort()
+        ctx.build_tree()
+        marked = []
+        for _ in range(2):
+            ctx.smoothing_h()
+            ctx.neighbours()
+            marked.append(int(ctx.debug_array("tree_search")[:n].sum()))
+            x, y, z = ctx.get_pos(True).T.copy()
+            off, lst = O.neighbours(x, y, z, ctx.get("h", True))
+            assert np.diff(off).max() <= 512
+            go, gl = ctx.neighbour_lists()
+            assert np.array_equal(go, off) and np.array_equal(gl, lst)
+        assert marked[0] > n // 8 and (marked[1] > n // 8) == (heavy > 0)
