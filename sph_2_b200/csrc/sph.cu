@@ -28,6 +28,13 @@
 #ifndef SPH_FORCE_MINB
 #define SPH_FORCE_MINB 5
 #endif
+// the same of the FP64 passes: bound by the latency of their dependent FP64
+// chains, they gain from 24 warps per SM (80 registers) over the 16 of their
+// 105 (force 65k 111 / 107 -> 100 / 82 us with w only where it is used; 4
+// blocks spill: 99 / 81, 10k 21 -> 23; lists and density 100k 141 -> 129)
+#ifndef SPH_FP64_MINB
+#define SPH_FP64_MINB 3
+#endif
 
 // Lanes per particle: the configured number, or more where a cloud would leave
 // the chip idle (a pass is then as long as one lane's share of a list).  us with
@@ -271,7 +278,7 @@ __global__ void __launch_bounds__(256)
 // from that list; a row that is not a complete candidate set (overflow, or h
 // above the candidate radius) marks every particle.
 template <class R, int LANES>
-__global__ void __launch_bounds__(256, std::is_same<R, float>::value ? SPH_LISTS_MINB : 1)
+__global__ void __launch_bounds__(256, std::is_same<R, float>::value ? SPH_LISTS_MINB : SPH_FP64_MINB)
     k_cand_density_divcurl(int n, const double4 *__restrict__ p0,
                            const typename R4<R>::T *__restrict__ p1,
                            typename R4<R>::T *__restrict__ p2, const int *__restrict__ crows,
@@ -389,7 +396,7 @@ __global__ void __launch_bounds__(256, std::is_same<R, float>::value ? SPH_LISTS
 // du_i  =  sum m_j (P_i/rho_i^2 + PI_ij/2) v_ij . gradW_ij,
 // vsig_i = max_j (c_i + c_j - 3 w_ij), w_ij = v_ij.r_ij/(r_ij + 1e-5).
 template <class R, int LANES>
-__global__ void __launch_bounds__(256, std::is_same<R, float>::value ? SPH_FORCE_MINB : 1)
+__global__ void __launch_bounds__(256, std::is_same<R, float>::value ? SPH_FORCE_MINB : SPH_FP64_MINB)
     k_force(int n, const double4 *__restrict__ p0, const typename R4<R>::T *__restrict__ p1,
             const typename R4<R>::T *__restrict__ p2, const int *__restrict__ rows,
             const int *__restrict__ cnt, int K, int av_mode, int balsara, R alpha, R beta, R eta,
@@ -406,6 +413,8 @@ __global__ void __launch_bounds__(256, std::is_same<R, float>::value ? SPH_FORCE
         const int c = cnt[i];
         const int *row = rows + (size_t)i * K;
         const R eta2 = eta * eta;
+        // w enters the signal velocity and the Gadget viscosity only
+        const bool want_w = want_acc || av_mode != SPH_AV_MG83;
         for (int k = sl; k < c; k += LANES) {
             const int j = row[k];
             const double4 pj = ld_pos<R>(p0 + j);
@@ -419,7 +428,7 @@ __global__ void __launch_bounds__(256, std::is_same<R, float>::value ? SPH_FORCE
             const R gx = nW * dx, gy = nW * dy, gz = nW * dz;
             const R ux = vi.x - vj.x, uy = vi.y - vj.y, uz = vi.z - vj.z;
             const R vr = ux * dx + uy * dy + uz * dz;
-            const R w = qdiv<R>(vr, rr + R(1e-5));
+            const R w = want_w ? qdiv<R>(vr, rr + R(1e-5)) : R(0);
             R PI = R(0);
             if (vr <= R(0)) {
                 const R rhoij = R(0.5) * (qi.x + qj.x);
