@@ -368,8 +368,9 @@ __device__ __forceinline__ void part_sums(const V4 *sa, int m, const V4 &p, R ep
     }
 }
 
-template <bool POT>
-__global__ void __launch_bounds__(WALK_WARPS * 32, POT ? 1 : 6)
+// (BLOCKS per SM: run_walk)
+template <bool POT, int BLOCKS>
+__global__ void __launch_bounds__(WALK_WARPS * 32, POT ? 1 : BLOCKS)
     k_walk(const int *__restrict__ ngroup_p, const int *__restrict__ gstart, const int *__restrict__ gcount,
            const int *__restrict__ gcloud, const int *__restrict__ croot,
            const float4 *__restrict__ pw, const float4 *__restrict__ wA,
@@ -1417,8 +1418,15 @@ int run_walk(sph_ctx *ctx, cudaStream_t s) {
     // (the FP64 walk takes blocks at every size)
     const int warps = walk_warps(ctx);
     auto kern = warps == 4 ? k_walk_block<R, POT, 4> : k_walk_block<R, POT, 2>;
-    if constexpr (std::is_same<R, float>::value)
-        if (warps == 1) kern = k_walk<POT>;
+    if constexpr (std::is_same<R, float>::value) {
+        // Registers for six blocks per SM, or for five where they are the
+        // faster ones.  us alone, six / five:  with expansions 110k 362 / 352,
+        // 131k 387 / 373, 200k 482 / 476, 400k 890 / 900, 1M 1847 / 1880; without
+        // 260k 751 / 734, 400k 1168 / 1139, 1M 2975 / 2950.  Beside the SPH passes
+        // of a step the smaller footprint counts (1M 22.9 / 23.4 ms).
+        const bool five = !ctx->in_step && (ctx->cfg.theta_local <= 0.0 || ctx->n <= 1500 * ctx->num_sms);
+        if (warps == 1) kern = five ? k_walk<POT, 5> : k_walk<POT, 6>;
+    }
     const int block = 32 * (warps > 1 ? warps : WALK_WARPS);
     if (warps > 1) {
         grid0 = max(1, div_up(ctx->n, 16) + ctx->ncloud);

@@ -53,12 +53,13 @@ def test_walk_fp64(n, clouds):
         assert np.abs(ctx.get("pot", True) - pot).max() < max(scale(pot), 1e-13)
 
 
-# with expansions the lines are 340 and 740 per SM, without 340 and 1700; the
+# with expansions the lines are 340, 740 and (registers) 1500 per SM, without 340
+# and 1700; the
 # bounds are those of the opening angle (0.35 with 0.45 for small cells, 0.5)
 @pytest.mark.parametrize("n,clouds,local", [
     (1, 1, True), (2, 1, False), (33, 1, True), (40000, 1, True), (340 * SMS, 1, True),
     (340 * SMS + 1, 1, True), (340 * SMS + 1, 1, False), (740 * SMS, 2, True), (740 * SMS + 1, 1, True),
-    (1700 * SMS, 1, False), (1700 * SMS + 1, 1, False)])
+    (1500 * SMS, 1, True), (1500 * SMS + 1, 1, True), (1700 * SMS, 1, False), (1700 * SMS + 1, 1, False)])
 def test_walk_mixed(n, clouds, local):
     kw = dict(theta=0.35, theta_local=0.28, theta_small=0.45, small_cell=128) if local else dict(theta=0.5)
     with _loaded(n, "mixed", clouds, **kw) as ctx:
