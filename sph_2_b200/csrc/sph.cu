@@ -7,7 +7,7 @@
 // with uncoalesced float loads, and the all-pairs numba loops of
 // MPI_sph/sph_code/libsx.py:52-262 and shear.py:78-485 (same formulas).
 //
-// Mapping: LANES consecutive lanes own one particle (LANES = ngb_lanes, the
+// Mapping: LANES consecutive lanes own one particle (pass_lanes: ngb_lanes or more, the
 // "neighbour chunk width", 4..32).  They read that particle's row of the
 // neighbour list contiguously and gather the neighbours' packed records
 // (p0 = double4 x,y,z,h; p1 = Real4 v,m; p2 = Real4 rho,P/rho^2,c,f); rows are
