@@ -1008,7 +1008,7 @@ __device__ __forceinline__ bool newton_rows(const SearchArgs &A, const NewtonArg
             live = false;
         }
         if (!__any_sync(FULL, live)) break;
-        if (it > 1) eval_rows<R, SPLIT>(A, B, live, i, h, craw, Ssum, Dsum);
+        if (SPLIT > 1 || it > 1) eval_rows<R, SPLIT>(A, B, live, i, h, craw, Ssum, Dsum);
         if (!live) continue;
         const double h3 = h * h * h;
         const double rho = SPH_SIG / h3 * Ssum;
@@ -1144,7 +1144,6 @@ __device__ __forceinline__ void newton_units(SearchSmem &smem, int ngroup, const
                     // inside the search kept most lanes waiting (10k FP64 150 -> 137 us)
                     craw = group_search<2, R, SPLIT>(smem, A, root, act, i, pi, 2.0 * hci, nullptr,
                                                      &chunks);
-                    eval_rows<R, SPLIT>(A, B, act && craw <= A.K, i, pi.w, craw, S0, D0);
                 } else {
                     HSums<R> hs;
                     hs.inv_h = R(1.0 / pi.w);
@@ -1155,7 +1154,7 @@ __device__ __forceinline__ void newton_units(SearchSmem &smem, int ngroup, const
             } else {
                 // the unit kept its rows (no lane searches)
                 if (keep) craw = A.cnt[i];
-                eval_rows<R, SPLIT>(A, B, keep, i, pi.w, craw, S0, D0);
+                if constexpr (SPLIT == 1) eval_rows<R, SPLIT>(A, B, keep, i, pi.w, craw, S0, D0);
                 run = keep;
             }
             act = newton_rows<R, SPLIT>(A, B, run, i, pi, hci, craw, S0, D0, any,
