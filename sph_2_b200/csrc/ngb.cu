@@ -1192,17 +1192,21 @@ __device__ __forceinline__ double ref_dist(const double4 &pi, const double4 &pj)
 }
 
 // The distances of one particle's row, entry 32 e + lane in d[e] (infinity past
-// the row's c <= 512 entries): each row is gathered once, by the whole warp.
-constexpr int SEL_MAX = 16;
-struct RowDist {
-    double d[SEL_MAX];
+// the row's c <= 32 N entries, N 4 or 16): each row is gathered once, by the
+// whole warp.  Most rows have 70 to 110 entries: the short form has no branch per
+// entry and a quarter of the code, which otherwise waited for instructions (count
+// iteration of 30k particles 248 -> 172 us, 100k 652 -> 408; k-th neighbour 50 of
+// 100k 443 -> 338).
+constexpr int SEL_MAX = 16, SEL_SHORT = 4;
+template <int N> struct RowDist {
+    double d[N];
     int c;
     __device__ __forceinline__ RowDist(const SearchArgs &A, int i, const double4 &pi, int craw)
         : c(craw) {
         const int lane = threadIdx.x & 31;
         const int *row = A.cidx + (size_t)i * A.K;
 #pragma unroll
-        for (int e = 0; e < SEL_MAX; e++) {
+        for (int e = 0; e < N; e++) {
             d[e] = INFINITY;
             if (32 * e < c && 32 * e + lane < c) d[e] = ref_dist(pi, A.p0[row[32 * e + lane]]);
         }
@@ -1224,8 +1228,9 @@ struct RowDist {
             int n = 0;
             double below = 0.0, above = INFINITY;
 #pragma unroll
-            for (int e = 0; e < SEL_MAX; e++) {
-                if (32 * e < c) {
+            for (int e = 0; e < N; e++) {
+                // (the few of a short row all at once: past the end at infinity)
+                if (N <= SEL_SHORT || 32 * e < c) {
                     const bool in = d[e] <= v;
                     n += __popc(__ballot_sync(FULL, in));
                     if (in) below = fmax(below, d[e]);
@@ -1334,12 +1339,15 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, 4)
                 // every row entry lies within 2 hc up to the rounding of the
                 // search's r^2 test
                 const double bound = 2.0 * __shfl_sync(FULL, hc, src) * (1.0 + 1e-9);
-                const RowDist R(A, ii, A.p0[ii], cc);
-                const double a = R.kth(B.lo_n, bound), b = R.kth(B.hi_n + 1, bound);
-                if ((lane & ~(SPLIT - 1)) == src) {
-                    t_lo = a;
-                    t_hi = b;
-                }
+                const auto both = [&](const auto &R) {
+#pragma unroll 1
+                    for (int q = 0; q < 2; q++) {
+                        const double v = R.kth(q ? B.hi_n + 1 : B.lo_n, bound);
+                        if ((lane & ~(SPLIT - 1)) == src) (q ? t_hi : t_lo) = v;
+                    }
+                };
+                if (cc <= 32 * SEL_SHORT) both(RowDist<SEL_SHORT>(A, ii, A.p0[ii], cc));
+                else both(RowDist<SEL_MAX>(A, ii, A.p0[ii], cc));
             }
             if (act) act = count_lane(A, B, own, h, hc, it, craw, t_lo, t_hi, round == B.rounds - 1);
         }
@@ -1381,8 +1389,9 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, 4)
                 const int src = __ffs(m) - 1;
                 const int ii = __shfl_sync(FULL, u.i, src), cc = __shfl_sync(FULL, craw, src);
                 const double bound = 2.0 * __shfl_sync(FULL, hc, src) * (1.0 + 1e-9);
-                const RowDist R(A, ii, A.p0[ii], cc);
-                const double v = R.kth(k + 1, bound);
+                const double v = cc <= 32 * SEL_SHORT
+                                     ? RowDist<SEL_SHORT>(A, ii, A.p0[ii], cc).kth(k + 1, bound)
+                                     : RowDist<SEL_MAX>(A, ii, A.p0[ii], cc).kth(k + 1, bound);
                 if ((lane & ~(SPLIT - 1)) == src) d = v;
             }
             if (!act) continue;

@@ -50,3 +50,22 @@ def test_units(n, precision):
         assert len(fits) > 0.9 * n
         for i in fits:
             assert np.array_equal(lst[off[i]:off[i + 1]], ol[oo[i]:oo[i + 1]])
+
+
+@pytest.mark.parametrize("n", [150, 2000, 20000])
+@pytest.mark.parametrize("k", [1, 60, 127, 200])
+def test_kth_short_and_long_rows(n, k):
+    """Rows on both sides of 128 entries, the k-th distance to the bit."""
+    pos = np.random.default_rng(n + k).uniform(-1.0, 1.0, size=(n, 3))
+    if k >= n:
+        pytest.skip("fewer particles than neighbours")
+    with Context(Config(n_max=n, precision="fp64", max_ngb=512)) as ctx:
+        ctx.load(pos, None, None, np.full(n, 0.3), None)
+        ctx.sort()
+        ctx.build_tree()
+        ctx.smoothing_length_kth(k)
+        assert ctx.status()["h_noconv"] == 0
+        h = ctx.get("h")
+        for i in np.random.default_rng(2).integers(0, n, 60):
+            dx, dy, dz = (pos - pos[i]).T
+            assert h[i] == 0.5 * np.sort(np.sqrt(dx * dx + dy * dy + dz * dz))[k]
