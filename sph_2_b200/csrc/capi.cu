@@ -659,6 +659,7 @@ int sph_load(sph_ctx *ctx, int32_t n, const int32_t *cloud, const double *x, con
             k_load<double><<<div_up(n, 256), 256, 0, s>>>(n, a, (double4 *)ctx->p1, (double4 *)ctx->pw);
         if ((rc = launch_rows_invalidate(ctx))) return rc;
     }
+    if ((rc = launch_units_reset(ctx))) return rc;
     CK(cudaStreamSynchronize(s));
     ctx->tree_ok = ctx->lists_ok = ctx->rho_ok = ctx->divcurl_ok = ctx->cand_ok = false;
     ctx->p2_dirty = true;

@@ -210,9 +210,11 @@ int sph_write_restart(sph_ctx *ctx, const char *path) {
         if (n > 0) CK(cudaMemcpy(buf.data(), a, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost));
         ok = F.write(buf.data(), sizeof(double) * 3 * n);
     }
-    // a context resumed from this file starts with a full rebuild; so does
-    // this one, so that both continue alike
+    // a context resumed from this file starts with a full rebuild and a new
+    // context's units; so does this one, so that both continue alike
     ctx->topo_ok = false;
+    int rc = launch_units_reset(ctx);
+    if (rc) return rc;
     return ok ? SPH_OK : SPH_ERR_IO;
 }
 
@@ -265,7 +267,7 @@ int sph_read_restart(sph_ctx *ctx, const char *path) {
     CK(cudaMemset(ctx->dt_bits, 0xff, 8 * nc));
     CK(cudaMemset(ctx->d_ngroup, 0, sizeof(int)));
     int rc = launch_pack_p1(ctx);
-    if (rc) return rc;
+    if (rc || (rc = launch_units_reset(ctx))) return rc;
     CK(cudaStreamSynchronize(s));
     ctx->tree_ok = ctx->lists_ok = ctx->rho_ok = ctx->divcurl_ok = ctx->cand_ok = false;
     ctx->p2_dirty = true;

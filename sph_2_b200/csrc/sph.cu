@@ -711,6 +711,14 @@ int launch_rows_invalidate(sph_ctx *ctx) {
     return SPH_OK;
 }
 
+// The next h iteration chooses its units as a new context's first does: the
+// last one's longest search belongs to neither a load nor a restart file, and
+// the units decide the order of a row and with it the rounding of its sums.
+int launch_units_reset(sph_ctx *ctx) {
+    CK(cudaMemsetAsync(ctx->kept_cnt + 3, 0, 2 * sizeof(int), ctx->stream));
+    return SPH_OK;
+}
+
 // track: the storage order is that of the last pack, so the records' moves
 // are added to the distances moved (the candidate rows stay usable);
 // otherwise the rows are dropped

@@ -139,7 +139,8 @@ struct sph_ctx {
     int *rows_ok = nullptr;  // device flag: the rows, hsr and dmv belong to the storage order
     bool rows_host = false;  // host view of rows_ok, for the choice of launches only
     int *kept_cnt = nullptr;     // [0] particles whose row the last h iteration kept, [3] its longest
-                                 // search, [4] whether units are single particles (5 ints)
+                                 // search, [4] whether units are single particles (5 ints;
+                                 // launch_units_reset)
     bool kept_counted = false;   // that count belongs to the last h iteration
     bool lists_ok = false, rho_ok = false, divcurl_ok = false;
 
@@ -420,6 +421,7 @@ int launch_dt_commit(sph_ctx *ctx);
 int launch_energies(sph_ctx *ctx, double *out10_host);
 int launch_pack_p1(sph_ctx *ctx, bool track = false);
 int launch_rows_invalidate(sph_ctx *ctx);
+int launch_units_reset(sph_ctx *ctx);
 int launch_export_neighbours(sph_ctx *ctx, int64_t *off_dev, int *lst_dev, int64_t cap);
 int launch_cooling_exact(sph_ctx *ctx);
 int launch_cooling_table(sph_ctx *ctx);
