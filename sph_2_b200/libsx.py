@@ -87,7 +87,10 @@ def _columns(vectors, scalars):
         raise ValueError("mix of host arrays and CUDA tensors in one call")
     if kinds.pop():
         import torch
-        keep = [a[:, :3].to(torch.float64).t().contiguous() for a in vectors]
+        for a in vectors:
+            if len(a.shape) < 2 or a.shape[1] < 3:   # as a[:, 2] of an array does
+                raise IndexError(f"an (n, 3) array is needed, got {tuple(a.shape)}")
+        keep = [a[:, :3].to(torch.float64).transpose(0, 1).contiguous() for a in vectors]
         cols = [c for t in keep for c in t]
         cols += [a.to(torch.float64).contiguous() for a in scalars]
         # the library reads them on its own stream: let torch's work finish first
