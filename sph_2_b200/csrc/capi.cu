@@ -3,6 +3,8 @@
 // reference allocates and frees the neighbour list and tree every step,
 // EVR.cu:1148, 1417-1446), field transfer in original particle order, the
 // phase entry points, the prologue and the CUDA-graph step.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -65,6 +67,48 @@ int queue_launch(sph_ctx *ctx, cudaStream_t s, int slot, const void *kernel, int
 namespace {
 
 constexpr int LOAD_STAGE = 16384;  // largest load from host arrays through pinned staging
+
+// Whether the context's kernels may use `bytes` at p as they lie: memory of its
+// device (or managed), aligned to `align`, all of it in one allocation.  What may
+// not be used so is copied: a copy takes other devices' memory and any
+// alignment, and refuses what is no range of device memory.  One object serves
+// one call and looks an allocation up once for all arrays in it.
+struct InPlace {
+    const sph_ctx *ctx;
+    CUdeviceptr begin = 0, end = 0;  // the last allocation found usable
+    bool operator()(const void *p, size_t bytes, size_t align) {
+        const CUdeviceptr q = (CUdeviceptr)p;
+        if (q % align) return false;
+        return (q >= begin && q + bytes <= end) || (find(p) && q + bytes <= end);
+    }
+    bool find(const void *p) {
+        typedef CUresult(CUDAAPI * Range)(CUdeviceptr *, size_t *, CUdeviceptr);
+        static const Range range = [] {
+            void *f = nullptr;
+            cudaDriverEntryPointQueryResult r;
+            return cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &r) ==
+                                   cudaSuccess &&
+                           r == cudaDriverEntryPointSuccess
+                       ? (Range)f
+                       : nullptr;
+        }();
+        cudaPointerAttributes a{};
+        begin = end = 0;
+        if (!range || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (!(a.type == cudaMemoryTypeManaged || (a.type == cudaMemoryTypeDevice && a.device == ctx->device)))
+            return false;
+        size_t size = 0;
+        if (range(&begin, &size, (CUdeviceptr)p) != CUDA_SUCCESS) {
+            begin = 0;
+            return false;
+        }
+        end = begin + size;
+        return true;
+    }
+};
 
 template <class T>
 int dalloc(sph_ctx *ctx, T **p, size_t count) {
@@ -628,10 +672,12 @@ int sph_load(sph_ctx *ctx, int32_t n, const int32_t *cloud, const double *x, con
                     k++;
                 }
             CK(cudaMemcpyAsync(dev, ctx->load_stage, sizeof(double) * k * n, cudaMemcpyHostToDevice, s));
-        } else if (host) {
+        } else {
+            InPlace usable{ctx};
             for (int k = 0; k < 9; k++)
-                if (in[k]) {
-                    CK(cudaMemcpyAsync(ctx->st[0][k], in[k], sizeof(double) * n, cudaMemcpyHostToDevice, s));
+                if (in[k] && (host || !usable(in[k], sizeof(double) * n, sizeof(double)))) {
+                    CK(cudaMemcpyAsync(ctx->st[0][k], in[k], sizeof(double) * n,
+                                       host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s));
                     in[k] = ctx->st[0][k];
                 }
         }
@@ -1000,19 +1046,35 @@ static int direct_common(sph_ctx *ctx, const double *eps, int32_t nt, const int3
     const int *tg = targets;
     double *res = out;
     const double *ep = eps;
-    void *tmp = nullptr;  // device copies of host arrays: eps, results, targets
-    if (host) {
-        const size_t ne = eps ? ctx->n : 0, no = (size_t)width * nt;
-        CK(cudaMalloc(&tmp, sizeof(double) * (ne + no) + sizeof(int) * nt));
-        double *d = (double *)tmp;
-        ep = d;
-        res = d + ne;
-        int *t = (int *)(res + no);
-        tg = t;
+    // device copies of eps, the results and the targets, where the kernels
+    // cannot use the caller's arrays as they lie (targets under the results
+    // would be overwritten while other blocks read them)
+    void *tmp = nullptr;
+    const size_t be = sizeof(double) * ctx->n, bo = sizeof(double) * width * nt, bt = sizeof(int) * nt;
+    InPlace usable{ctx};
+    const bool ce = eps && (host || !usable(eps, be, sizeof(double)));
+    const bool ct = host || !usable(targets, bt, sizeof(int));
+    const bool co = host || !usable(out, bo, sizeof(double)) ||
+                    ((char *)out < (const char *)targets + bt && (const char *)targets < (char *)out + bo);
+    if (ce || ct || co) {
+        CK(cudaMalloc(&tmp, (ce ? be : 0) + (co ? bo : 0) + (ct ? bt : 0)));
+        char *d = (char *)tmp;
+        const cudaMemcpyKind kind = host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
         // copies on the context's non-blocking stream, ordered before the kernels
-        cudaError_t e = cudaMemcpyAsync(t, targets, sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream);
-        if (e == cudaSuccess && eps)
-            e = cudaMemcpyAsync(d, eps, sizeof(double) * ctx->n, cudaMemcpyHostToDevice, ctx->stream);
+        cudaError_t e = cudaSuccess;
+        if (ce) {
+            e = cudaMemcpyAsync(d, eps, be, kind, ctx->stream);
+            ep = (double *)d;
+            d += be;
+        }
+        if (co) {
+            res = (double *)d;
+            d += bo;
+        }
+        if (ct && e == cudaSuccess) {
+            e = cudaMemcpyAsync(d, targets, bt, kind, ctx->stream);
+            tg = (int *)d;
+        }
         if (e != cudaSuccess) {
             cudaFree(tmp);
             return ctx_fail(ctx, e, "cudaMemcpyAsync", __LINE__);
@@ -1027,8 +1089,9 @@ static int direct_common(sph_ctx *ctx, const double *eps, int32_t nt, const int3
         rc = launch_gravity_direct(ctx, nt, tg, res);
     }
     cudaError_t e = cudaSuccess;
-    if (!rc && host)
-        e = cudaMemcpyAsync(out, res, sizeof(double) * width * nt, cudaMemcpyDeviceToHost, ctx->stream);
+    if (!rc && co)
+        e = cudaMemcpyAsync(out, res, bo, host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice,
+                            ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (tmp) cudaFree(tmp);
     if (!rc && e != cudaSuccess) return ctx_fail(ctx, e, "direct sum", __LINE__);
