@@ -94,7 +94,9 @@ extern "C" {
 #define SPH_S_NONFINITE 6     /* non-finite inputs seen                          */
 #define SPH_S_WALK_STACK_MAX 7/* deepest traversal stack seen in the gravity walk */
 #define SPH_S_WAIT_TIMEOUT 8  /* bounded device waits that gave up (tensor-core MLP
-                                 tiles; their rows go to the exact solver)        */
+                                 tiles: their rows go to the exact solver; tiles of
+                                 the sort: they count the keys before them). The
+                                 results are the same                             */
 #define SPH_NSTATUS 9
 
 #define SPH_FLAG_DUDT_FUSED 1  /* du/dt in the force pass (one pass) instead of the
@@ -114,6 +116,10 @@ extern "C" {
 #define SPH_FLAG_NO_ROW_REUSE 512 /* search every particle in each h iteration
                                   instead of keeping a candidate row that the
                                   particles' moves since its search leave complete */
+#define SPH_FLAG_SORT_COUNT 1024 /* a tile of the sort counts the keys before it
+                                 instead of waiting for the other tiles' counts, as
+                                 one whose wait has passed its limit does: the same
+                                 permutation, slower                             */
 
 typedef struct sph_config {
     int32_t n_max;        /* particle capacity                                    */

@@ -38,6 +38,7 @@ FLAG_COOLING_TABLE = 64
 FLAG_STATIC_GRID = 128
 FLAG_MLP_WARP_MMA = 256
 FLAG_NO_ROW_REUSE = 512
+FLAG_SORT_COUNT = 1024
 PHASES = ["kick_drift", "sort", "tree", "smoothing_h", "neighbours", "density", "divcurl",
           "forces", "wait_kick", "dudt", "update_dt", "gravity"]
 MLP_NPARAM = 3 * 64 + 64 + 64 * 64 + 64 + 64 + 1

@@ -152,7 +152,10 @@ __device__ __forceinline__ unsigned long long morton_key(
 // and including it.
 constexpr unsigned LOCAL = 1u << 30, TOTAL = 2u << 30, VALUE = (1u << 30) - 1u;
 constexpr int LOOK = 4;  // tiles read per step of the look-back (8, 16: 1 to 4 % slower)
-constexpr int LOOK_LIMIT = 1 << 22;  // polls before a wait gives up
+// Polls of a thread that find nothing new before it gives up waiting and counts
+// its digit among the keys of the tiles that it has not added yet: the same sum
+// from the pass's input, so the permutation is right whatever the other tiles do.
+constexpr int LOOK_LIMIT = 1 << 22;
 
 __global__ void __launch_bounds__(SORT_THREADS)
     k_keys(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
@@ -197,7 +200,7 @@ template <int ITEMS, bool EXCHANGE>
 __global__ void __launch_bounds__(SORT_THREADS)
     k_radix_pass(const unsigned long long *__restrict__ kin, const int *__restrict__ vin,
                  unsigned long long *__restrict__ kout, int *__restrict__ vout, int n, int shift,
-                 const unsigned *__restrict__ tot, unsigned *state, unsigned *ticket,
+                 const unsigned *__restrict__ tot, unsigned *state, unsigned *ticket, int polls,
                  long long *status) {
     __shared__ unsigned cnt[SORT_WARPS][256];  // counts, then places, per warp and digit
     __shared__ unsigned tmp[SORT_WARPS], tmp2[SORT_WARPS];
@@ -248,8 +251,9 @@ __global__ void __launch_bounds__(SORT_THREADS)
     const unsigned start = scan256(tot[t], tmp);  // where digit t begins
     unsigned prev = 0;
     if (tile > 0) {
-        int spins = 0;
-        for (int b = tile - 1; b >= 0;) {
+        int b = tile - 1, left = polls;
+        bool end = false;
+        while (b >= 0 && !end && left > 0) {
             // up to LOOK earlier tiles at a time
             unsigned v[LOOK];
 #pragma unroll
@@ -258,7 +262,7 @@ __global__ void __launch_bounds__(SORT_THREADS)
                                         state[(size_t)(b - q) * 256 + t])
                                         .load(cuda::memory_order_relaxed)
                                   : (unsigned)TOTAL;
-            bool end = false, stall = false;
+            bool stall = false;
 #pragma unroll
             for (int q = 0; q < LOOK; q++) {
                 if (!end && !stall) {
@@ -271,11 +275,12 @@ __global__ void __launch_bounds__(SORT_THREADS)
                     }
                 }
             }
-            if (end) break;
-            if (stall && ++spins > LOOK_LIMIT) {
-                status_add(status, SPH_S_WAIT_TIMEOUT, 1);
-                break;
-            }
+            left -= stall;
+        }
+        if (b >= 0 && !end) {
+            const int before = (b + 1) * SORT_THREADS * ITEMS;
+            for (int k = 0; k < before; k++) prev += ((unsigned)(kin[k] >> shift) & 255u) == (unsigned)t;
+            if (polls) status_add(status, SPH_S_WAIT_TIMEOUT, 1);
         }
         mine.store(TOTAL | (prev + sum), cuda::memory_order_relaxed);
     }
@@ -302,7 +307,7 @@ __global__ void __launch_bounds__(SORT_THREADS)
             if (p < in) {
                 const unsigned long long v = xkey[p];
                 const unsigned pos = to[(unsigned)(v >> shift) & 255u] + (unsigned)p;
-                if (pos < (unsigned)n) {  // (always, unless a wait gave up)
+                if (pos < (unsigned)n) {
                     kout[pos] = v;
                     vout[pos] = xval[p];
                 }
@@ -442,12 +447,13 @@ int launch_sort(sph_ctx *ctx) {
     const auto pass = sort_items(n) == 2   ? k_radix_pass<2, false>
                       : sort_items(n) == 4 ? k_radix_pass<4, false>
                                            : k_radix_pass<8, true>;
+    const int polls = ctx->cfg.flags & SPH_FLAG_SORT_COUNT ? 0 : LOOK_LIMIT;
     const unsigned long long *kin = ctx->key_in;
     const int *vin = nullptr;
     for (int p = 0; p < SORT_PASSES; p++) {
         const int o = (p + 1) & 1;
         pass<<<tiles, SORT_THREADS, 0, s>>>(kin, vin, ctx->key[o], ctx->val[o], n, 8 * p, tot + 256 * p,
-                                            state + (size_t)p * 256 * tiles, ticket + p, ctx->status);
+                                            state + (size_t)p * 256 * tiles, ticket + p, polls, ctx->status);
         kin = ctx->key[o];
         vin = ctx->val[o];
     }
