@@ -93,7 +93,7 @@ __device__ __forceinline__ double div_1_1(double x) {
 // the count are those of the plain iteration.
 struct CoolRes {
     double u_old, dt, nH, ratefact, A, heat;
-    bool plain;  // finite, positive: the shortcuts' arithmetic holds
+    bool plain;  // finite, positive: the shortcuts' arithmetic and bounds hold
     __device__ __forceinline__ CoolRes(const CoolDev &c, double rho, double u_old_, double dt_)
         : u_old(u_old_), dt(dt_) {
         nH = c.XH * rho / MH_CGS;
@@ -220,6 +220,48 @@ struct CoolRes {
     }
 };
 
+// |du / u| > tol, dividing only where the product cannot tell
+__device__ __forceinline__ bool cool_wide(const CoolDev &c, double du, double u) {
+    const double x = fabs(du), y = c.tol * fabs(u);
+    if (x > y * (1.0 + 1e-14)) return true;
+    if (x < y * (1.0 - 1e-14)) return false;
+    return fabs(du / u) > c.tol;
+}
+
+// The iteration with every sign from the FP64 residual, for rows outside the
+// shortcuts' range (a step back in time, a heating rate below zero, magnitudes
+// beyond it): their bounds take every term to be positive.  Not inlined, so that
+// the other rows' registers do not pay for it.
+struct CoolOut {
+    double u;
+    int count;
+};
+static __device__ __noinline__ CoolOut cool_solve_bare(CoolDev c, double rho, double u_old, double dt) {
+    const CoolRes res(c, rho, u_old, dt);
+    double u = u_old, up = u, lo = u;
+    const double r0 = res.exact(c, u);
+    int guard = 0;
+    if (r0 > 0.0) {
+        while (res.exact(c, up) > 0.0 && guard++ < 2000) up /= 1.1;
+        lo = up;
+        up = lo * 1.1;
+    } else if (r0 < 0.0) {
+        while (res.exact(c, up) < 0.0 && guard++ < 2000) up *= 1.1;
+        lo = up / 1.1;
+    } else {
+        return {u, 0};
+    }
+    double du = u;
+    int it = 1;
+    while (cool_wide(c, du, u) && it < c.max_iter) {
+        u = 0.5 * (lo + up);
+        if (res.exact(c, u) > 0.0) up = u; else lo = u;
+        du = fabs(up - lo);
+        it++;
+    }
+    return {u, cool_wide(c, du, u) ? -1 : it};
+}
+
 // Returns the bisection count, -1 if the tolerance was not reached.  What is
 // known of r's sign is kept as r < 0 on [kl, a] and r > 0 on [b, kh]; with the
 // root enclosed, bracket and bisection only compare with it.  2^20 states of
@@ -229,6 +271,11 @@ struct CoolRes {
 // 49 thousand cycles a warp are the bracket's divisions.
 __device__ __forceinline__ int cool_solve(const CoolDev &c, double rho, double u_old, double dt, double *u_new) {
     const CoolRes res(c, rho, u_old, dt);
+    if (!res.plain) {
+        const CoolOut o = cool_solve_bare(c, rho, u_old, dt);
+        *u_new = o.u;
+        return o.count;
+    }
     double u = u_old, up = u, lo = u;
     const int s0 = res.sign(c, u);
     int guard = 0;
@@ -238,32 +285,30 @@ __device__ __forceinline__ int cool_solve(const CoolDev &c, double rho, double u
     }
     double kl = INFINITY, a = -INFINITY, b = INFINITY, kh = -INFINITY;
     bool enclosed = false;
-    if (res.plain) {
-        int k0, k1;
-        const double safe = res.reach(c, s0, k0, k1);
-        // r increases over the run (or the bin) beyond the reach: its root, if
-        // it is there
-        const CoolBin b0 = c.bin[k0];
-        const double e0 = k0 > 0 ? b0.T * c.invkT : 0.0;
-        const double e1 = k1 < c.nb - 1 ? c.bin[k1 + 1].T * c.invkT : 1e300;
-        const bool inc = res.rises(c, b0) && (k0 > 0 || b0.sm1 >= -1.f);
-        if (s0 > 0) {
-            kh = u_old;
-            b = safe * (1.0 + 1e-12);
-            if (inc) {
-                res.enclose(c, e0, safe, safe, a, b);
-                kl = e0;
-            }
-            enclosed = a > 0.0 && b < safe;
-        } else {
-            kl = u_old;
-            a = safe * (1.0 - 1e-12);
-            if (inc) {
-                res.enclose(c, safe, e1, safe, a, b);
-                kh = e1;
-            }
-            enclosed = b < 1e300 && a > safe;
+    int k0, k1;
+    const double safe = res.reach(c, s0, k0, k1);
+    // r increases over the run (or the bin) beyond the reach: its root, if
+    // it is there
+    const CoolBin b0 = c.bin[k0];
+    const double e0 = k0 > 0 ? b0.T * c.invkT : 0.0;
+    const double e1 = k1 < c.nb - 1 ? c.bin[k1 + 1].T * c.invkT : 1e300;
+    const bool inc = res.rises(c, b0) && (k0 > 0 || b0.sm1 >= -1.f);
+    if (s0 > 0) {
+        kh = u_old;
+        b = safe * (1.0 + 1e-12);
+        if (inc) {
+            res.enclose(c, e0, safe, safe, a, b);
+            kl = e0;
         }
+        enclosed = a > 0.0 && b < safe;
+    } else {
+        kl = u_old;
+        a = safe * (1.0 - 1e-12);
+        if (inc) {
+            res.enclose(c, safe, e1, safe, a, b);
+            kh = e1;
+        }
+        enclosed = b < 1e300 && a > safe;
     }
     auto sgn = [&](double v) {
         if (v >= b && v <= kh) return 1;
@@ -291,7 +336,7 @@ __device__ __forceinline__ int cool_solve(const CoolDev &c, double rho, double u
         while (sgn(up) < 0 && guard++ < 2000) up *= 1.1;
         lo = div_1_1(up);
     }
-    if (res.plain && !enclosed && res.monotone(c, lo, up)) {
+    if (!enclosed && res.monotone(c, lo, up)) {
         // (only what this confirms about the bracket counts)
         a = -INFINITY;
         b = INFINITY;
@@ -299,23 +344,23 @@ __device__ __forceinline__ int cool_solve(const CoolDev &c, double rho, double u
         kl = lo;
         kh = up;
     }
-    // |du / u| > tol, dividing only where the product cannot tell
-    auto wide = [&](double du) {
-        const double x = fabs(du), y = c.tol * fabs(u);
-        if (x > y * (1.0 + 1e-14)) return true;
-        if (x < y * (1.0 - 1e-14)) return false;
-        return fabs(du / u) > c.tol;
-    };
     double du = u;
     int it = 1;
-    while (wide(du) && it < c.max_iter) {
+    while (cool_wide(c, du, u) && it < c.max_iter) {
         u = 0.5 * (lo + up);
         if (sgn(u) > 0) up = u; else lo = u;
         du = fabs(up - lo);
         it++;
     }
     *u_new = u;
-    return wide(du) ? -1 : it;
+    return cool_wide(c, du, u) ? -1 : it;
+}
+
+// the same as a call, where few rows come to it
+static __device__ __noinline__ CoolOut cool_solve_call(const CoolDev &c, double rho, double u_old, double dt) {
+    CoolOut o;
+    o.count = cool_solve(c, rho, u_old, dt, &o.u);
+    return o;
 }
 
 
