@@ -93,6 +93,7 @@ __device__ __forceinline__ double div_1_1(double x) {
 // the count are those of the plain iteration.
 struct CoolRes {
     double u_old, dt, nH, ratefact, A, heat;
+    double sum;  // u_old + heat; infinite where not plain: no sign is certain then
     bool plain;  // finite, positive: the shortcuts' arithmetic and bounds hold
     __device__ __forceinline__ CoolRes(const CoolDev &c, double rho, double u_old_, double dt_)
         : u_old(u_old_), dt(dt_) {
@@ -101,6 +102,7 @@ struct CoolRes {
         A = ratefact * dt;
         heat = A * (c.gheat / nH);
         plain = u_old > 0.0 && u_old < 1e30 && A > 0.0 && A < 1e300 && heat >= 0.0 && heat < 1e300;
+        sum = plain ? u_old + heat : (double)INFINITY;
     }
     __device__ __forceinline__ int bin(const CoolDev &c, double T) const {
         const int k = (int)floorf((__log2f((float)T) - c.l2T0) * c.l2inv);
@@ -129,7 +131,7 @@ struct CoolRes {
         float sm1, rel;
         const double cool = fast(c, u, sm1, rel), r = u - u_old - (heat - cool);
         // (values outside the FP32 range give a bound that is not finite)
-        if (fabs(r) > cool * (double)rel + 1e-14 * (u + u_old + heat + cool)) return r > 0.0 ? 1 : -1;
+        if (fabs(r) > cool * (double)rel + 1e-14 * (u + sum + cool)) return r > 0.0 ? 1 : -1;
         const double re = exact(c, u);
         return re > 0.0 ? 1 : (re < 0.0 ? -1 : 0);
     }
@@ -231,7 +233,8 @@ __device__ __forceinline__ bool cool_wide(const CoolDev &c, double du, double u)
 // The iteration with every sign from the FP64 residual, for rows outside the
 // shortcuts' range (a step back in time, a heating rate below zero, magnitudes
 // beyond it): their bounds take every term to be positive.  Not inlined, so that
-// the other rows' registers do not pay for it.
+// the other rows' registers do not pay for it (2^20 plain rows: 279 us, against 292
+// with such rows in the loops below).
 struct CoolOut {
     double u;
     int count;
@@ -269,9 +272,13 @@ static __device__ __noinline__ CoolOut cool_solve_bare(CoolDev c, double rho, do
 // ms with sign() alone (a row takes 46 bracket steps and 17 bisections, the
 // longest of a warp 168), 0.26 ms with the reach and the enclosure, 13 of whose
 // 49 thousand cycles a warp are the bracket's divisions.
+// BARE: rows that are not plain leave by a call; without it they stay in these loops
+// with every sign exact, for kernels whose registers a call would cost more (the
+// tensor-core surrogate: 129 us, with it 135).
+template <bool BARE = true>
 __device__ __forceinline__ int cool_solve(const CoolDev &c, double rho, double u_old, double dt, double *u_new) {
     const CoolRes res(c, rho, u_old, dt);
-    if (!res.plain) {
+    if (BARE && !res.plain) {
         const CoolOut o = cool_solve_bare(c, rho, u_old, dt);
         *u_new = o.u;
         return o.count;
@@ -285,30 +292,32 @@ __device__ __forceinline__ int cool_solve(const CoolDev &c, double rho, double u
     }
     double kl = INFINITY, a = -INFINITY, b = INFINITY, kh = -INFINITY;
     bool enclosed = false;
-    int k0, k1;
-    const double safe = res.reach(c, s0, k0, k1);
-    // r increases over the run (or the bin) beyond the reach: its root, if
-    // it is there
-    const CoolBin b0 = c.bin[k0];
-    const double e0 = k0 > 0 ? b0.T * c.invkT : 0.0;
-    const double e1 = k1 < c.nb - 1 ? c.bin[k1 + 1].T * c.invkT : 1e300;
-    const bool inc = res.rises(c, b0) && (k0 > 0 || b0.sm1 >= -1.f);
-    if (s0 > 0) {
-        kh = u_old;
-        b = safe * (1.0 + 1e-12);
-        if (inc) {
-            res.enclose(c, e0, safe, safe, a, b);
-            kl = e0;
+    if (BARE || res.plain) {
+        int k0, k1;
+        const double safe = res.reach(c, s0, k0, k1);
+        // r increases over the run (or the bin) beyond the reach: its root, if
+        // it is there
+        const CoolBin b0 = c.bin[k0];
+        const double e0 = k0 > 0 ? b0.T * c.invkT : 0.0;
+        const double e1 = k1 < c.nb - 1 ? c.bin[k1 + 1].T * c.invkT : 1e300;
+        const bool inc = res.rises(c, b0) && (k0 > 0 || b0.sm1 >= -1.f);
+        if (s0 > 0) {
+            kh = u_old;
+            b = safe * (1.0 + 1e-12);
+            if (inc) {
+                res.enclose(c, e0, safe, safe, a, b);
+                kl = e0;
+            }
+            enclosed = a > 0.0 && b < safe;
+        } else {
+            kl = u_old;
+            a = safe * (1.0 - 1e-12);
+            if (inc) {
+                res.enclose(c, safe, e1, safe, a, b);
+                kh = e1;
+            }
+            enclosed = b < 1e300 && a > safe;
         }
-        enclosed = a > 0.0 && b < safe;
-    } else {
-        kl = u_old;
-        a = safe * (1.0 - 1e-12);
-        if (inc) {
-            res.enclose(c, safe, e1, safe, a, b);
-            kh = e1;
-        }
-        enclosed = b < 1e300 && a > safe;
     }
     auto sgn = [&](double v) {
         if (v >= b && v <= kh) return 1;
@@ -336,7 +345,7 @@ __device__ __forceinline__ int cool_solve(const CoolDev &c, double rho, double u
         while (sgn(up) < 0 && guard++ < 2000) up *= 1.1;
         lo = div_1_1(up);
     }
-    if (!enclosed && res.monotone(c, lo, up)) {
+    if ((BARE || res.plain) && !enclosed && res.monotone(c, lo, up)) {
         // (only what this confirms about the bracket counts)
         a = -INFINITY;
         b = INFINITY;
@@ -354,13 +363,6 @@ __device__ __forceinline__ int cool_solve(const CoolDev &c, double rho, double u
     }
     *u_new = u;
     return cool_wide(c, du, u) ? -1 : it;
-}
-
-// the same as a call, where few rows come to it
-static __device__ __noinline__ CoolOut cool_solve_call(const CoolDev &c, double rho, double u_old, double dt) {
-    CoolOut o;
-    o.count = cool_solve(c, rho, u_old, dt, &o.u);
-    return o;
 }
 
 

@@ -881,7 +881,7 @@ __global__ void __launch_bounds__(tc::ROWS, tc::CTAS)
 
 // in-step cooling with the tensor-core surrogate, 128 rows per CTA
 __global__ void __launch_bounds__(tc::ROWS, tc::CTAS)
-    k_cool_mlp_tc(const __grid_constant__ CoolDev c, int n, const double *__restrict__ rho, double *__restrict__ u,
+    k_cool_mlp_tc(CoolDev c, int n, const double *__restrict__ rho, double *__restrict__ u,
                   const int *__restrict__ cloud, const double *__restrict__ dt, double ur,
                   double uu, double ut, const __nv_bfloat16 *__restrict__ pk,
                   const float *__restrict__ P, double err_tol, int *__restrict__ list, int cap,
@@ -917,9 +917,8 @@ __global__ void __launch_bounds__(tc::ROWS, tc::CTAS)
             } else {
                 status_add(status, SPH_S_MLP_FALLBACK, 1);
                 if (!to_list(list, cap, i)) {
-                    const CoolOut o = cool_solve_call(c, rho_c, u0, dt_c);
-                    if (o.count < 0) status_add(status, SPH_S_COOL_NOCONV, 1);
-                    u[i] = o.u / uu;
+                    if (cool_solve<false>(c, rho_c, u0, dt_c, &un) < 0) status_add(status, SPH_S_COOL_NOCONV, 1);
+                    u[i] = un / uu;
                 }
             }
         }
@@ -929,7 +928,7 @@ __global__ void __launch_bounds__(tc::ROWS, tc::CTAS)
 
 // the same for standalone arrays (cgs), with the per-row fallback flag
 __global__ void __launch_bounds__(tc::ROWS, tc::CTAS)
-    k_cool_mlp_arrays_tc(const __grid_constant__ CoolDev c, int n, const double *__restrict__ rho,
+    k_cool_mlp_arrays_tc(CoolDev c, int n, const double *__restrict__ rho,
                          const double *__restrict__ u_old, const double *__restrict__ dtv,
                          double *__restrict__ u_new, int *__restrict__ fell_back,
                          const __nv_bfloat16 *__restrict__ pk, const float *__restrict__ P,
@@ -961,7 +960,8 @@ __global__ void __launch_bounds__(tc::ROWS, tc::CTAS)
             } else {
                 fb = 1;
                 if (!to_list(list, cap, i)) {
-                    u_new[i] = cool_solve_call(c, r, u0, d).u;
+                    cool_solve<false>(c, r, u0, d, &un);
+                    u_new[i] = un;
                 }
             }
             if (fell_back) fell_back[i] = fb;
