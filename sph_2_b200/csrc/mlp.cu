@@ -217,7 +217,9 @@ struct GradSmem {
 
 // The two kernels of a training step follow each other in programmatic stream
 // order: the next one's blocks start while the last one's finish and wait here
-// for all of it (its writes included) before they touch global memory.
+// for all of it (its writes included) before they touch global memory.  What that
+// kernel writes (pk and P, part) is no __restrict__ const here: the qualifier
+// lets the compiler read it by non-coherent loads and ahead of the wait.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -247,8 +249,7 @@ __device__ __forceinline__ void ldm4t(const __nv_bfloat16 *p, unsigned r[4]) {
 
 __global__ void __launch_bounds__(256, GBLOCKS)
     k_mlp_grad(int n, const float *__restrict__ X, const float *__restrict__ T, float inv_n,
-               const __nv_bfloat16 *__restrict__ pk, const float *__restrict__ P,
-               float *__restrict__ part) {
+               const __nv_bfloat16 *pk, const float *P, float *__restrict__ part) {
     __shared__ GradSmem S;
     const int t = threadIdx.x, w = t >> 5, lane = t & 31, gid = lane >> 2, tig = lane & 3;
     for (int e = t; e < 2 * GROWS * LDX / 2; e += 256) reinterpret_cast<unsigned *>(S.X)[e] = 0u;
@@ -466,8 +467,8 @@ struct AdamArgs {
 };
 template <bool ADAM>
 __global__ void __launch_bounds__(256)
-    k_mlp_update(int nblk, const float *__restrict__ part, float *__restrict__ grad,
-                 float *__restrict__ loss, AdamArgs A) {
+    k_mlp_update(int nblk, const float *part, float *__restrict__ grad, float *__restrict__ loss,
+                 AdamArgs A) {
     __shared__ float sum[8][32];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = blockIdx.x * 32 + lane;
