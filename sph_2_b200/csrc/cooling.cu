@@ -72,16 +72,12 @@ int sph_cooling_setup(sph_ctx *ctx, const sph_cooling_params *p, const double *l
     CK(cudaMemcpyAsync(ctx->cool_table, log_lambda, sizeof(double) * (p->n_bins + 1),
                        cudaMemcpyHostToDevice, ctx->stream));
     {
-        // Lambda(T_e) / T_e at the bin edges, for the surrogate's monotonicity test
         const double dl = (p->logT1 - p->logT0) / p->n_bins;
-        std::vector<double> lamT(p->n_bins + 1);
-        for (int e = 0; e <= p->n_bins; e++) lamT[e] = pow(10.0, log_lambda[e] - (p->logT0 + e * dl));
-        CK(cudaMemcpyAsync(ctx->cool_table + COOL_EDGES, lamT.data(), sizeof(double) * (p->n_bins + 1),
-                           cudaMemcpyHostToDevice, ctx->stream));
         std::vector<CoolBin> bin(p->n_bins);
         for (int e = 0; e < p->n_bins; e++) {
             const double slope = (log_lambda[e + 1] - log_lambda[e]) / dl;
-            bin[e] = {lamT[e], pow(10.0, -(p->logT0 + e * dl)), pow(10.0, p->logT0 + e * dl),
+            const double lt = p->logT0 + e * dl;
+            bin[e] = {pow(10.0, log_lambda[e] - lt), pow(10.0, -lt), pow(10.0, lt),
                       (float)(slope - 1.0), (short)e, (short)e, log_lambda[e], slope,
                       log_lambda[e + 1] - log_lambda[e], 0.0};
             if (slope < 0.0 && bin[e].sm1 >= -1.f) bin[e].sm1 = nextafterf(-1.f, -2.f);

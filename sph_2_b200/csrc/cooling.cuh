@@ -21,19 +21,18 @@ struct __align__(16) CoolBin {
     double lamT, invT, T;  // Lambda(T_e) / T_e, 1 / T_e, T_e
     float sm1;             // d ln Lambda / d ln T - 1
     short dn, un;
-    double logL, s, diff;  // log10 Lambda(T_e), the slope as cool_lambda forms it, the rise
+    double logL, s, diff;  // log10 Lambda(T_e), the slope, the rise
     double pad;
 };
 constexpr int COOL_EDGES = 4097;  // edges of the largest table
-// the cooling tables in one allocation: log Lambda and Lambda / T at the edges,
-// a CoolBin per bin, and (log Lambda, slope) per bin in FP32
-constexpr size_t COOL_AT_BIN = sizeof(double) * 2 * (COOL_EDGES + 1);
+// the cooling tables in one allocation: log Lambda at the edges, a CoolBin per bin,
+// and (log Lambda, slope) per bin in FP32
+constexpr size_t COOL_AT_BIN = sizeof(double) * (COOL_EDGES + 1);
 constexpr size_t COOL_AT_BINF = COOL_AT_BIN + sizeof(CoolBin) * COOL_EDGES;
 constexpr size_t COOL_BYTES = COOL_AT_BINF + sizeof(float2) * COOL_EDGES;
 
 struct CoolDev {
     const double *logL;
-    const double *lamT;  // Lambda(T_e) / T_e at the bin edges T_e (host-computed)
     const CoolBin *bin;
     const float2 *binf;  // (log10 Lambda(T_e), slope) in FP32
     int nb;
@@ -44,24 +43,8 @@ struct CoolDev {
     int max_iter;
 };
 
-__device__ __forceinline__ double cool_lambda(const CoolDev &c, double T, double *slope) {
-    const double lt = log10(T);
-    const double dl = (c.logT1 - c.logT0) / c.nb;
-    int k = (int)floor((lt - c.logT0) / dl);
-    k = k < 0 ? 0 : (k > c.nb - 1 ? c.nb - 1 : k);
-    const double s = (c.logL[k + 1] - c.logL[k]) / dl;
-    const double ll = c.logL[k] + s * (lt - (c.logT0 + k * dl));
-    if (slope) *slope = s;
-    return exp10(ll);
-}
-
-__device__ __forceinline__ double cool_net(const CoolDev &c, double u, double nH) {
-    const double T = (c.gamma - 1.0) * c.mu * MH_CGS / KB_CGS * u;
-    return c.gheat / nH - cool_lambda(c, T, nullptr);
-}
-
-// cool_lambda(c, T, nullptr), the same operations with the bin's slope from the
-// table.  One copy of its log10 and exp10: inlined at each of the solve's ten
+// The cooling function Lambda(T): a power of T in each bin of the table, the end
+// bins' beyond it.  One copy of its log10 and exp10: inlined at each of the solve's ten
 // call sites they overran the instruction cache (no_instruction the first
 // stall, 5.3 of 11.8 cycles per issue).
 static __device__ __noinline__ double cool_lambda_call(const CoolBin *bin, int nb, double logT0,
@@ -365,97 +348,6 @@ __device__ __forceinline__ int cool_solve(const CoolDev &c, double rho, double u
     return cool_wide(c, du, u) ? -1 : it;
 }
 
-
-// Newton-step estimate of the error of an approximate solution u of
-// u - u_old - ratefact * net(u) * dt = 0:  delta = r(u) / r'(u), with
-// r'(u) = 1 + ratefact * dt * s * Lambda(T) / u (Lambda ~ T^s inside a bin,
-// T ~ u).  Returns |delta|/u, or +inf where r' <= 0 (the estimate is void).
-__device__ __forceinline__ double cool_error_estimate(const CoolDev &c, double rho, double u_old,
-                                                      double dt, double u) {
-    const double nH = c.XH * rho / MH_CGS;
-    const double ratefact = nH * nH / rho;
-    const double T = (c.gamma - 1.0) * c.mu * MH_CGS / KB_CGS * u;
-    double s;
-    const double lam = cool_lambda(c, T, &s);
-    const double r = u - u_old - ratefact * (c.gheat / nH - lam) * dt;
-    const double rp = 1.0 + ratefact * dt * s * lam / u;
-    if (!(rp > 0.0) || !(u > 0.0)) return INFINITY;
-    return fabs(r / rp) / u;
-}
-
-// Newton steps of the implicit equation from an approximate solution *u (the
-// surrogate's prediction): at each iterate r(u) and r'(u) give the error
-// estimate |r/r'|/u; the iterate is kept as soon as that estimate is within
-// tol / 4, else u <- u - r/r' (when r' > 0 and the step keeps u positive),
-// at most four steps.  *est <- the estimate of the returned *u (+inf when it
-// is void).  One cooling-function evaluation per iterate.
-__device__ __forceinline__ void cool_newton_polish(const CoolDev &c, double rho, double u_old,
-                                                   double dt, double *u, double *est, double tol) {
-    const double nH = c.XH * rho / MH_CGS;
-    const double ratefact = nH * nH / rho;
-    const double kT = (c.gamma - 1.0) * c.mu * MH_CGS / KB_CGS;
-    double uu = *u;
-    *est = INFINITY;
-    for (int it = 0; it < 5; it++) {
-        double s;
-        const double lam = cool_lambda(c, kT * uu, &s);
-        const double r = uu - u_old - ratefact * (c.gheat / nH - lam) * dt;
-        const double rp = 1.0 + ratefact * dt * s * lam / uu;
-        if (!(rp > 0.0) || !(uu > 0.0)) break;  // the estimate is void here
-        const double e = fabs(r / rp) / uu;
-        *u = uu;
-        *est = e;
-        if (e <= 0.25 * tol || it == 4) break;
-        const double u1 = uu - r / rp;
-        if (!(u1 > 0.0)) break;
-        uu = u1;
-    }
-}
-
-// True when r(u) = u - u_old - ratefact*net(u)*dt is strictly increasing on
-// [u_lo, u_hi]: r'(u) = 1 + ratefact*dt*s*Lambda(T)/u.  Inside a table bin
-// Lambda ~ T^s, so Lambda/u ~ T^(s-1): r' > 1 where s >= 0, and where s < 0 r'
-// grows with T, so its smallest value in a bin is at the bin's lower end.  The
-// interval is monotone iff r' > 0 at T(u_lo) (when its bin has s < 0) and at
-// the lower edge of every bin with s < 0 that starts inside the interval;
-// Lambda/T at the edges is tabulated, so only T(u_lo) needs a transcendental.
-__device__ __forceinline__ bool cool_monotone(const CoolDev &c, double rho, double dt, double u_lo,
-                                              double u_hi) {
-    const double nH = c.XH * rho / MH_CGS;
-    const double A = nH * nH / rho * dt;
-    const double kT = (c.gamma - 1.0) * c.mu * MH_CGS / KB_CGS;
-    const double dl = (c.logT1 - c.logT0) / c.nb;
-    const double T0 = kT * u_lo, T1 = kT * u_hi;
-    if (!(T0 > 0.0) || !(T1 >= T0)) return false;
-    const double l0 = log10(T0), l1 = log10(T1);
-    int k = (int)floor((l0 - c.logT0) / dl);
-    k = k < 0 ? 0 : (k > c.nb - 1 ? c.nb - 1 : k);
-    double s = (c.logL[k + 1] - c.logL[k]) / dl;
-    if (s < 0.0) {
-        const double lam = exp10(c.logL[k] + s * (l0 - (c.logT0 + k * dl)));
-        if (!(1.0 + A * s * lam * kT / T0 > 0.0)) return false;
-    }
-    // lower edges of the bins after T0's bin, up to T1 (edge k at logT0 + k dl;
-    // below bin 0 and above bin nb-1 the end slopes continue, no edges)
-    int kend = (int)floor((l1 - c.logT0) / dl);
-    kend = kend > c.nb - 1 ? c.nb - 1 : kend;
-    for (int e = k + 1; e <= kend; e++) {
-        s = (c.logL[e + 1] - c.logL[e]) / dl;
-        if (s < 0.0) {
-            if (!(1.0 + A * s * c.lamT[e] * kT > 0.0)) return false;
-        }
-    }
-    return true;
-}
-
-// accept a surrogate solution un (after cool_newton_polish, estimate est)?
-__device__ __forceinline__ bool cool_accept(const CoolDev &c, double rho, double u_old, double dt,
-                                            double un, double est, double tol) {
-    if (!(est <= tol) || !(un > 0.0)) return false;
-    const double lo = fmin(u_old, un / 1.1), hi = fmax(u_old, un * 1.1);
-    return cool_monotone(c, rho, dt, lo, hi);
-}
-
 // ---- the surrogate's side in FP32 -------------------------------------------
 // The surrogate is accepted to a relative error of mlp_err_tol (1e-3 by
 // default), far above FP32 rounding, so its Newton polish, error estimate and
@@ -479,6 +371,12 @@ __device__ __forceinline__ float cool_lambda_f(const CoolDev &c, float T, float 
     return __exp10f(b.x + b.y * (lt - (lT0 + k * dl)));
 }
 
+// Newton steps of u - u_old - ratefact net(u) dt = 0 from an approximate solution
+// *u (the surrogate's prediction): at each iterate r(u) and r'(u) = 1 + ratefact
+// dt s Lambda(T) / u (Lambda ~ T^s inside a bin, T ~ u) give the error estimate
+// |r / r'| / u; the iterate is kept as soon as that is within tol / 4, else
+// u <- u - r / r' (while r' > 0 and u stays positive), at most four steps.
+// *est <- the estimate of the returned *u (+inf where it is void).
 __device__ __forceinline__ void cool_newton_polish_f(const CoolDev &c, double rho, double u_old,
                                                      double dt, double *u, double *est, double tol) {
     const double nHd = c.XH * rho / MH_CGS;
@@ -504,6 +402,11 @@ __device__ __forceinline__ void cool_newton_polish_f(const CoolDev &c, double rh
     }
 }
 
+// True when r(u) increases strictly on [u_lo, u_hi].  Inside a bin Lambda / u ~
+// T^(s-1): r' > 1 where s >= 0, and where s < 0 r' grows with T, so it is smallest
+// at the bin's lower end.  r' > 0 at T(u_lo) (when its bin has s < 0) and at the
+// lower edge of every bin with s < 0 that starts inside the interval decides;
+// Lambda / T at the edges is tabulated, so only T(u_lo) needs a transcendental.
 __device__ __forceinline__ bool cool_monotone_f(const CoolDev &c, double rho, double dt, double u_lo,
                                                 double u_hi) {
     // A = ratefact * dt can pass the FP32 range: it is applied in FP64 to
@@ -542,6 +445,7 @@ __device__ __forceinline__ bool cool_monotone_f(const CoolDev &c, double rho, do
     return true;
 }
 
+// accept a surrogate solution un (after the polish, estimate est)?
 __device__ __forceinline__ bool cool_accept_f(const CoolDev &c, double rho, double u_old, double dt,
                                               double un, double est, double tol) {
     if (!(est <= tol) || !(un > 0.0)) return false;
@@ -553,7 +457,6 @@ static inline CoolDev cool_dev_of(const sph_ctx *ctx) {
     const sph_cooling_params &p = ctx->cool;
     CoolDev c;
     c.logL = ctx->cool_table;
-    c.lamT = ctx->cool_table + COOL_EDGES;
     c.bin = (const CoolBin *)((const char *)ctx->cool_table + COOL_AT_BIN);
     c.binf = (const float2 *)((const char *)ctx->cool_table + COOL_AT_BINF);
     c.nb = p.n_bins;
