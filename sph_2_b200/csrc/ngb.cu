@@ -1257,18 +1257,22 @@ template <int N> struct RowDist {
 // t_hi, the (hi_n + 1)-th.  The iteration's only state is h, so a particle
 // whose 2 h would pass its candidate radius 2 hc stops and resumes after a
 // wider search: the sequence of h is that of one uninterrupted iteration.
-// `narrow`: a row of this particle has overflowed.
+// The wider radius is a guess from the row's count; `step` is the radius that h
+// alone would have led to by now, B.grow past h whenever h passes it.  A guess
+// whose row overflows (a clump just outside the window, a row capacity just above
+// it) goes back to that, and `guess` ends: the particle then takes the small
+// steps to the end.
 // Returns whether the particle has to be searched again.
 __device__ __forceinline__ bool count_lane(const SearchArgs &A, const CountArgs &B, bool own,
-                                           double &h, double &hc, int &it, bool &narrow, int craw,
-                                           double t_lo, double t_hi, bool last_round) {
+                                           double &h, double &hc, double &step, bool &guess, int &it,
+                                           int craw, double t_lo, double t_hi, bool last_round) {
     const double cap = hc;
     bool ok = false, done = false, again = false;
     if (craw > A.K) {
-        // the row cannot hold every candidate: narrow the radius towards a
-        // half-full row and search again
-        hc = cap * fmax(0.5, cbrt(0.5 * A.K / (double)craw));
-        narrow = true;
+        // the row cannot hold every candidate: narrow the radius, for a row that
+        // no guess has widened towards a half-full one, and search again
+        hc = guess && cap > step ? step : cap * fmax(0.5, cbrt(0.5 * A.K / (double)craw));
+        guess = false;
         again = true;
     } else {
         // every j with d_j < 2 lim is in the row: the search's r^2 test is
@@ -1295,6 +1299,7 @@ __device__ __forceinline__ bool count_lane(const SearchArgs &A, const CountArgs 
                 h = xsub(h, xmul(B.frac, h));
             } else if (!(t_lo < h2)) {
                 h = xadd(h, xmul(B.frac, h));
+                if (h > step * (1.0 - 1e-12)) step = h * B.grow;
             } else {
                 ok = true;
                 break;
@@ -1303,11 +1308,10 @@ __device__ __forceinline__ bool count_lane(const SearchArgs &A, const CountArgs 
         }
         if (!ok && !done && !again) again = true;  // h passed the radius
         // the wider radius: past h, and past where a uniform density holds
-        // the window's count; past h alone once a row has overflowed, which
-        // that guess would only do again (a clump just outside the window)
+        // the window's count
         if (again)
-            hc = narrow ? h * B.grow
-                        : fmax(h * B.grow, cap * fmin(1.5, cbrt(1.2 * (B.hi_n + 1) / (double)max(craw, 1))));
+            hc = guess ? fmax(h * B.grow, cap * fmin(1.5, cbrt(1.2 * (B.hi_n + 1) / (double)max(craw, 1))))
+                       : h * B.grow;
     }
     if (again && own) status_add(A.status, SPH_S_H_RETRY, 1);
     again = again && !last_round;
@@ -1333,7 +1337,8 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, 4)
         const int root = A.croot[A.gcloud[u.g]];
         double h = pi.w, hc = B.hc[u.i];
         int it = 0;
-        bool act = u.in, narrow = false;
+        double step = hc;
+        bool act = u.in, guess = true;
         for (int round = 0; round < B.rounds && __any_sync(FULL, act); round++) {
             const int craw = group_search<2, double, SPLIT>(smem[w], A, root, act, u.i, pi, 2.0 * hc);
             double t_lo = INFINITY, t_hi = INFINITY;
@@ -1353,7 +1358,7 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, 4)
                 if (cc <= 32 * SEL_SHORT) both(RowDist<SEL_SHORT>(A, ii, A.p0[ii], cc));
                 else both(RowDist<SEL_MAX>(A, ii, A.p0[ii], cc));
             }
-            if (act) act = count_lane(A, B, own, h, hc, it, narrow, craw, t_lo, t_hi, round == B.rounds - 1);
+            if (act) act = count_lane(A, B, own, h, hc, step, guess, it, craw, t_lo, t_hi, round == B.rounds - 1);
         }
         if (u.in && own) {
             B.hc[u.i] = hc;
@@ -1615,8 +1620,7 @@ int launch_smoothing_h_count(sph_ctx *ctx, int n_target, int n_tol, double frac,
     B.grow = H_GROW_COUNT;
     // each round widens the radius by at least H_GROW_COUNT, so 16 rounds
     // cover a 3.4x change of h; one more for a guess that overflows the row
-    // and one for the half-full row it falls back to
-    B.rounds = 18;
+    B.rounds = 17;
     int rc;
     SPH_SPLIT(ctx, rc, search_launch(ctx, k_cand_count<SPLIT>, SPLIT, A, B));
     if (rc) return rc;

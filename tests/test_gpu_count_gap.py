@@ -43,3 +43,58 @@ def test_clump_outside_the_window(max_ngb, clump, at, copies):
         h = ctx.get("h")
         for i in centre[:: max(1, copies // 4)]:
             assert h[i] == O.ref_h_smooth_fast(i, i + 1, pos, h0, 2000)[0]
+
+
+def _small_steps(d, h, cap, K, lo, hi, frac, rounds, max_iter):
+    """The iteration over rows of at most K candidates, widened by 8 % past h at a
+    time: h where it ends inside the window, None where the rounds run out.
+    d: the particle's sorted distances, cap: half the first radius."""
+    it = 0
+    for _ in range(rounds):
+        c = np.searchsorted(d, 2.0 * cap, "right")
+        if c > K:
+            cap *= max(0.5, np.cbrt(0.5 * K / c))
+            continue
+        lim = cap * (1.0 - 1e-12)
+        n = lambda r: np.searchsorted(d[:c], r, "left")
+        if h > lim:
+            if n(2.0 * lim) <= hi:
+                cap = h * 1.08
+                continue
+            while h > lim:
+                h -= frac * h
+                it += 1
+        while h <= lim and it <= max_iter:
+            if n(2.0 * h) > hi:
+                h -= frac * h
+            elif n(2.0 * h) < lo:
+                h += frac * h
+            else:
+                return h
+            it += 1
+        cap = h * 1.08
+    return None
+
+
+@pytest.mark.parametrize("n,K,target,tol", [(6000, 64, 56, 4), (6000, 64, 58, 1), (30_000, 64, 50, 5), (3000, 128, 120, 6)])
+def test_rows_barely_above_the_window(n, K, target, tol):
+    """Where small steps of the radius end inside the window, so does the
+    iteration, with the same h."""
+    rng = np.random.default_rng(n + K)
+    pos = rng.uniform(-1.0, 1.0, size=(n, 3))
+    h0 = (target / n) ** (1 / 3) * rng.uniform(0.3, 1.2, n)
+    with Context(Config(n_max=n, precision="fp64", max_ngb=K)) as ctx:
+        ctx.load(pos, None, None, h0, None)
+        ctx.sort()
+        ctx.build_tree()
+        ctx.smoothing_h_count(n_target=target, n_tol=tol, max_iter=1500)
+        h = ctx.get("h")
+    ended = 0
+    for i in rng.integers(0, n, 400):
+        dx, dy, dz = (pos - pos[i]).T
+        d = np.sort(np.sqrt(dx * dx + dy * dy + dz * dz))
+        want = _small_steps(d, h0[i], 1.08 * h0[i], K, target - tol, target + tol, 0.003, 16, 1500)
+        if want is not None:
+            ended += 1
+            assert h[i] == want
+    assert ended
