@@ -38,7 +38,11 @@ constexpr int SEARCH_WARPS = 4;
 // iteration leaves 8 lanes for 32 or 32 for 8 (k_kept_shift)
 constexpr int SPLIT32_PER_SM = 34, SPLIT8_PER_SM = 68, SPLIT4_PER_SM = 140, SPLIT2_PER_SM = 300;
 constexpr double LONG8 = 1.6, LONG32 = 0.45;
-constexpr int SSTK = 512;
+// A node that does not fit the stack would leave particles out of rows and lists.
+// A round of `take` nodes adds at most `take` entries, so near the stack's end a
+// round takes fewer, down to one, whose descent the last SRES entries hold (63
+// key bits and 27 index bits of equal keys).
+constexpr int SSTK = 512, SRES = 96;
 constexpr unsigned FULL = 0xffffffffu;
 // pending bucket particles: ranges of consecutive slots, range r starting at
 // slot rf[r] and at offset rs[r] of the pending stream (rs ascending; at most
@@ -425,7 +429,7 @@ __device__ __forceinline__ int group_search(SearchSmem &S, const SearchArgs &A, 
 
     while (sp > 0 || nflat > 0) {
         if (sp > 0) {
-            const int take = min(sp, 32);
+            const int take = min(min(sp, 32), max(1, SSTK - SRES - sp));
             sp -= take;
             int nd = 0, f = 0, cn = 0, cl = 0, cr = 0;
             bool open = false;
