@@ -1264,19 +1264,19 @@ template <int N> struct RowDist {
 // The wider radius is a guess from the row's count; `step` is the radius that h
 // alone would have led to by now, B.grow past h whenever h passes it.  A guess
 // whose row overflows (a clump just outside the window, a row capacity just above
-// it) goes back to that, and `guess` ends: the particle then takes the small
-// steps to the end.
+// it) goes back to that, and the particle takes the small steps to the end (step
+// infinite).
 // Returns whether the particle has to be searched again.
 __device__ __forceinline__ bool count_lane(const SearchArgs &A, const CountArgs &B, bool own,
-                                           double &h, double &hc, double &step, bool &guess, int &it,
+                                           double &h, double &hc, double &step, int &it,
                                            int craw, double t_lo, double t_hi, bool last_round) {
     const double cap = hc;
     bool ok = false, done = false, again = false;
     if (craw > A.K) {
         // the row cannot hold every candidate: narrow the radius, for a row that
         // no guess has widened towards a half-full one, and search again
-        hc = guess && cap > step ? step : cap * fmax(0.5, cbrt(0.5 * A.K / (double)craw));
-        guess = false;
+        hc = cap > step ? step : cap * fmax(0.5, cbrt(0.5 * A.K / (double)craw));
+        step = INFINITY;
         again = true;
     } else {
         // every j with d_j < 2 lim is in the row: the search's r^2 test is
@@ -1314,8 +1314,9 @@ __device__ __forceinline__ bool count_lane(const SearchArgs &A, const CountArgs 
         // the wider radius: past h, and past where a uniform density holds
         // the window's count
         if (again)
-            hc = guess ? fmax(h * B.grow, cap * fmin(1.5, cbrt(1.2 * (B.hi_n + 1) / (double)max(craw, 1))))
-                       : h * B.grow;
+            hc = step < INFINITY
+                     ? fmax(h * B.grow, cap * fmin(1.5, cbrt(1.2 * (B.hi_n + 1) / (double)max(craw, 1))))
+                     : h * B.grow;
     }
     if (again && own) status_add(A.status, SPH_S_H_RETRY, 1);
     again = again && !last_round;
@@ -1342,7 +1343,7 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, 4)
         double h = pi.w, hc = B.hc[u.i];
         int it = 0;
         double step = hc;
-        bool act = u.in, guess = true;
+        bool act = u.in;
         for (int round = 0; round < B.rounds && __any_sync(FULL, act); round++) {
             const int craw = group_search<2, double, SPLIT>(smem[w], A, root, act, u.i, pi, 2.0 * hc);
             double t_lo = INFINITY, t_hi = INFINITY;
@@ -1362,7 +1363,7 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, 4)
                 if (cc <= 32 * SEL_SHORT) both(RowDist<SEL_SHORT>(A, ii, A.p0[ii], cc));
                 else both(RowDist<SEL_MAX>(A, ii, A.p0[ii], cc));
             }
-            if (act) act = count_lane(A, B, own, h, hc, step, guess, it, craw, t_lo, t_hi, round == B.rounds - 1);
+            if (act) act = count_lane(A, B, own, h, hc, step, it, craw, t_lo, t_hi, round == B.rounds - 1);
         }
         if (u.in && own) {
             B.hc[u.i] = hc;
