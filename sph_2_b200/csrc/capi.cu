@@ -162,12 +162,13 @@ struct LoadArgs {
     double *dt;
     unsigned long long *dt_bits;
     double dt0;
-    int one_cloud;
+    int one_cloud, *units;  // units: as launch_units_reset clears them
 };
 template <class R>
 __global__ void k_load(int n, LoadArgs a, typename R4<R>::T *__restrict__ p1,
                        typename R4<R>::T *__restrict__ pw) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) a.units[0] = a.units[1] = 0;
     if (a.one_cloud && i == 0) {
         a.cloud_start[0] = 0;
         a.cloud_start[1] = n;
@@ -699,13 +700,13 @@ int sph_load(sph_ctx *ctx, int32_t n, const int32_t *cloud, const double *x, con
         a.dt_bits = ctx->dt_bits;
         a.dt0 = dt0;
         a.one_cloud = cloud ? 0 : 1;
+        a.units = ctx->kept_cnt + 3;
         if (ctx->cfg.precision == SPH_PREC_MIXED)
             k_load<float><<<div_up(n, 256), 256, 0, s>>>(n, a, (float4 *)ctx->p1, (float4 *)ctx->pw);
         else
             k_load<double><<<div_up(n, 256), 256, 0, s>>>(n, a, (double4 *)ctx->p1, (double4 *)ctx->pw);
         if ((rc = launch_rows_invalidate(ctx))) return rc;
     }
-    if ((rc = launch_units_reset(ctx))) return rc;
     CK(cudaStreamSynchronize(s));
     ctx->tree_ok = ctx->lists_ok = ctx->rho_ok = ctx->divcurl_ok = ctx->cand_ok = false;
     ctx->p2_dirty = true;
