@@ -686,16 +686,16 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, POT ? 1 : BLOCKS)
 // warp, every warp for all of the group's particles; the warps' sums are
 // added at the end.  The group's box, its tests, and so its interactions are
 // those of k_walk.
-// A node that does not fit the stack is missing from the sums, so the stack holds
-// 16 rounds, as k_walk's does, and a round takes fewer nodes near its end, down
-// to one: a round of `take` nodes adds at most `take` entries, and the last BRES
-// hold the descent of one node at a time (63 key bits and the index bits of equal
-// keys: below 100 levels).  (8 rounds without that lost nodes of 100k particles at
-// theta 0.05 in buckets of one.)
-constexpr int BRES = 128;
+// A node that does not fit the stack would be missing from the sums, so near its end a
+// round takes fewer nodes, down to one: a round of `take` nodes adds at most `take`
+// entries, and the last BRES hold the descent of one node at a time (63 key bits
+// and the index bits of equal keys: below 100 levels).  (Without that 100k particles
+// at theta 0.05 in buckets of one lost nodes.  2048 entries, which only such walks
+// use, take shared memory from the resident blocks: 4 warps 1 to 4 % slower.)
+constexpr int BSTK = 1024, BRES = 128;
 // (BW warps, BT threads per group)
 template <class R, int BW> struct BlockWalkSmem {
-    static constexpr int BT = 32 * BW, BSTK = 16 * BT;
+    static constexpr int BT = 32 * BW;
     static constexpr bool PACKED = std::is_same<R, float>::value;
     typedef typename R4<R>::T V4;
     int stk[BSTK];
@@ -723,7 +723,7 @@ __global__ void __launch_bounds__(32 * BW)
                  SgArgs sg) {
     typedef typename R4<R>::T V4;
     constexpr bool PACKED = std::is_same<R, float>::value;
-    constexpr int BT = 32 * BW, BSTK = BlockWalkSmem<R, BW>::BSTK;
+    constexpr int BT = 32 * BW;
     __shared__ BlockWalkSmem<R, BW> S;
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
     const unsigned lt = (1u << lane) - 1u;
