@@ -1371,21 +1371,30 @@ __global__ void __cluster_dims__(DS_CLUSTER, 1, 1) __launch_bounds__(DS_WARPS * 
     cluster.sync();  // the others' sums stay until they are read
 }
 
-// Warps per group of the walk (k_walk_block; 1: k_walk).  us of one walk of an
-// Evrard sphere with 1 / 2 / 4 warps:
-//   FP64, theta 0.5:  10k 188 / 113 / 89;  45k 353 / 292 / 267;  100k 661 / 601 /
-//     593;  131k 843 / 763 / 775;  500k 3229 / 3123 / 3315
-//   FP32 with expansions (theta 0.35):  10k 144 / 83 / 59;  45k 240 / 192 / 179;
-//     65k 254 / 229 / 233;  100k 347 / 330 / 351;  131k 386 / 393 / 426
-//   FP32 without (theta 0.5):  10k 98 / 59 / 47;  45k 200 / 145 / 143;  100k 320 /
-//     290 / 311;  200k 593 / 573 / 643;  300k 853 / 872 / 979
-// The lines are in particles per SM.  (The super-group pre-walk in the same
-// form gained nothing: 131k 55 / 62 / 53 us.)
+// Warps per group of the walk (k_walk_block; 1: k_walk).  More of them shorten a
+// group's evaluations, but its rounds of the tree stay as many, and fewer groups are
+// resident: a shallow walk (clumps, a flat cloud, a wide angle: 200 to 400
+// interactions a particle) is made of rounds and loses as soon as its groups need a
+// second wave, a deep one (1000 to 4000) gains well beyond.  us of one walk with 1 /
+// 2 / 4 warps (FP64: the walk of one warp per group as it was / 2 / 4), deep: an Evrard
+// sphere, shallow: clumps of 300:
+//   FP64, theta 0.5, deep:  22k 266 / 195 / 157;  30k 317 / 216 / 206;  45k 366 /
+//     301 / 280;  100k 660 / 600 / 604;  shallow:  22k 86 / 70 / 74;  30k 97 / 90 /
+//     102;  45k 134 / 119 / 145;  100k 237 / 249 / 313;  theta 0.7:  100k 185 / 198 / 263
+//   FP32 with expansions (theta 0.35), deep:  22k 147 / 118 / 107;  30k 159 / 122 /
+//     125;  45k 185 / 171 / 165;  60k 203 / 200 / 210;  shallow:  22k 69 / 68 / 76;
+//     30k 72 / 75 / 92;  45k 80 / 91 / 117;  60k 94 / 105 / 144
+//   FP32 without (theta 0.5), deep:  22k 135 / 105 / 96;  30k 152 / 110 / 115;  45k
+//     204 / 158 / 157;  60k 216 / 192 / 200;  110k 345 / 334 / 353;  shallow:  22k 55 /
+//     54 / 61;  30k 61 / 63 / 81;  45k 69 / 79 / 117;  60k 85 / 100 / 148;  110k 135 /
+//     177 / 265
+// The lines are in particles per SM, where the shallow loss has come up to the deep
+// gain.  (The super-group pre-walk in the same form gained nothing: 131k 55 / 62 / 53 us.)
 int walk_warps(const sph_ctx *ctx) {
     const long long n = ctx->n, sm = ctx->num_sms;
-    if (ctx->cfg.precision == SPH_PREC_FP64) return n <= 750 * sm ? 4 : 2;
-    const int two = ctx->cfg.theta_local > 0.0 ? 740 : 1700;
-    return n <= 340 * sm ? 4 : n <= two * sm ? 2 : 1;
+    if (ctx->cfg.precision == SPH_PREC_FP64) return n <= 200 * sm ? 4 : 2;
+    const int two = ctx->cfg.theta_local > 0.0 ? 340 : 400;
+    return n <= 150 * sm ? 4 : n <= two * sm ? 2 : 1;
 }
 
 template <class R, bool POT>

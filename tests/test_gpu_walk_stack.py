@@ -23,10 +23,11 @@ def _positions(kind, n):
     return r[:, None] * d / np.linalg.norm(d, axis=1)[:, None]
 
 
-# 4 warps a group up to 750 particles per SM (111,000), 2 above
-@pytest.mark.parametrize("kind,n,theta", [("evrard", 100_000, 0.05), ("evrard", 110_000, 0.1),
-                                          ("core", 30_000, 0.1), ("core", 112_000, 0.1),
-                                          ("octaves", 100_000, 0.1), ("octaves", 112_000, 0.1)])
+# 4 warps a group up to 200 particles per SM (29,600), 2 above
+@pytest.mark.parametrize("kind,n,theta", [("evrard", 29_000, 0.05), ("evrard", 100_000, 0.05),
+                                          ("evrard", 110_000, 0.1), ("core", 29_000, 0.05),
+                                          ("core", 112_000, 0.1), ("octaves", 29_000, 0.05),
+                                          ("octaves", 29_000, 0.1), ("octaves", 112_000, 0.1)])
 def test_every_node_is_summed(kind, n, theta):
     pos, leaf = _positions(kind, n), 1
     with Context(Config(n_max=n, precision="fp64", theta=theta, leaf_size=leaf)) as ctx:
