@@ -11,7 +11,8 @@ rounding and the bucket sizes of the tree:
 The tuner times graph-replayed steps of the caller's loaded state on the
 device (CUDA events, sph_time_steps) for each candidate and walks the space
 by coordinate descent: leaf size first (the walk is the largest phase), then
-lanes, then block size.  Tuning advances the state by (warmup + steps) steps
+lanes, then block size.  (A cloud below 300 particles per SM takes at least 8
+lanes whatever the setting, so its lane candidates up to 8 run alike.)  Tuning advances the state by (warmup + steps) steps
 per candidate.  The choice is stored in a JSON cache keyed by the workload's
 signature (particles, clouds, precision, opening angles, GPU name), so the
 next run of the same workload starts from it without searching.

@@ -253,7 +253,7 @@ static __device__ __noinline__ CoolOut cool_solve_bare(CoolDev c, double rho, do
 // root enclosed, bracket and bisection only compare with it.  2^20 states of
 // the training range: 1.49 ms with every sign from the FP64 residual, 0.65
 // ms with sign() alone (a row takes 46 bracket steps and 17 bisections, the
-// longest of a warp 168), 0.26 ms with the reach and the enclosure, 13 of whose
+// longest of a warp 168), 0.25 ms with the reach and the enclosure, 13 of whose
 // 49 thousand cycles a warp are the bracket's divisions.
 // BARE: rows that are not plain leave by a call; without it they stay in these loops
 // with every sign exact, for kernels whose registers a call would cost more (the

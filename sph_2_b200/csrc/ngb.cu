@@ -752,7 +752,9 @@ struct ReuseArgs {
 //   10k FP64  460 / 685 at the start, 699 / 817 after 60 steps, 1552 / 1006 after 120
 //   7k FP64   311 / 472, 539 / 651, 1620 / 927;  5k FP64  283 / 337, 639 / 508, 1056 / 555
 // so the last iteration's longest search decides, 8 lanes up to LONG8 chunks per
-// particle of an SM's share, and back below LONG32 of them.  (The same by a
+// particle of an SM's share, and back below LONG32 of them.  (A load and a
+// restart begin anew: launch_units_reset.  Clouds above SPLIT8_PER_SM, with 4
+// lanes or fewer, have no such choice: the same was not measured there.)  (The same by a
 // second launch for the particles left after the first round: 10k 1422 after 150
 // steps, against 1936 without and 1092 with 32 lanes.)
 __global__ void k_kept_shift(int *kept, int long8, int long32) {
